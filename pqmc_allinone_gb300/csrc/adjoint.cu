@@ -18,38 +18,56 @@
 #include "chain.cuh"
 #include "linalg.cuh"
 #include "update_dev.cuh"
+#include "wrap.cuh"
 
 namespace pqmc {
 
 // dE/dx of the closed-form propagators (get_expKV_epsocz / _epsoc /
-// epsocz_block), entry (i,j); the general generator uses a central
-// difference of dev_get_expkv.
-__device__ cplx closed_dentry(const DevModel& M, int pf, int pla, double x, int i, int j) {
+// epsocz_block): the scalars every entry of a plaquette shares ...
+struct DEscal {
+  double dch, f, df;   // d cosh(n)/dx, sinh(n)/n, d(sinh(n)/n)/dx
+};
+__device__ __forceinline__ DEscal closed_dscal(const DevModel& M, int pf, double x) {
+  const int pd = M.pdim;
+  const cplx kc = M.k_coe[pf], vc = M.v_coe[pf];
+  // norm(x) and dnorm/dx
+  double norm, dnorm;
+  if (M.expkv_kind == PQMC_EXPKV_EPSOCZ_BLOCK) {
+    const cplx* K = M.kmat + (size_t)pd * pd * pf;
+    const cplx* V = M.vmat + (size_t)pd * pd * pf;
+    const cplx vx = cscale(vc, x);
+    cplx h11 = cadd(cmul(kc, K[0 + pd * 2]), cmul(vx, V[0 + pd * 2]));
+    cplx h21 = cadd(cmul(kc, K[1 + pd * 2]), cmul(vx, V[1 + pd * 2]));
+    cplx d11 = cmul(vc, V[0 + pd * 2]), d21 = cmul(vc, V[1 + pd * 2]);
+    double s = cabs2(h11) + cabs2(h21);
+    const double rs = sqrt(s);
+    norm = M.delt * rs;
+    double ds = 2.0 * (h11.x * d11.x + h11.y * d11.y + h21.x * d21.x + h21.y * d21.y);
+    dnorm = M.delt * ds / (2.0 * rs);
+  } else {
+    double a = cabsd(kc), b = cabsd(vc);
+    double s = a * a + (b * x) * (b * x);
+    const double rs = sqrt(s);
+    norm = M.delt * rs;
+    dnorm = M.delt * (b * b * x) / rs;
+  }
+  const double ch = cosh(norm), sh = sinh(norm);
+  DEscal q;
+  q.dch = sh * dnorm;
+  q.f = sh / norm;
+  q.df = (ch - q.f) * dnorm / norm;
+  return q;
+}
+// ... and entry (i,j)
+__device__ __forceinline__ cplx closed_dentry(const DevModel& M, int pf, int pla, double x, const DEscal& q, int i,
+                                              int j) {
   const int pd = M.pdim, dim = M.pf_dim[pf];
   const cplx kc = M.k_coe[pf], vc = M.v_coe[pf];
   const cplx* K = M.kmat + (size_t)pd * pd * pf;
   const cplx* V = M.vmat + (size_t)pd * pd * pf;
   const cplx* BC = M.bcp + (size_t)pd * pd * (pla + (size_t)M.max_pla * pf);
   const bool cross = M.cross[pla + M.max_pla * pf] != 0;
-  // norm(x) and dnorm/dx
-  double norm, dnorm;
-  if (M.expkv_kind == PQMC_EXPKV_EPSOCZ_BLOCK) {
-    const cplx vx = cscale(vc, x);
-    cplx h11 = cadd(cmul(kc, K[0 + pd * 2]), cmul(vx, V[0 + pd * 2]));
-    cplx h21 = cadd(cmul(kc, K[1 + pd * 2]), cmul(vx, V[1 + pd * 2]));
-    cplx d11 = cmul(vc, V[0 + pd * 2]), d21 = cmul(vc, V[1 + pd * 2]);
-    double s = cabs2(h11) + cabs2(h21);
-    norm = M.delt * sqrt(s);
-    double ds = 2.0 * (h11.x * d11.x + h11.y * d11.y + h21.x * d21.x + h21.y * d21.y);
-    dnorm = M.delt * ds / (2.0 * sqrt(s));
-  } else {
-    double a = cabsd(kc), b = cabsd(vc);
-    double s = a * a + (b * x) * (b * x);
-    norm = M.delt * sqrt(s);
-    dnorm = M.delt * (b * b * x) / sqrt(s);
-  }
-  const double ch = cosh(norm), sh = sinh(norm);
-  if (i == j) return mk(sh * dnorm);
+  if (i == j) return mk(q.dch);
   const int h = dim / 2;
   bool upper = (i < h && j >= h), lower = (i >= h && j < h);
   if (!upper && !lower) return mk(0.0);
@@ -63,46 +81,80 @@ __device__ cplx closed_dentry(const DevModel& M, int pf, int pla, double x, int 
     dsub = cmul(dsub, BC[a + pd * b]);
   }
   // d/dx [sub sinh(n)/n] = dsub sinh/n + sub (cosh n - sinh/n) dn / n
-  double f = sh / norm, df = (ch - f) * dnorm / norm;
-  cplx e = cadd(cscale(dsub, f), cscale(sub, df));
+  cplx e = cadd(cscale(dsub, q.f), cscale(sub, q.df));
   return upper ? e : cconj(e);
 }
 
-// Gradient of one family at one slice: grad(b, t) for the family's plaquettes.
-__global__ void k_grad_family(DevModel M, int pf, int t, const cplx* __restrict__ G, const double* __restrict__ field,
-                              const cplx* __restrict__ expkv_inv, double* grad, double scale) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= M.pf_npla[pf] || !M.pf_v_exist[pf]) return;
-  const int dim = M.pf_dim[pf], pd = M.pdim, ns = M.ns;
-  const int b = M.bf[p + M.max_pla * pf];
-  const double x = field[b + (size_t)M.n_bf * t];
-  int S[4];
-  for (int k = 0; k < dim; ++k) S[k] = M.site[k + pd * (p + M.max_pla * pf)];
-  cplx dE[16];
-  if (M.expkv_kind == PQMC_EXPKV_GENERAL) {
-    cplx ep[16], em[16];
-    const double h = 1e-5 * (1.0 + fabs(x));
-    dev_get_expkv(M, pf, p, x + h, false, ep);
-    dev_get_expkv(M, pf, p, x - h, false, em);
-    for (int k = 0; k < dim * dim; ++k) dE[k] = cscale(csub(ep[k], em[k]), 0.5 / h);
-  } else {
-    for (int j = 0; j < dim; ++j)
-      for (int i = 0; i < dim; ++i) dE[i + dim * j] = closed_dentry(M, pf, p, x, i, j);
+// One family at one slice of the gradient's left-to-right pass: the trace
+// terms grad(b, t) of its plaquettes from G, and the wrap of G by it
+// (left_evolve).  Both read the same G and neither the other's result, so
+// they share a launch: the first n_gb CTAs take the plaquettes, 16 lanes
+// each, one entry of E^-1 dE per lane; the rest the wrap's pairs.  The
+// plaquette part is one chain of FP64 transcendentals (sqrt, cosh, sinh,
+// three divisions), formed once per plaquette on all 16 lanes at the price
+// of one: a thread per plaquette that formed them again for each of its 16
+// entries took 84 us a family at 10x10 and 69 at 4x4.
+__global__ void __launch_bounds__(WRAP_THREADS) k_grad_wrap(
+    DevModel M, int pf, int t, int n_gb, const double* __restrict__ field, double* grad, double scale, int n_items,
+    const int* __restrict__ ipla, const int* __restrict__ isites, const int* __restrict__ idim,
+    const cplx* __restrict__ expkv, const cplx* __restrict__ expkv_inv, const cplx* __restrict__ G,
+    cplx* __restrict__ gout) {
+  if ((int)blockIdx.x >= n_gb) {
+    wrap_pair(M, pf, t, 1, n_items, ipla, isites, idim, expkv, expkv_inv, G, gout, (int)blockIdx.x - n_gb);
+    return;
   }
-  // A = E^-1 dE (expKV_inv is E^-1), trace with G(S,S):  sum_ab A_ab G(S_b, S_a)
-  const cplx* Ei = expkv_inv + M.kv_base(p, pf, t);
-  cplx tr = mk(0.0);
-  for (int a = 0; a < dim; ++a)
-    for (int bb = 0; bb < dim; ++bb) {
-      cplx aab = mk(0.0);
-      for (int k = 0; k < dim; ++k) aab = cfma(Ei[a + pd * k], dE[k + dim * bb], aab);
-      tr = cfma(aab, G[S[bb] + (size_t)ns * S[a]], tr);
-    }
-  grad[b + (size_t)M.n_bf * t] = scale * tr.x;
+  __shared__ cplx s_pm[WRAP_PAIRS][2][16];   // E at x + h and x - h (general form)
+  const int grp = threadIdx.x >> 4, lane = threadIdx.x & 31, sl = lane & 15, base = lane & 16;
+  const int p = (int)blockIdx.x * WRAP_PAIRS + grp;
+  const bool on = p < M.pf_npla[pf];
+  const int dim = M.pf_dim[pf], pd = M.pdim, ns = M.ns;
+  const int i = sl % dim, j = sl / dim;
+  const bool act = on && sl < dim * dim;
+  const int b = on ? M.bf[p + M.max_pla * pf] : 0;
+  const double x = on ? field[b + (size_t)M.n_bf * t] : 0.0;
+  // G(S_j, S_i) and row i of E^-1, in flight during the scalars
+  cplx g = mk(0.0), ei[4];
+  if (act) g = G[M.site[j + pd * (p + M.max_pla * pf)] + (size_t)ns * M.site[i + pd * (p + M.max_pla * pf)]];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) ei[k] = (act && k < dim) ? expkv_inv[M.kv_base(p, pf, t) + i + pd * k] : mk(0.0);
+  cplx de = mk(0.0);
+  if (M.expkv_kind == PQMC_EXPKV_GENERAL) {   // central difference of the exponential, one side per lane
+    const double h = 1e-5 * (1.0 + fabs(x));
+    if (on && sl < 2) dev_get_expkv(M, pf, p, sl ? x - h : x + h, false, s_pm[grp][sl]);
+    __syncwarp();
+    if (act) de = cscale(csub(s_pm[grp][0][sl], s_pm[grp][1][sl]), 0.5 / h);
+  } else if (on) {
+    const DEscal q = closed_dscal(M, pf, x);
+    if (act) de = closed_dentry(M, pf, p, x, q, i, j);
+  }
+  __syncwarp();
+  // Tr[E^-1 dE G(S,S)] = sum_ij (E^-1 dE)_ij G(S_j, S_i)
+  cplx a = mk(0.0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const cplx dk = shfl_c(de, base + k + dim * j);
+    if (k < dim) a = cfma(ei[k], dk, a);
+  }
+  double tr = act ? fma(a.x, g.x, -(a.y * g.y)) : 0.0;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
+  if (on && sl == 0) grad[b + (size_t)M.n_bf * t] = scale * tr;
 }
 
-int launch_propagate(pqmc_chain* c, cplx* X, int n, int t_from, int t_to, bool forward);
-int launch_wrap(pqmc_chain* c, int pf, int time, bool left);
+static int launch_grad_wrap(pqmc_chain* c, int pf, int tau, double* grad, double scale) {
+  const int npla = c->h_pf_npla[pf];
+  if (npla == 0 || !c->h_pf_v_exist[pf]) return launch_wrap(c, pf, tau, true);
+  const WrapItems& w = c->wrap[pf];
+  const int n_gb = (npla + WRAP_PAIRS - 1) / WRAP_PAIRS;
+  k_grad_wrap<<<n_gb + wrap_blocks(w.n_items), WRAP_THREADS, 0, c->stream>>>(
+      c->M, pf, tau - 1, n_gb, c->field, grad, scale, w.n_items, w.d_pla, w.d_sites, w.d_dim, c->expkv, c->expkv_inv,
+      c->g, c->g_alt);
+  PQMC_LAUNCHED();
+  cplx* t = c->g;
+  c->g = c->g_alt;
+  c->g_alt = t;
+  return PQMC_OK;
+}
 
 }  // namespace pqmc
 
@@ -173,14 +225,7 @@ extern "C" int pqmc_logweight_grad(pqmc_chain* c, double* logw_out, double* grad
     PQMC_TRY(lu_solve(s, ne, ns, c->pbp, c->ipiv, c->lmat, ne));
     PQMC_TRY(zgemm(s, 'N', 'N', ns, ns, ne, mk(1.0), c->rmat, ns, c->lmat, ne, mk(0.0), c->g, ns));
     for (int tau = t0 + 1; tau <= t1; ++tau) {
-      for (int pf = 0; pf < c->n_pf; ++pf) {
-        const int npla = c->h_pf_npla[pf];
-        if (npla > 0 && c->h_pf_v_exist[pf]) {
-          k_grad_family<<<(npla + 63) / 64, 64, 0, s>>>(c->M, pf, tau - 1, c->g, c->field, c->expkv_inv, grad_dev, scale);
-          PQMC_LAUNCHED();
-        }
-        PQMC_TRY(launch_wrap(c, pf, tau, true));
-      }
+      for (int pf = 0; pf < c->n_pf; ++pf) PQMC_TRY(launch_grad_wrap(c, pf, tau, grad_dev, scale));
     }
     PQMC_TRY(launch_propagate(c, c->rmat, ne, t0 + 1, t1, true));
     if (t1 < nt) PQMC_TRY(house_qr(s, ns, ne, c->rmat, c->tau, c->dtmp));

@@ -10,6 +10,7 @@
 #include "chain.cuh"
 #include "linalg.cuh"
 #include "rng.cuh"
+#include "wrap.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -26,8 +27,6 @@ void set_error(const char* fmt, ...) {
   va_end(ap);
   t_err = buf;
 }
-
-static __device__ __forceinline__ cplx ldg_c(const cplx* p) { return __ldcg(p); }
 
 // ---------------------------------------------------------------------------
 // init_expKV for every (family, plaquette, slice) (mod_phonon_field.f90:423-450)
@@ -69,54 +68,18 @@ int launch_init_expkv(pqmc_chain* c, int t0, int nt) {
 // Two-way wrap of G by one family (left_evolve/right_evolve with two_way,
 // src/mod_evolution.f90:236-328): out(Sr,Sc) = A_r G(Sr,Sc) B_c over all
 // pairs of cover items; left: A = expKV, B = expKV_inv; right: swapped.
-__global__ void k_wrap(DevModel M, int pf, int t, int left, int n_items, const int* __restrict__ ipla,
-                       const int* __restrict__ isites, const int* __restrict__ idim,
-                       const cplx* __restrict__ expkv, const cplx* __restrict__ expkv_inv,
-                       const cplx* __restrict__ gin, cplx* __restrict__ gout) {
-  const long pair = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (pair >= (long)n_items * n_items) return;
-  const int ir = (int)(pair % n_items), ic = (int)(pair / n_items);
-  const int ns = M.ns, pd = M.pdim;
-  const int dr = idim[ir], dc = idim[ic];
-  int Sr[4], Sc[4];
-  for (int k = 0; k < dr; ++k) Sr[k] = isites[4 * ir + k];
-  for (int k = 0; k < dc; ++k) Sc[k] = isites[4 * ic + k];
-  cplx g[16], h[16];
-  for (int b = 0; b < dc; ++b)
-    for (int a = 0; a < dr; ++a) g[a + 4 * b] = gin[Sr[a] + (size_t)ns * Sc[b]];
-  const int pr = ipla[ir], pc = ipla[ic];
-  const cplx* A = (pr >= 0) ? (left ? expkv : expkv_inv) + M.kv_base(pr, pf, t) : nullptr;
-  const cplx* B = (pc >= 0) ? (left ? expkv_inv : expkv) + M.kv_base(pc, pf, t) : nullptr;
-  for (int b = 0; b < dc; ++b)
-    for (int a = 0; a < dr; ++a) {
-      cplx s;
-      if (A) {
-        s = mk(0.0);
-        for (int k = 0; k < dr; ++k) s = cfma(A[a + pd * k], g[k + 4 * b], s);
-      } else {
-        s = g[a + 4 * b];
-      }
-      h[a + 4 * b] = s;
-    }
-  for (int b = 0; b < dc; ++b)
-    for (int a = 0; a < dr; ++a) {
-      cplx s;
-      if (B) {
-        s = mk(0.0);
-        for (int k = 0; k < dc; ++k) s = cfma(h[a + 4 * k], B[k + pd * b], s);
-      } else {
-        s = h[a + 4 * b];
-      }
-      gout[Sr[a] + (size_t)ns * Sc[b]] = s;
-    }
+// Arithmetic in wrap_pair (wrap.cuh), 16 lanes per pair.
+__global__ void __launch_bounds__(WRAP_THREADS) k_wrap(DevModel M, int pf, int t, int left, int n_items,
+                                                       const int* __restrict__ ipla, const int* __restrict__ isites,
+                                                       const int* __restrict__ idim, const cplx* __restrict__ expkv,
+                                                       const cplx* __restrict__ expkv_inv,
+                                                       const cplx* __restrict__ gin, cplx* __restrict__ gout) {
+  wrap_pair(M, pf, t, left, n_items, ipla, isites, idim, expkv, expkv_inv, gin, gout, (int)blockIdx.x);
 }
 
 int launch_wrap(pqmc_chain* c, int pf, int time, bool left) {
   const WrapItems& w = c->wrap[pf];
-  long pairs = (long)w.n_items * w.n_items;
-  int threads = 64;
-  int blocks = (int)((pairs + threads - 1) / threads);
-  k_wrap<<<blocks, threads, 0, c->stream>>>(c->M, pf, time - 1, left ? 1 : 0, w.n_items, w.d_pla, w.d_sites,
+  k_wrap<<<wrap_blocks(w.n_items), WRAP_THREADS, 0, c->stream>>>(c->M, pf, time - 1, left ? 1 : 0, w.n_items, w.d_pla, w.d_sites,
                                             w.d_dim, c->expkv, c->expkv_inv, c->g, c->g_alt);
   PQMC_LAUNCHED();
   cplx* t = c->g;
