@@ -193,6 +193,7 @@ extern "C" int pqmc_logweight_grad(pqmc_chain* c, double* logw_out, double* grad
     st = PQMC_ERR_CUDA;
   }
   if (st == PQMC_OK) info = h.lu_info;
+  if (st == PQMC_OK && h.lin_err != 0) st = check_factor(c, "logweight_grad");
   if (st == PQMC_OK && info != 0) {
     set_error("logweight_grad: zero pivot %d", info);
     st = PQMC_ERR_SINGULAR;
@@ -220,15 +221,14 @@ extern "C" int pqmc_logweight_grad(pqmc_chain* c, double* logw_out, double* grad
     // left factor that pairs with R at tau = t0 is the checkpoint at t0
     const cplx* Xl = ck + (size_t)ns * ne * (t0 / ng);
     PQMC_TRY(zgemm(s, 'C', 'N', ne, ne, ns, mk(1.0), Xl, ns, c->rmat, ns, mk(0.0), c->pbp, ne));
-    PQMC_TRY(lu_factor(s, ne, c->pbp, c->ipiv, &c->sc->lu_info, c->lcol));
     PQMC_TRY(herm_t(s, ns, ne, Xl, c->lmat));
-    PQMC_TRY(lu_solve(s, ne, ns, c->pbp, c->ipiv, c->lmat, ne));
+    PQMC_TRY(lu_solve(s, ne, c->pbp, ns, c->lmat, ne, c->lcol, c->ipiv, &c->sc->lu_info, c->g_alt, &c->sc->lin_err));
     PQMC_TRY(zgemm(s, 'N', 'N', ns, ns, ne, mk(1.0), c->rmat, ns, c->lmat, ne, mk(0.0), c->g, ns));
     for (int tau = t0 + 1; tau <= t1; ++tau) {
       for (int pf = 0; pf < c->n_pf; ++pf) PQMC_TRY(launch_grad_wrap(c, pf, tau, grad_dev, scale));
     }
     PQMC_TRY(launch_propagate(c, c->rmat, ne, t0 + 1, t1, true));
-    if (t1 < nt) PQMC_TRY(house_qr(s, ns, ne, c->rmat, c->tau, c->dtmp));
+    if (t1 < nt) PQMC_TRY(house_qr(s, ns, ne, c->rmat, c->dtmp, c->g_alt, &c->sc->lin_err));
   }
   // restore the chain's Green's function
   c->g = gsave;
@@ -236,6 +236,8 @@ extern "C" int pqmc_logweight_grad(pqmc_chain* c, double* logw_out, double* grad
   PQMC_CUDA(cudaMemcpyAsync(c->g, gtmp, sizeof(cplx) * (size_t)ns * ns, cudaMemcpyDeviceToDevice, s));
   PQMC_CUDA(cudaFreeAsync(gtmp, s));
   PQMC_CUDA(cudaFreeAsync(ck, s));
+  int late = 0;
+  PQMC_CUDA(cudaMemcpyAsync(&late, &c->sc->lin_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   PQMC_CUDA(cudaStreamSynchronize(s));
-  return PQMC_OK;
+  return late ? check_factor(c, "logweight_grad") : PQMC_OK;
 }

@@ -4,6 +4,7 @@
 // (:46-195, :330-408) and the C-ABI that replaces those subroutines.
 #include <cooperative_groups.h>
 #include <stdarg.h>
+#include <stddef.h>
 #include <string.h>
 #include <mutex>
 #include <string>
@@ -266,17 +267,35 @@ __global__ void k_scalars_zero(DevScalars* sc) {
   sc->sumlogd = mk(0.0);
 }
 
+// waits for the stream and reports a zero pivot or a wait that ran out inside
+// a factorisation
+int check_factor(pqmc_chain* c, const char* what) {
+  int h[2] = {0, 0};
+  static_assert(offsetof(DevScalars, lin_err) == offsetof(DevScalars, lu_info) + sizeof(int), "read back together");
+  PQMC_CUDA(cudaMemcpyAsync(h, &c->sc->lu_info, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+  PQMC_CUDA(cudaStreamSynchronize(c->stream));
+  if (h[1] != 0) {
+    PQMC_CUDA(cudaMemsetAsync(&c->sc->lin_err, 0, sizeof(int), c->stream));
+    set_error("%s: a wait inside a factorisation ran out", what);
+    return h[1];
+  }
+  if (h[0] != 0) {
+    set_error("%s: zero pivot %d", what, h[0]);
+    return PQMC_ERR_SINGULAR;
+  }
+  return PQMC_OK;
+}
+
 // cal_g_and_det_T0 with the left factor held as X = lmat^H (Ns x nelec)
 static int cal_g_and_det(pqmc_chain* c, const cplx* X, const cplx* R, bool compare) {
   const int ns = c->ns, ne = c->nelec;
   cudaStream_t s = c->stream;
   PQMC_TRY(zgemm(s, 'C', 'N', ne, ne, ns, mk(1.0), X, ns, R, ns, mk(0.0), c->pbp, ne));
-  PQMC_TRY(lu_factor(s, ne, c->pbp, c->ipiv, &c->sc->lu_info, c->lcol));
-  PQMC_TRY(lu_logdet(s, ne, c->pbp, c->ipiv, &c->sc->logdet));
+  PQMC_TRY(herm_t(s, ns, ne, X, c->lmat));
+  PQMC_TRY(lu_solve(s, ne, c->pbp, ns, c->lmat, ne, c->lcol, c->ipiv, &c->sc->lu_info, c->g_alt, &c->sc->lin_err));
+  PQMC_TRY(lu_logdet(s, ne, c->lcol, c->ipiv, &c->sc->logdet));
   k_sumvec<<<1, 32, 0, s>>>(c->nblock, c->d_logsum, &c->sc->sumlogd);
   PQMC_LAUNCHED();
-  PQMC_TRY(herm_t(s, ns, ne, X, c->lmat));
-  PQMC_TRY(lu_solve(s, ne, ns, c->pbp, c->ipiv, c->lmat, ne));
   PQMC_TRY(zgemm(s, 'N', 'N', ns, ns, ne, mk(1.0), R, ns, c->lmat, ne, mk(0.0), c->g_alt, ns));
   if (compare) {
     double* e = reinterpret_cast<double*>(c->lcol);   // scratch scalar
@@ -291,14 +310,7 @@ static int cal_g_and_det(pqmc_chain* c, const cplx* X, const cplx* R, bool compa
   cplx* t = c->g;
   c->g = c->g_alt;
   c->g_alt = t;
-  int info = 0;
-  PQMC_CUDA(cudaMemcpyAsync(&info, &c->sc->lu_info, sizeof(int), cudaMemcpyDeviceToHost, s));
-  PQMC_CUDA(cudaStreamSynchronize(s));
-  if (info != 0) {
-    set_error("cal_g_and_det: zero pivot %d in P^H B P", info);
-    return PQMC_ERR_SINGULAR;
-  }
-  return PQMC_OK;
+  return check_factor(c, "cal_g_and_det");
 }
 
 static inline cplx* Qblk(pqmc_chain* c, int blk1) {  // 1-based block
@@ -335,7 +347,7 @@ int do_init_g(pqmc_chain* c, int start_time) {
     PQMC_TRY(launch_propagate(c, c->rmat, ne, p, end, true));
     if (end % c->ngroup == 0) {
       int blk = (end - 1) / c->ngroup + 2;
-      PQMC_TRY(house_qr(s, ns, ne, c->rmat, c->tau, Dblk(c, blk)));
+      PQMC_TRY(house_qr(s, ns, ne, c->rmat, Dblk(c, blk), c->g_alt, &c->sc->lin_err));
       PQMC_TRY(block_log(c, blk));
       PQMC_CUDA(cudaMemcpyAsync(Qblk(c, blk), c->rmat, qb, cudaMemcpyDeviceToDevice, s));
     }
@@ -362,7 +374,7 @@ int do_g_scratch(pqmc_chain* c, int time, bool forward, int loop) {
     if (blk < 2 || blk + 1 > c->nblock) { set_error("g_scratch: block %d out of range", blk); return PQMC_ERR_ARG; }
     PQMC_CUDA(cudaMemcpyAsync(c->rmat, Qblk(c, blk - 1), qb, cudaMemcpyDeviceToDevice, s));
     PQMC_TRY(launch_propagate(c, c->rmat, ne, time - c->ngroup, time - 1, true));
-    PQMC_TRY(house_qr(s, ns, ne, c->rmat, c->tau, Dblk(c, blk)));
+    PQMC_TRY(house_qr(s, ns, ne, c->rmat, Dblk(c, blk), c->g_alt, &c->sc->lin_err));
     PQMC_TRY(block_log(c, blk));
     PQMC_CUDA(cudaMemcpyAsync(Qblk(c, blk), c->rmat, qb, cudaMemcpyDeviceToDevice, s));
     return cal_g_and_det(c, Qblk(c, blk + 1), c->rmat, true);
@@ -372,7 +384,7 @@ int do_g_scratch(pqmc_chain* c, int time, bool forward, int loop) {
   if (blk < 2 || blk + 1 > c->nblock) { set_error("g_scratch: block %d out of range", blk); return PQMC_ERR_ARG; }
   PQMC_CUDA(cudaMemcpyAsync(c->xmat, Qblk(c, blk + 1), qb, cudaMemcpyDeviceToDevice, s));
   PQMC_TRY(launch_propagate(c, c->xmat, ne, time + c->ngroup - 1, time, false));
-  PQMC_TRY(house_qr(s, ns, ne, c->xmat, c->tau, Dblk(c, blk)));
+  PQMC_TRY(house_qr(s, ns, ne, c->xmat, Dblk(c, blk), c->g_alt, &c->sc->lin_err));
   PQMC_TRY(block_log(c, blk));
   PQMC_CUDA(cudaMemcpyAsync(Qblk(c, blk), c->xmat, qb, cudaMemcpyDeviceToDevice, s));
   return cal_g_and_det(c, c->xmat, Qblk(c, blk - 1), true);
@@ -392,7 +404,7 @@ int do_new_weight(pqmc_chain* c) {
     int lo = p - c->ngroup + 1;
     if (lo >= 1) {
       PQMC_TRY(launch_propagate(c, c->xmat, ne, p, lo, false));
-      PQMC_TRY(house_qr(s, ns, ne, c->xmat, c->tau, c->dtmp));
+      PQMC_TRY(house_qr(s, ns, ne, c->xmat, c->dtmp, c->g_alt, &c->sc->lin_err));
       k_sumlog<<<1, 256, 0, s>>>(ne, c->dtmp, &c->sc->sumlogd, 1);
       PQMC_LAUNCHED();
       p = lo - 1;
@@ -404,15 +416,11 @@ int do_new_weight(pqmc_chain* c) {
   k_sumlog<<<1, 256, 0, s>>>(ne, Dblk(c, 1), &c->sc->sumlogd, 1);
   PQMC_LAUNCHED();
   PQMC_TRY(zgemm(s, 'C', 'N', ne, ne, ns, mk(1.0), c->xmat, ns, Qblk(c, 1), ns, mk(0.0), c->pbp, ne));
-  PQMC_TRY(lu_factor(s, ne, c->pbp, c->ipiv, &c->sc->lu_info, c->lcol));
-  PQMC_TRY(lu_logdet(s, ne, c->pbp, c->ipiv, &c->sc->logdet));
+  PQMC_TRY(lu_solve(s, ne, c->pbp, 0, nullptr, ne, c->lcol, c->ipiv, &c->sc->lu_info, c->g_alt, &c->sc->lin_err));
+  PQMC_TRY(lu_logdet(s, ne, c->lcol, c->ipiv, &c->sc->logdet));
   k_finish_weight<<<1, 1, 0, s>>>(c->sc, c->M.tr_weight, c->M.ncopy, 0);
   PQMC_LAUNCHED();
-  int info = 0;
-  PQMC_CUDA(cudaMemcpyAsync(&info, &c->sc->lu_info, sizeof(int), cudaMemcpyDeviceToHost, s));
-  PQMC_CUDA(cudaStreamSynchronize(s));
-  if (info != 0) { set_error("cal_new_weight: zero pivot %d", info); return PQMC_ERR_SINGULAR; }
-  return PQMC_OK;
+  return check_factor(c, "cal_new_weight");
 }
 
 // cal_new_weight_T0 of the current field from the trial state alone (no
@@ -432,7 +440,7 @@ int do_new_weight_ck(pqmc_chain* c, cplx* ck) {
   for (int p = nt; p >= 1;) {
     const int lo = ((p - 1) / ng) * ng + 1;   // slices [lo, p]
     PQMC_TRY(launch_propagate(c, c->xmat, ne, p, lo, false));
-    PQMC_TRY(house_qr(s, ns, ne, c->xmat, c->tau, c->dtmp));
+    PQMC_TRY(house_qr(s, ns, ne, c->xmat, c->dtmp, c->g_alt, &c->sc->lin_err));
     k_sumlog<<<1, 256, 0, s>>>(ne, c->dtmp, &c->sc->sumlogd, 1);
     PQMC_LAUNCHED();
     PQMC_CUDA(cudaMemcpyAsync(ck + (size_t)ns * ne * ((lo - 1) / ng), c->xmat, qb, cudaMemcpyDeviceToDevice, s));
@@ -441,8 +449,8 @@ int do_new_weight_ck(pqmc_chain* c, cplx* ck) {
   k_sumlog<<<1, 256, 0, s>>>(ne, c->slater_d, &c->sc->sumlogd, 1);
   PQMC_LAUNCHED();
   PQMC_TRY(zgemm(s, 'C', 'N', ne, ne, ns, mk(1.0), c->xmat, ns, c->slater_q, ns, mk(0.0), c->pbp, ne));
-  PQMC_TRY(lu_factor(s, ne, c->pbp, c->ipiv, &c->sc->lu_info, c->lcol));
-  PQMC_TRY(lu_logdet(s, ne, c->pbp, c->ipiv, &c->sc->logdet));
+  PQMC_TRY(lu_solve(s, ne, c->pbp, 0, nullptr, ne, c->lcol, c->ipiv, &c->sc->lu_info, c->g_alt, &c->sc->lin_err));
+  PQMC_TRY(lu_logdet(s, ne, c->lcol, c->ipiv, &c->sc->logdet));
   k_finish_weight<<<1, 1, 0, s>>>(c->sc, c->M.tr_weight, c->M.ncopy, 0);
   PQMC_LAUNCHED();
   return PQMC_OK;
@@ -547,7 +555,6 @@ int chain_alloc(pqmc_chain* c, const pqmc_model* m, cudaStream_t s) {
   PQMC_TRY(dalloc(&c->xmat, (size_t)c->ns * c->nelec));
   PQMC_TRY(dalloc(&c->lmat, (size_t)c->ns * c->nelec));
   PQMC_TRY(dalloc(&c->pbp, (size_t)c->nelec * c->nelec));
-  PQMC_TRY(dalloc(&c->tau, (size_t)c->nelec));
   PQMC_TRY(dalloc(&c->dtmp, (size_t)c->nelec));
   PQMC_TRY(dalloc(&c->lcol, (size_t)c->nelec + 2));
   PQMC_TRY(dalloc(&c->ipiv, (size_t)c->nelec));
@@ -615,7 +622,7 @@ int chain_alloc(pqmc_chain* c, const pqmc_model* m, cudaStream_t s) {
 int chain_free(pqmc_chain* c) {
   ft_free(c);
   void* ptrs[] = {c->d_logsum, c->pre, c->d_model_blob, c->field, c->expkv, c->expkv_inv, c->g, c->g_alt, c->q_string, c->d_string,
-                  c->slater_q, c->slater_d, c->rmat, c->xmat, c->lmat, c->pbp, c->tau, c->dtmp, c->lcol,
+                  c->slater_q, c->slater_d, c->rmat, c->xmat, c->lmat, c->pbp, c->dtmp, c->lcol,
                   c->ipiv, c->ctl, c->sc, c->m_cell_sites, c->m_cell_bf, c->m_cell_xnb, c->m_cell_ynb,
                   c->m_cell_cross, c->m_c2_of, c->m_kphase, c->m_acc, c->m_gtmp};
   for (void* p : ptrs)

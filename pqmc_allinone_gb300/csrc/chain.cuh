@@ -23,8 +23,8 @@ struct DevScalars {
   long long neg_acc;
   int rng[5];
   int lu_info;
+  int lin_err;          // a wait inside a factorisation ran out (PQMC_ERR_TIMEOUT)
   int status;
-  int pad;
 };
 
 // Control record the proposer publishes at every grid barrier of the update
@@ -84,7 +84,6 @@ struct pqmc_chain {
   cplx* xmat = nullptr;             // (Ns,nelec) left factor, adjoint layout
   cplx* lmat = nullptr;             // (nelec,Ns)
   cplx* pbp = nullptr;              // (nelec,nelec)
-  cplx* tau = nullptr;              // (nelec)
   cplx* dtmp = nullptr;             // (nelec)
   cplx* lcol = nullptr;             // (nelec)
   int* ipiv = nullptr;              // (nelec)
@@ -139,6 +138,7 @@ int launch_init_expkv(pqmc_chain* c, int t0, int nt);
 int launch_update(pqmc_chain* c, int pf, int time);
 int update_setup(pqmc_chain* c);
 int launch_wrap(pqmc_chain* c, int pf, int time, bool left);
+int check_factor(pqmc_chain* c, const char* what);
 int launch_propagate(pqmc_chain* c, cplx* X, int n, int t_from, int t_to, bool forward);
 int do_init_g(pqmc_chain* c, int start_time);
 int do_g_scratch(pqmc_chain* c, int time, bool forward, int loop);

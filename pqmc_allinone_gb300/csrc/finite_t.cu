@@ -50,7 +50,6 @@ struct FtState {
   cplx* qa = nullptr;    // cal_new_weight's own string
   cplx* ra = nullptr;
   cplx* da = nullptr;
-  cplx* tau = nullptr;   // (Ns)
   cplx* dtmp = nullptr;
   cplx* lcol = nullptr;
   cplx* scal = nullptr;  // [0] ln det M, [1] sum ln Dr_gt, [2] sum ln Dl_gt, [3] ln det Q of qa
@@ -247,7 +246,7 @@ static int ft_step(pqmc_chain* c, const cplx* qin, const cplx* din, const cplx* 
   PQMC_LAUNCHED();
   k_ft_gather_cols<<<n, 128, 0, s>>>(n, f.x, f.perm, f.y);
   PQMC_LAUNCHED();
-  PQMC_TRY(house_qr_r(s, n, n, f.y, f.tau, f.dtmp, f.t1, lnq_out));
+  PQMC_TRY(house_qr_r(s, n, n, f.y, f.dtmp, f.t1, lnq_out, c->g_alt, &c->sc->lin_err));
   k_ft_rdiag<<<(n + 127) / 128, 128, 0, s>>>(n, f.t1, dout);
   PQMC_LAUNCHED();
   k_ft_rscale<<<ew_grid((long)n * n), 256, 0, s>>>(n, f.t1, dout);
@@ -273,17 +272,19 @@ static int ft_cal_g_and_det(pqmc_chain* c, const cplx* x, const cplx* dl, const 
   PQMC_TRY(zgemm(s, 'N', 'C', n, n, n, mk(1.0), rr, n, y, n, mk(0.0), f.t2, n));   // R_r Y^H
   k_ft_mix<<<ew_grid(nn), 256, 0, s>>>(n, f.t1, f.t2, dl, dr);
   PQMC_LAUNCHED();
-  PQMC_TRY(lu_factor(s, n, f.t1, f.ipiv, &c->sc->lu_info, f.lcol));
-  PQMC_TRY(lu_logdet(s, n, f.t1, f.ipiv, f.scal));
+  if (cal_g) {
+    PQMC_TRY(herm_t(s, n, n, qr, f.t2));                                        // Q_r^H
+    k_ft_rowdiv_gt<<<ew_grid(nn), 256, 0, s>>>(n, f.t2, dr);
+    PQMC_LAUNCHED();
+  }
+  // M^-1 Dr_gt^-1 Q_r^H beside the factorisation
+  PQMC_TRY(lu_solve(s, n, f.t1, cal_g ? n : 0, f.t2, n, f.lcol, f.ipiv, &c->sc->lu_info, c->g_alt, &c->sc->lin_err));
+  PQMC_TRY(lu_logdet(s, n, f.lcol, f.ipiv, f.scal));
   k_ft_sumlog_gt<<<1, 256, 0, s>>>(n, dr, dl, f.scal + 1);
   PQMC_LAUNCHED();
   k_ft_lnparts<<<1, 1, 0, s>>>(c->sc, f.scal, lnq_r, lnq_l);
   PQMC_LAUNCHED();
   if (cal_g) {
-    PQMC_TRY(herm_t(s, n, n, qr, f.t2));                                        // Q_r^H
-    k_ft_rowdiv_gt<<<ew_grid(nn), 256, 0, s>>>(n, f.t2, dr);
-    PQMC_LAUNCHED();
-    PQMC_TRY(lu_solve(s, n, n, f.t1, f.ipiv, f.t2, n));                         // M^-1 Dr_gt^-1 Q_r^H
     k_ft_rowdiv_gt<<<ew_grid(nn), 256, 0, s>>>(n, f.t2, dl);
     PQMC_LAUNCHED();
     PQMC_TRY(zgemm(s, 'N', 'N', n, n, n, mk(1.0), x, n, f.t2, n, mk(0.0), c->g_alt, n));
@@ -305,14 +306,7 @@ static int ft_cal_g_and_det(pqmc_chain* c, const cplx* x, const cplx* dl, const 
     c->g = c->g_alt;
     c->g_alt = t;
   }
-  int info = 0;
-  PQMC_CUDA(cudaMemcpyAsync(&info, &c->sc->lu_info, sizeof(int), cudaMemcpyDeviceToHost, s));
-  PQMC_CUDA(cudaStreamSynchronize(s));
-  if (info != 0) {
-    set_error("cal_g_and_det_FT: zero pivot %d in the scale-separated middle matrix", info);
-    return PQMC_ERR_SINGULAR;
-  }
-  return PQMC_OK;
+  return check_factor(c, "cal_g_and_det_FT");
 }
 
 static int ft_identity_block(pqmc_chain* c, int b) {
@@ -406,7 +400,7 @@ static int ft_alloc(T** p, size_t n) {
 int ft_free(pqmc_chain* c) {
   if (!c->ft) return PQMC_OK;
   FtState& f = *c->ft;
-  void* ptrs[] = {f.q, f.r, f.d, f.lnq, f.x, f.y, f.t1, f.t2, f.qa, f.ra, f.da, f.tau, f.dtmp, f.lcol, f.scal,
+  void* ptrs[] = {f.q, f.r, f.d, f.lnq, f.x, f.y, f.t1, f.t2, f.qa, f.ra, f.da, f.dtmp, f.lcol, f.scal,
                   f.ipiv, f.perm, f.norm};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -434,7 +428,6 @@ static int ft_setup(pqmc_chain* c) {
   for (cplx** w : work)
     if (st == PQMC_OK) st = ft_alloc(w, nn);
   if (st == PQMC_OK) st = ft_alloc(&f.da, n);
-  if (st == PQMC_OK) st = ft_alloc(&f.tau, n);
   if (st == PQMC_OK) st = ft_alloc(&f.dtmp, n);
   if (st == PQMC_OK) st = ft_alloc(&f.lcol, n + 2);
   if (st == PQMC_OK) st = ft_alloc(&f.scal, 4);

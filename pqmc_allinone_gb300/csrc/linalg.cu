@@ -1,14 +1,12 @@
 // linalg.cu -- FP64 complex dense kernels for the stabilisation path:
 // GEMM, Householder QR with Q formation (zgeqrf/zungqr conventions), LU with
-// partial pivoting (zgetf2 conventions), multi-RHS LU solve and log-det.
+// partial pivoting (zgetf2's pivots) with the right-hand sides solved in the
+// same pass, and log-det.
 //
 // GB300 runs FP64 at a small fraction of its FP32 rate, so every routine
 // spreads its work over all SMs: the factorisations are cooperative kernels
-// (one grid barrier per elimination stage), the products are tiled GEMMs.
-#include <cooperative_groups.h>
+// that pipeline over columns, the products are tiled GEMMs.
 #include "linalg.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace pqmc {
 
@@ -78,300 +76,547 @@ int zgemm(cudaStream_t s, char ta, char tb, int m, int n, int k, cplx alpha, con
 }
 
 // ---------------------------------------------------------------------------
-// block-wide sum of a double (all threads get the result)
-__device__ __forceinline__ double block_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  double t = (threadIdx.x < nw) ? red[threadIdx.x] : 0.0;
-  if (w == 0)
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (threadIdx.x == 0) red[32] = t;
-  __syncthreads();
-  double r = red[32];
-  __syncthreads();
-  return r;
+// Column pipeline shared by the two factorisations.  Columns are dealt out to
+// CTAs of 128 threads (a warp on each SM quarter) and stay in shared memory;
+// the CTA that finishes a column publishes it once in the work matrix `pub`,
+// which starts out filled with a bit pattern no published value has, and the
+// others poll the very words they need: a published value is its own flag,
+// so a step costs one L2 round trip and no grid barrier.  The launch is
+// cooperative (every CTA resident); every poll is bounded.
+constexpr int LT = 128;
+constexpr unsigned long long LA_EMPTY = ~0ull;   // memset 0xff; a NaN pattern publish() never writes
+
+__device__ __forceinline__ void publish(cplx* p, cplx v) {
+  unsigned long long x = (unsigned long long)__double_as_longlong(v.x), y = (unsigned long long)__double_as_longlong(v.y);
+  if (x == LA_EMPTY) x = 0x7ff8000000000000ull;
+  if (y == LA_EMPTY) y = 0x7ff8000000000000ull;
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
 }
 
-// block-wide max of a double (all threads get the result)
-__device__ __forceinline__ double block_max(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  double t = (threadIdx.x < nw) ? red[threadIdx.x] : 0.0;
-  if (w == 0)
-    for (int o = 16; o > 0; o >>= 1) t = fmax(t, __shfl_xor_sync(0xffffffffu, t, o));
-  if (threadIdx.x == 0) red[32] = t;
-  __syncthreads();
-  double r = red[32];
-  __syncthreads();
-  return r;
+// rows k >= k0 with k % LT == threadIdx.x of a published column into dst, as
+// they arrive.  False when a word did not come in ~2 s.
+__device__ __forceinline__ bool poll_col(const cplx* src, cplx* dst, int k0, int m) {
+  const long long t0 = clock64();
+  for (int k = k0 + (((int)threadIdx.x - k0) & (LT - 1)); k < m; k += 4 * LT) {
+    unsigned need = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (k + e * LT < m) need |= 1u << e;
+    while (need) {
+      unsigned long long x[4], y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (need >> e & 1u)
+          asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                       : "=l"(x[e]), "=l"(y[e])
+                       : "l"(src + k + e * LT)
+                       : "memory");
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if ((need >> e & 1u) && x[e] != LA_EMPTY && y[e] != LA_EMPTY) {
+          dst[k + e * LT] = mk(__longlong_as_double((long long)x[e]), __longlong_as_double((long long)y[e]));
+          need &= ~(1u << e);
+        }
+      if (need && clock64() - t0 > (4LL << 30)) return false;
+    }
+  }
+  return true;
 }
 
-__device__ __forceinline__ cplx block_csum(cplx v, double* red) {
-  double re = block_sum(v.x, red);
-  double im = block_sum(v.y, red);
-  return mk(re, im);
+// own rows k >= k0 (k % LT == threadIdx.x) of a column whose words this thread
+// has seen published (or published itself), asynchronously
+__device__ __forceinline__ void fetch_col(const cplx* src, cplx* dst, int k0, int m) {
+  for (int k = k0 + (((int)threadIdx.x - k0) & (LT - 1)); k < m; k += LT)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + k)),
+                 "l"(src + k)
+                 : "memory");
+}
+__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// sums of four doubles over the CTA, to every thread, with one barrier and 8
+// FP64 additions in a row (lanes take over one of the four values as the
+// tree narrows; 20 + 12 for four plain trees).  red: [2][4][4], the half
+// alternates from call to call.  The order is the same in every CTA.
+__device__ __forceinline__ void cta_sum4(double& a, double& b, double& c, double& d, double (*red)[4][4], int& half) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool up = lane & 16, u8 = lane & 8;
+  double k0 = up ? c : a, k1 = up ? d : b;
+  k0 += __shfl_xor_sync(full, up ? a : c, 16);
+  k1 += __shfl_xor_sync(full, up ? b : d, 16);
+  double k = u8 ? k1 : k0;
+  k += __shfl_xor_sync(full, u8 ? k0 : k1, 8);
+  k += __shfl_xor_sync(full, k, 4);
+  k += __shfl_xor_sync(full, k, 2);
+  k += __shfl_xor_sync(full, k, 1);
+  if ((lane & 7) == 0) red[half][lane >> 3][warp] = k;
+  __syncthreads();
+  double r = red[half][(lane >> 2) & 3][lane & 3];
+  r += __shfl_xor_sync(full, r, 1);
+  r += __shfl_xor_sync(full, r, 2);
+  a = __shfl_sync(full, r, 0);
+  b = __shfl_sync(full, r, 4);
+  c = __shfl_sync(full, r, 8);
+  d = __shfl_sync(full, r, 12);
+  half ^= 1;
+}
+
+// power of two as a double, |e| <= 1022
+__device__ __forceinline__ double pow2i(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
+// biased exponent of the larger component
+__device__ __forceinline__ int top_exp(cplx v) {
+  return max((__double2hiint(v.x) & 0x7fffffff) >> 20, (__double2hiint(v.y) & 0x7fffffff) >> 20);
+}
+// the CTA's largest v >= 0 to every thread (two barriers)
+__device__ __forceinline__ int cta_max(int v, int* red) {
+  v = __reduce_max_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = max(max(red[0], red[1]), max(red[2], red[3]));
+  __syncthreads();
+  return v;
+}
+
+// zlarfg for the column [alpha; x], ss = sum |x|^2, kept as the vector
+// u = [z; x], z = alpha - beta, that is z times zlarfg's v: then
+// H^H = I + c u u^H with c = 1/(beta z), and tau = -z/beta.  One square root
+// and one division, and two products fewer in a step's chain than with v.
+struct Reflector {
+  cplx z, c;
+  double beta;
+};
+__device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2) {   // n2 = |alpha|^2 + ss
+  Reflector h;
+  // signs and zeros are looked at as bits: an FP64 comparison costs what a multiplication costs
+  const long long sign = ~__double_as_longlong(alpha.x) & (1ll << 63);
+  h.beta = __longlong_as_double(__double_as_longlong(sqrt(n2)) | sign);
+  h.z = mk(alpha.x - h.beta, alpha.y);
+  const double den = h.beta * fma(h.z.x, h.z.x, h.z.y * h.z.y);
+  const double r = ((threadIdx.x & 1) ? -h.z.y : h.z.x) / den;   // both components in one division
+  h.c = mk(__shfl_sync(0xffffffffu, r, 0), __shfl_sync(0xffffffffu, r, 1));
+  if (__double_as_longlong(ss) == 0 && (__double_as_longlong(alpha.y) << 1) == 0) {   // nothing below the diagonal: H = I
+    h.z = h.c = mk(0.0);
+    h.beta = alpha.x;
+  }
+  return h;
 }
 
 // ---------------------------------------------------------------------------
-// Householder QR in place (zgeqr2): column i reflector by block 0, then every
-// block applies H_i^H to its share of the trailing columns.  Then Q formation
-// (zung2r).  A is m x n (lda = m), m >= n.  d receives diag(R) (real in the
-// LAPACK convention).  Matches zqdr (src/mod_matrixlib.f90:323-334) with the
-// unit-diagonal R discarded as the reference does for the hot path.  With
-// Rout the upper triangle of R (n x n, diagonal = d) is copied out before Q
-// is formed, and with lndet ln det Q = sum over the reflectors of
-// ln det(I - tau v v^H) = ln(-tau / conj(tau)) (a phase; 0 for tau = 0).
-// scaled: the reflector norms are taken as max |x| * |x / max|, as LAPACK's
-// dznrm2 avoids overflow, for columns whose entries pass 1e154 (the graded
-// finite-temperature strings); the projector path keeps the plain sum.
-__global__ void __launch_bounds__(256) k_house_qr(int m, int n, cplx* A, cplx* tau, cplx* d, cplx* Rout,
-                                                  cplx* lndet, int scaled) {
-  cg::grid_group grid = cg::this_grid();
-  __shared__ double red[33];
+// Householder QR in place with Q formed (zgeqr2 + zung2r).  A is m x n
+// (lda = m), m >= n; d receives diag(R) (real in the LAPACK convention).
+// Matches zqdr (src/mod_matrixlib.f90:323-334) with the unit-diagonal R
+// discarded as the reference does for the hot path.  With Rout the upper
+// triangle of R (n x n, diagonal = d) is written too, and with lndet
+// ln det Q = sum over the reflectors of ln det(I - tau v v^H)
+// = ln(-z / conj(z)) (a phase; 0 for z = 0).
+//
+// What is published is the raw column (rows >= i after the reflectors before
+// it), so its norm is off the critical path: every CTA forms it beside its
+// own dot product, and the chain of a step is one poll, one reduction, a
+// square root, a division and the update of the next column, which its CTA
+// publishes before it turns to its others.  Q's columns need only reflectors
+// that their CTA has already seen, so their formation starts without waiting
+// for the rest.  Bound by that chain (n steps) and, in a step, by the FP64
+// pipe.  A column whose entries pass 2^+-256 is held times a power of two
+// (exact), and a remainder whose squares could vanish is scaled up before its
+// norm is taken, as LAPACK's dznrm2 avoids overflow (the graded
+// finite-temperature strings pass 1e154).
+//
+// dynamic shared memory: nst columns of the ring, z and c of n reflectors, the local columns' exponents, the local columns if `in_smem`
+// (else they stay in A).
+__global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d, cplx* Rout, cplx* lndet, cplx* pub,
+                                                 int in_smem, int nst, int* err) {
+  extern __shared__ cplx qr_dyn[];
+  __shared__ double red[2][4][4];
+  __shared__ int redi[4];
+  __shared__ cplx s_al[2], s_aj[2][2];
+  __shared__ int s_fail;
+  const int tid = threadIdx.x, b = blockIdx.x, G = gridDim.x;
+  const int nl = (n - b + G - 1) / G;   // local columns b, b + G, ...
+  cplx* xs = qr_dyn;
+  cplx* s_z = xs + (size_t)nst * m;
+  cplx* s_c = s_z + n;
+  double* s_up = reinterpret_cast<double*>(s_c + n);   // power of two on x (1 but for vanishing remainders)
+  int* s_exp = reinterpret_cast<int*>(s_up + 2 * ((n + 1) / 2));
+  cplx* cols = s_c + n + (n + 1) / 2 + (nl + 3) / 4;
+  auto col = [&](int l) { return in_smem ? cols + (size_t)l * m : A + (size_t)m * (b + (size_t)l * G); };
+  int half = 0;
+  if (tid == 0) s_fail = 0;
+  for (int l = 0; l < nl; ++l) {
+    const cplx* src = A + (size_t)m * (b + (size_t)l * G);
+    cplx* c = col(l);
+    int e = 0;
+    for (int k = tid; k < m; k += LT) {
+      const cplx v = src[k];
+      e = max(e, top_exp(v));
+      if (in_smem) c[k] = v;
+    }
+    e = cta_max(e, redi) - 1023;
+    e = (e < -256 || e > 256) ? min(max(e, -1000), 1000) : 0;
+    if (e)
+      for (int k = tid; k < m; k += LT) c[k] = cscale(c[k], pow2i(-e));
+    if (tid == 0) s_exp[l] = e;
+  }
+  __syncthreads();
+  if (b == 0)
+    for (int k = tid; k < m; k += LT) publish(pub + k, col(0)[k]);
+  int li = 0, jown = b;   // the next local column, local and global
   for (int i = 0; i < n; ++i) {
-    cplx* col = A + (size_t)m * i;
-    if (blockIdx.x == 0) {
-      // zlarfg on col[i..m-1]
-      double xnorm;
-      if (scaled) {
-        double mx = 0.0;
-        for (int k = i + 1 + threadIdx.x; k < m; k += blockDim.x) mx = fmax(mx, fmax(fabs(col[k].x), fabs(col[k].y)));
-        mx = block_max(mx, red);
-        double ss = 0.0;
-        if (mx > 0.0)
-          for (int k = i + 1 + threadIdx.x; k < m; k += blockDim.x) {
-            const double a = col[k].x / mx, b = col[k].y / mx;
-            ss += a * a + b * b;
-          }
-        xnorm = mx * sqrt(block_sum(ss, red));
-      } else {
-        double ss = 0.0;
-        for (int k = i + 1 + threadIdx.x; k < m; k += blockDim.x) ss += cabs2(col[k]);
-        xnorm = sqrt(block_sum(ss, red));
-      }
-      cplx alpha = col[i];
-      __shared__ cplx s_scale;
-      __shared__ double s_beta;
-      __shared__ int s_zero;
-      if (threadIdx.x == 0) {
-        if (xnorm == 0.0 && alpha.y == 0.0) {
-          tau[i] = mk(0.0);
-          s_zero = 1;
-          s_beta = alpha.x;
-        } else {
-          double w = fmax(fabs(alpha.x), fmax(fabs(alpha.y), xnorm));
-          double a1 = alpha.x / w, a2 = alpha.y / w, a3 = xnorm / w;
-          double nrm = w * sqrt(a1 * a1 + a2 * a2 + a3 * a3);
-          double beta = alpha.x >= 0.0 ? -nrm : nrm;
-          tau[i] = mk((beta - alpha.x) / beta, -alpha.y / beta);
-          s_scale = cdiv(mk(1.0), csub(alpha, mk(beta)));
-          s_beta = beta;
-          s_zero = 0;
-        }
-        d[i] = mk(s_beta);
-      }
-      __syncthreads();
-      if (!s_zero)
-        for (int k = i + 1 + threadIdx.x; k < m; k += blockDim.x) col[k] = cmul(s_scale, col[k]);
-      __syncthreads();
-      if (threadIdx.x == 0) col[i] = mk(s_beta);
+    const bool own = i == jown;
+    const int l0 = own ? li + 1 : li;   // first local column right of i
+    cplx* x = xs;
+    if (own) {
+      for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) x[k] = col(li)[k];
+    } else if (!poll_col(pub + (size_t)m * i, x, i, m)) {
+      s_fail = 1;
     }
-    grid.sync();
-    // apply H_i^H = I - conj(tau) v v^H to columns j > i; v = [1; col[i+1..]]
-    const cplx ct = cconj(tau[i]);
-    for (int j = i + 1 + blockIdx.x; j < n; j += gridDim.x) {
-      cplx* cj = A + (size_t)m * j;
-      cplx w = mk(0.0);
-      for (int k = i + threadIdx.x; k < m; k += blockDim.x) {
-        cplx v = (k == i) ? mk(1.0) : col[k];
-        w = cadd(w, cmulc(v, cj[k]));
+    const bool row_i = tid == (i & (LT - 1));
+    cplx* c0 = l0 < nl ? col(l0) : nullptr;
+    double ss = 0.0, zero = 0.0;
+    cplx w = mk(0.0);
+    for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) {
+      const cplx v = x[k];
+      ss = fma(v.x, v.x, fma(v.y, v.y, ss));
+      if (c0) w = cfma(cconj(v), c0[k], w);
+    }
+    const int h0 = half;
+    if (row_i) {
+      s_al[h0] = x[i];
+      if (c0) s_aj[h0][0] = c0[i];
+    }
+    cta_sum4(w.x, w.y, ss, zero, red, half);
+    if (s_fail) {
+      if (tid == 0) atomicExch(err, PQMC_ERR_TIMEOUT);
+      return;
+    }
+    const cplx alpha = s_al[h0], aj0 = c0 ? s_aj[h0][0] : mk(0.0);
+    Reflector h;
+    double up_x = 1.0, beta_x;
+    const double n2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
+    if (__double2hiint(n2) < (1023 - 664) << 20) {   // below 2^-664 squares may have vanished: scale up
+      int e = 0;
+      for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) e = max(e, top_exp(x[k]));
+      e = cta_max(e, redi);
+      const int up = e ? min(1023 - e, 1000) : 1000;
+      up_x = pow2i(up);
+      double s2 = 0.0, z1 = 0.0;
+      w = mk(0.0);
+      for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) {
+        const cplx v = cscale(x[k], up_x);
+        x[k] = v;
+        s2 += cabs2(v);
+        if (c0) w = cfma(cconj(v), c0[k], w);
       }
-      w = block_csum(w, red);
-      cplx f = cmul(ct, w);
-      for (int k = i + threadIdx.x; k < m; k += blockDim.x) {
-        cplx v = (k == i) ? mk(1.0) : col[k];
-        cj[k] = csub(cj[k], cmul(v, f));
+      cta_sum4(w.x, w.y, s2, z1, red, half);
+      const cplx al = cscale(alpha, up_x);
+      h = reflector(al, s2, s2 + cabs2(al));
+      beta_x = h.beta * pow2i(-up);
+    } else {
+      h = reflector(alpha, ss, n2);
+      beta_x = h.beta;
+    }
+    if (tid == 0) {
+      s_z[i] = h.z;
+      s_c[i] = h.c;
+      s_up[i] = up_x;
+    }
+    if (row_i) x[i] = h.z;   // u
+    // H_i^H on the local columns right of i, the next column first
+    for (int l = l0; l < nl; ++l) {
+      cplx* c = col(l);
+      cplx aj = aj0;
+      if (l != l0) {
+        w = mk(0.0);
+        double z1 = 0.0, z2 = 0.0;
+        for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) w = cfma(cconj(x[k]), c[k], w);
+        const int h1 = half;
+        if (row_i) s_aj[h1][0] = c[i];
+        cta_sum4(w.x, w.y, z1, z2, red, half);
+        aj = s_aj[h1][0];
+      }
+      const cplx f = cmul(h.c, cfma(cconj(h.z), aj, w));   // c u^H a
+      const bool next = l == l0 && (own ? jown + G : jown) == i + 1;
+      for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
+        const cplx v = cfma(x[k], f, c[k]);
+        c[k] = v;
+        if (next && k > i) publish(pub + (size_t)m * (i + 1) + k, v);
       }
     }
-    grid.sync();
+    if (own) {   // diag(R), R
+      const int e = s_exp[li];
+      const double up = pow2i(e);
+      if (tid == 0) d[i] = mk(beta_x * up);
+      if (Rout)
+        for (int k = tid; k < n; k += LT)
+          Rout[k + (size_t)n * i] = k < i ? cscale(col(li)[k], up) : k == i ? mk(beta_x * up) : mk(0.0);
+      if (l0 >= nl) break;
+      ++li;
+      jown += G;
+    }
   }
-  if (Rout) {
-    for (int j = blockIdx.x; j < n; j += gridDim.x)
-      for (int k = threadIdx.x; k < n; k += blockDim.x) Rout[k + (size_t)n * j] = k <= j ? A[k + (size_t)m * j] : mk(0.0);
-    grid.sync();
-  }
-  if (lndet && blockIdx.x == 0 && threadIdx.x == 0) {
-    double ph = 0.0;
-    for (int i = 0; i < n; ++i) {
-      const cplx t = tau[i];
+  __threadfence();
+  __syncthreads();
+  if (lndet && (n - 1) % G == b) {
+    double ph = 0.0, z1 = 0.0, z2 = 0.0, z3 = 0.0;
+    for (int i = tid; i < n; i += LT) {
+      const cplx t = s_z[i];
       if (t.x != 0.0 || t.y != 0.0) {
         const cplx z = cdiv(cneg(t), cconj(t));
         ph += atan2(z.y, z.x);
       }
     }
-    lndet[0] = mk(0.0, ph);
+    cta_sum4(ph, z1, z2, z3, red, half);
+    if (tid == 0) lndet[0] = mk(0.0, ph);
   }
-  // zung2r: Q = H_1 ... H_n applied to the first n unit columns
-  for (int i = n - 1; i >= 0; --i) {
-    cplx* col = A + (size_t)m * i;
-    const cplx t = tau[i];
-    for (int j = i + 1 + blockIdx.x; j < n; j += gridDim.x) {
-      cplx* cj = A + (size_t)m * j;
-      cplx w = mk(0.0);
-      for (int k = i + threadIdx.x; k < m; k += blockDim.x) {
-        cplx v = (k == i) ? mk(1.0) : col[k];
-        w = cadd(w, cmulc(v, cj[k]));
-      }
-      w = block_csum(w, red);
-      cplx f = cmul(t, w);
-      for (int k = i + threadIdx.x; k < m; k += blockDim.x) {
-        cplx v = (k == i) ? mk(1.0) : col[k];
-        cj[k] = csub(cj[k], cmul(v, f));
-      }
-    }
-    grid.sync();
-    if (blockIdx.x == (i % gridDim.x)) {
-      for (int k = threadIdx.x; k < m; k += blockDim.x) {
-        if (k > i) col[k] = cmul(cneg(t), col[k]);
-        else if (k == i) col[k] = csub(mk(1.0), t);
-        else col[k] = mk(0.0);
-      }
-    }
-    grid.sync();
+  // zung2r: column j of Q = H_1 ... H_j e_j, the local columns together; the
+  // published columns come back through the ring, nst - 1 steps ahead
+  const int jlast = b + (nl - 1) * G, ring = nst - 1;   // nst is 2 or 4
+  li = nl - 1;
+  jown = jlast;
+  for (int u = 1; u < nst; ++u) {
+    const int i = jlast - u;
+    if (i >= 0) fetch_col(pub + (size_t)m * i, xs + (size_t)(i & ring) * m, i, m);
+    fetch_commit();
   }
+  for (int i = jlast; i >= 0; --i) {
+    const cplx z = s_z[i], cc = cconj(s_c[i]);   // H_i = I + conj(c) u u^H
+    const double up_x = s_up[i];
+    const bool row_i = tid == (i & (LT - 1));
+    const int ls = li + 1;
+    if (i != jlast) {
+      if (nst == 4) fetch_wait<2>();
+      else fetch_wait<0>();
+      cplx* x = xs + (size_t)(i & ring) * m;
+      if (up_x != 1.0)
+        for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) x[k] = cscale(x[k], up_x);
+      for (int l = ls; l < nl; l += 2) {
+        cplx* c0 = col(l);
+        cplx* c1 = l + 1 < nl ? col(l + 1) : nullptr;
+        cplx w0 = mk(0.0), w1 = mk(0.0);
+        for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) {
+          const cplx v = cconj(x[k]);
+          w0 = cfma(v, c0[k], w0);
+          if (c1) w1 = cfma(v, c1[k], w1);
+        }
+        const int h0 = half;
+        if (row_i) {
+          s_aj[h0][0] = c0[i];
+          if (c1) s_aj[h0][1] = c1[i];
+        }
+        cta_sum4(w0.x, w0.y, w1.x, w1.y, red, half);
+        const cplx q0 = s_aj[h0][0], q1 = c1 ? s_aj[h0][1] : mk(0.0);
+        const cplx f0 = cmul(cc, cfma(cconj(z), q0, w0));
+        const cplx f1 = cmul(cc, cfma(cconj(z), q1, w1));
+        if (row_i) x[i] = z;   // u
+        for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
+          c0[k] = cfma(x[k], f0, c0[k]);
+          if (c1) c1[k] = cfma(x[k], f1, c1[k]);
+        }
+      }
+      const int in = i - (nst - 1);
+      if (in >= 0) fetch_col(pub + (size_t)m * in, xs + (size_t)(in & ring) * m, in, m);
+      fetch_commit();
+    }
+    if (i == jown) {   // H_i e_i
+      cplx* c = col(li--);
+      jown -= G;
+      const cplx t = cmul(cc, cconj(z)), g = cscale(t, up_x);
+      for (int k = tid; k < m; k += LT) c[k] = k > i ? cmul(g, c[k]) : k == i ? cfma(t, z, mk(1.0)) : mk(0.0);
+    }
+  }
+  if (in_smem)
+    for (int l = 0; l < nl; ++l) {
+      cplx* dst = A + (size_t)m * (b + (size_t)l * G);
+      for (int k = tid; k < m; k += LT) dst[k] = col(l)[k];
+    }
 }
 
 // ---------------------------------------------------------------------------
-// LU with partial pivoting in place (zgetf2), n x n, lda = n.  ipiv 0-based.
-// info[0] = first zero pivot (1-based) or 0.  lcol is an n-vector of scratch.
-__global__ void __launch_bounds__(256) k_lu(int n, cplx* A, int* ipiv, int* info, cplx* lcol) {
-  cg::grid_group grid = cg::this_grid();
-  __shared__ double sv[256];
-  __shared__ int si[256];
-  if (blockIdx.x == 0 && threadIdx.x == 0) info[0] = 0;
+// LU with partial pivoting (zgetf2's pivots: largest |re| + |im|, ties to the
+// lowest row) of A (n x n, lda = n, destroyed) and A X = B solved in place on
+// B (n x nrhs), in one pass: the right-hand sides are further columns of the
+// elimination, then each CTA substitutes back on its own ones.  Rows are not
+// moved: a row leaves when it becomes a pivot row, so the row every thread
+// reads in a step is one nobody writes.  diag: the pivots in order, perm: the
+// rows they came from, info[0]: first zero pivot (1-based) or 0.
+// Bound like k_house_qr by the chain of a step: poll, the pivot search (on
+// the bits, as integers), one reciprocal, the next column's update.
+__global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx* B, int ldb, cplx* diag, int* perm,
+                                                 int* info, cplx* pub, int in_smem, int nst, int* err) {
+  extern __shared__ cplx lu_dyn[];
+  __shared__ unsigned long long s_key[2][4];
+  __shared__ int s_row[2][4];
+  __shared__ int s_fail;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.x, G = gridDim.x, T = n + nrhs;
+  const int nl = (T - b + G - 1) / G;
+  cplx* xs = lu_dyn;
+  cplx* s_rec = xs + (size_t)nst * n;          // reciprocals of the pivots
+  cplx* s_sol = s_rec + n;                     // a solution in progress (!in_smem)
+  int* s_prow = reinterpret_cast<int*>(s_sol + (in_smem ? 0 : n));
+  int* s_ord = s_prow + n;                     // step at which a row became the pivot row
+  cplx* cols = s_rec + n + (in_smem ? 0 : n) + (2 * n + 3) / 4;
+  auto gcol = [&](int l) {
+    const size_t j = b + (size_t)l * G;
+    return j < (size_t)n ? A + (size_t)n * j : B + (size_t)ldb * (j - n);
+  };
+  auto col = [&](int l) { return in_smem ? cols + (size_t)l * n : gcol(l); };
+  if (tid == 0) s_fail = 0;
+  for (int k = tid; k < n; k += LT) s_ord[k] = n;
+  if (in_smem)
+    for (int l = 0; l < nl; ++l)
+      for (int k = tid; k < n; k += LT) col(l)[k] = gcol(l)[k];
+  __syncthreads();
+  if (b == 0)
+    for (int k = tid; k < n; k += LT) publish(pub + k, col(0)[k]);
+  const bool last_owner = (n - 1) % G == b;
+  int first_zero = 0;
+  int li = 0, jown = b;   // the next local column, local and global
   for (int j = 0; j < n; ++j) {
-    cplx* cj = A + (size_t)n * j;
-    if (blockIdx.x == 0) {
-      double best = -1.0;
-      int bi = j;
-      for (int i = j + threadIdx.x; i < n; i += blockDim.x) {
-        double v = fabs(cj[i].x) + fabs(cj[i].y);
-        if (v > best) { best = v; bi = i; }
+    const bool own = j == jown;
+    const int l0 = own ? li + 1 : li;
+    cplx* x = xs + (size_t)(j & 1) * n;   // two in turn: every thread reads the pivot's entry
+    if (own) {
+      for (int k = tid; k < n; k += LT) x[k] = col(li)[k];
+    } else if (!poll_col(pub + (size_t)n * j, x, 0, n)) {
+      s_fail = 1;
+    }
+    // pivot: the largest |re| + |im| of the rows that are left
+    unsigned long long key = 0;
+    int row = 0x7fffffff;
+    for (int k = tid; k < n; k += LT) {
+      if (s_ord[k] < n) continue;
+      const unsigned long long q = (unsigned long long)__double_as_longlong(fabs(x[k].x) + fabs(x[k].y));
+      if (row == 0x7fffffff || q > key) { key = q; row = k; }
+    }
+    {
+      const unsigned full = 0xffffffffu, hi = (unsigned)(key >> 32);
+      const unsigned mh = __reduce_max_sync(full, row != 0x7fffffff ? hi : 0u);
+      const bool ch = row != 0x7fffffff && hi == mh;
+      const unsigned ml = __reduce_max_sync(full, ch ? (unsigned)key : 0u);
+      const int mr = __reduce_min_sync(full, ch && (unsigned)key == ml ? row : 0x7fffffff);
+      if (lane == 0) {
+        s_key[j & 1][warp] = (unsigned long long)mh << 32 | ml;
+        s_row[j & 1][warp] = mr;
       }
-      sv[threadIdx.x] = best;
-      si[threadIdx.x] = bi;
-      __syncthreads();
-      for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-          double ov = sv[threadIdx.x + s];
-          int oi = si[threadIdx.x + s];
-          if (ov > sv[threadIdx.x] || (ov == sv[threadIdx.x] && oi < si[threadIdx.x])) {
-            sv[threadIdx.x] = ov;
-            si[threadIdx.x] = oi;
-          }
+    }
+    __syncthreads();
+    if (s_fail) {
+      if (tid == 0) atomicExch(err, PQMC_ERR_TIMEOUT);
+      return;
+    }
+    int p = 0x7fffffff;
+    unsigned long long pk = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned long long k2 = s_key[j & 1][q];
+      const int r2 = s_row[j & 1][q];
+      if (r2 != 0x7fffffff && (p == 0x7fffffff || k2 > pk || (k2 == pk && r2 < p))) { p = r2; pk = k2; }
+    }
+    const cplx piv = x[p];
+    // 1/piv, scaled by a power of two so that no square leaves the range
+    cplx rec = mk(0.0);
+    if (((__double_as_longlong(piv.x) | __double_as_longlong(piv.y)) << 1) != 0) {
+      const int e = min(max(top_exp(piv) - 1023, -1000), 1000);
+      const double s = pow2i(-e);
+      const cplx q = cscale(piv, s);
+      const double r = s / fma(q.x, q.x, q.y * q.y);
+      rec = mk(q.x * r, -q.y * r);
+    } else if (!first_zero) {
+      first_zero = j + 1;
+    }
+    if (tid == (p & (LT - 1))) s_ord[p] = j;   // only this thread looks at this row's step
+    if (tid == 0) {
+      s_rec[j] = rec;
+      s_prow[j] = p;
+      if (last_owner) {
+        diag[j] = piv;
+        perm[j] = p;
+      }
+    }
+    for (int l = l0; l < nl; ++l) {
+      cplx* c = col(l);
+      const cplx f = cneg(cmul(rec, c[p]));
+      const bool next = l == l0 && (own ? jown + G : jown) == j + 1 && j + 1 < n;
+      for (int k = tid; k < n; k += LT) {
+        if (s_ord[k] == n) c[k] = cfma(x[k], f, c[k]);
+        if (next) publish(pub + (size_t)n * (j + 1) + k, c[k]);
+      }
+    }
+    if (own) {
+      if (l0 >= nl) break;
+      ++li;
+      jown += G;
+    }
+  }
+  if (last_owner && tid == 0) info[0] = first_zero;
+  // ---- back substitution: x_j = y(p_j) / u_jj, y(p_k) -= U(p_k, j) x_j -----
+  const int lr = b >= n ? 0 : (n - b + G - 1) / G;   // first local right-hand side
+  if (lr >= nl) return;
+  __threadfence();
+  __syncthreads();
+  const int nb = in_smem ? nl - lr : 1;
+  for (int r0 = lr; r0 < nl; r0 += nb) {
+    for (int u = 0; u < nst - 1; ++u) {
+      const int j = n - 1 - u;
+      if (j >= 0) fetch_col(pub + (size_t)n * j, xs + (size_t)(j & (nst - 1)) * n, 0, n);
+      fetch_commit();
+    }
+    for (int j = n - 1; j >= 0; --j) {
+      if (nst == 4) fetch_wait<2>();
+      else fetch_wait<0>();
+      const cplx* u = xs + (size_t)(j & (nst - 1)) * n;
+      const int p = s_prow[j];
+      const cplx rec = s_rec[j];
+      __syncthreads();   // the rows of step j + 1 are in
+      for (int l = r0; l < r0 + nb; ++l) {
+        cplx* y = col(l);
+        const cplx xj = cmul(y[p], rec);
+        const cplx f = cneg(xj);
+        for (int k = tid; k < n; k += LT)
+          if (s_ord[k] < j) y[k] = cfma(u[k], f, y[k]);
+        if (tid == 0) {
+          if (in_smem) B[j + (size_t)ldb * (b + (size_t)l * G - n)] = xj;
+          else s_sol[j] = xj;
         }
-        __syncthreads();
       }
-      const int jp = si[0];
-      const cplx piv = cj[jp];
-      const bool zero = (piv.x == 0.0 && piv.y == 0.0);
-      if (threadIdx.x == 0) {
-        ipiv[j] = jp;
-        if (zero && info[0] == 0) info[0] = j + 1;
-      }
-      // swapped + scaled column j, published in lcol (rows > j)
-      cplx rec = zero ? mk(0.0) : cdiv(mk(1.0), piv);
-      for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
-        cplx v = (i == jp) ? cj[j] : cj[i];
-        lcol[i] = zero ? v : cmul(v, rec);
-      }
-      __syncthreads();
-      for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) cj[i] = lcol[i];
-      if (threadIdx.x == 0) cj[j] = piv;
+      const int jn = j - (nst - 1);
+      if (jn >= 0) fetch_col(pub + (size_t)n * jn, xs + (size_t)(jn & (nst - 1)) * n, 0, n);
+      fetch_commit();
     }
-    grid.sync();
-    const int jp = ipiv[j];
-    for (int k = blockIdx.x; k < n; k += gridDim.x) {
-      if (k == j) continue;
-      cplx* ck = A + (size_t)n * k;
-      if (jp != j && threadIdx.x == 0) {
-        cplx t = ck[j];
-        ck[j] = ck[jp];
-        ck[jp] = t;
-      }
+    if (!in_smem) {
       __syncthreads();
-      if (k > j) {
-        const cplx u = ck[j];
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) ck[i] = csub(ck[i], cmul(lcol[i], u));
-      }
+      for (int k = tid; k < n; k += LT) gcol(r0)[k] = s_sol[k];
       __syncthreads();
     }
-    grid.sync();
   }
 }
 
-// Solve A X = B in place on B (n x nrhs, ldb = n) from the LU factors.
-// One warp per right-hand side.
-__global__ void k_lu_solve(int n, int nrhs, const cplx* __restrict__ LU, const int* __restrict__ ipiv,
-                           cplx* B, int ldb) {
-  const int lane = threadIdx.x & 31;
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (c >= nrhs) return;
-  cplx* b = B + (size_t)ldb * c;
-  if (lane == 0)
-    for (int j = 0; j < n; ++j) {
-      int p = ipiv[j];
-      if (p != j) { cplx t = b[j]; b[j] = b[p]; b[p] = t; }
-    }
-  __syncwarp();
-  // forward: unit lower
-  for (int i = 1; i < n; ++i) {
-    cplx s = mk(0.0);
-    for (int j = lane; j < i; j += 32) s = cfma(LU[i + (size_t)n * j], b[j], s);
-    for (int o = 16; o > 0; o >>= 1) {
-      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-    }
-    if (lane == 0) b[i] = csub(b[i], s);
-    __syncwarp();
+// log det from the pivots: the reference forms the product of the diagonal
+// (zdet_lapack, src/mod_matrixlib.f90:624-653) and takes its log; here the
+// sum of logs, one pivot per thread (the product alone was a chain of n
+// complex multiplications with a log each: 624 us at n = 196), taken back to
+// the principal branch of that product where it stays in the double range.
+__global__ void __launch_bounds__(LT) k_lu_logdet(int n, const cplx* diag, const int* perm, cplx* out) {
+  __shared__ double red[2][4][4];
+  int half = 0;
+  double re = 0.0, im = 0.0, odd = 0.0, zero = 0.0;
+  for (int i = threadIdx.x; i < n; i += LT) {
+    const cplx l = clog_(diag[i]);
+    re += l.x;
+    im += l.y;
+    int inv = 0;   // parity of the permutation
+    const int pi = perm[i];
+    for (int k = 0; k < i; ++k) inv ^= perm[k] > pi;
+    odd += inv;
   }
-  for (int i = n - 1; i >= 0; --i) {
-    cplx s = mk(0.0);
-    for (int j = i + 1 + lane; j < n; j += 32) s = cfma(LU[i + (size_t)n * j], b[j], s);
-    for (int o = 16; o > 0; o >>= 1) {
-      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-    }
-    if (lane == 0) b[i] = cdiv(csub(b[i], s), LU[i + (size_t)n * i]);
-    __syncwarp();
-  }
-}
-
-// log det from the LU factors: the reference forms the product of the
-// diagonal (zdet_lapack, src/mod_matrixlib.f90:624-653) and takes its log;
-// when the product leaves the double range the sum of logs is used.
-__global__ void k_lu_logdet(int n, const cplx* LU, const int* ipiv, cplx* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int s = 1;
-  cplx d = mk(1.0), ls = mk(0.0);
-  for (int i = 0; i < n; ++i) {
-    if (ipiv[i] != i) s = -s;
-    cplx u = LU[i + (size_t)n * i];
-    d = cmul(d, u);
-    ls = cadd(ls, clog_(u));
-  }
-  if (s < 0) {
-    d = cneg(d);
-    ls = cadd(ls, mk(0.0, 3.14159265358979323846));
-  }
-  double ad = cabsd(d);
-  out[0] = (ad > 1e-290 && ad < 1e290) ? clog_(d) : ls;
+  cta_sum4(re, im, odd, zero, red, half);
+  if (threadIdx.x != 0) return;
+  const double pi = 3.14159265358979323846;
+  if (fmod(odd, 2.0) != 0.0) im += pi;
+  if (fabs(re) < 667.0) im = remainder(im, 2.0 * pi);   // |det| in 1e-290 .. 1e290
+  out[0] = mk(re, im);
 }
 
 int coop_grid(const void* fn, int threads, int want) {
@@ -385,36 +630,69 @@ int coop_grid(const void* fn, int threads, int want) {
   return want < 1 ? 1 : want;
 }
 
-int house_qr(cudaStream_t s, int m, int n, cplx* A, cplx* tau, cplx* d) {
-  return house_qr_r(s, m, n, A, tau, d, nullptr, nullptr);
+// Grid and shared memory of a column pipeline over `ncol` columns of `len`
+// rows.  Two CTAs per SM while their columns fit in half its shared memory
+// (at Ns = 392, nelec = 196 a CTA has one column of the QR), one while they
+// fit in all of it, and past that the columns stay in global memory.
+// `fixed`: complex entries besides the ring and the columns.
+struct PipeShape {
+  int grid, in_smem, nst;
+  size_t smem;
+};
+template <typename FIXED>
+static int pipe_shape(const void* fn, int ncol, int len, FIXED fixed, PipeShape* out) {
+  int dev = 0, nsm = 0;
+  PQMC_CUDA(cudaGetDevice(&dev));
+  PQMC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const struct { int per, nst, in; size_t lim; } opt[] = {
+      {1, 4, 1, 110 * 1024}, {2, 4, 1, 110 * 1024}, {1, 4, 1, 220 * 1024}, {1, 2, 1, 220 * 1024}, {1, 4, 0, 220 * 1024}, {1, 2, 0, 220 * 1024}};
+  for (const auto& o : opt) {
+    PipeShape q;
+    q.grid = ncol < o.per * nsm ? ncol : o.per * nsm;
+    q.in_smem = o.in;
+    q.nst = o.nst;
+    const int nl = (ncol + q.grid - 1) / q.grid;
+    q.smem = sizeof(cplx) * ((size_t)o.nst * len + fixed(nl, o.in) + (o.in ? (size_t)nl * len : 0));
+    if (q.smem > o.lim || (&o == opt && nl > 2)) continue;
+    PQMC_CUDA(raise_dyn_smem((const char*)fn, (int)q.smem));
+    int per = 0;
+    PQMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, LT, q.smem));
+    if (per * nsm < q.grid) continue;
+    *out = q;
+    return PQMC_OK;
+  }
+  set_error("dense factorisation: columns of %d entries do not fit in shared memory", len);
+  return PQMC_ERR_ARG;
 }
 
-int house_qr_r(cudaStream_t s, int m, int n, cplx* A, cplx* tau, cplx* d, cplx* R, cplx* lndet) {
-  int nb = coop_grid((const void*)k_house_qr, 256, n);
-  int scaled = (R != nullptr || lndet != nullptr) ? 1 : 0;
-  void* args[] = {&m, &n, &A, &tau, &d, &R, &lndet, &scaled};
-  PQMC_CUDA(cudaLaunchCooperativeKernel((const void*)k_house_qr, nb, 256, args, 0, s));
+int house_qr(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* work, int* err) {
+  return house_qr_r(s, m, n, A, d, nullptr, nullptr, work, err);
+}
+
+int house_qr_r(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* R, cplx* lndet, cplx* work, int* err) {
+  PipeShape q;
+  PQMC_TRY(pipe_shape((const void*)k_house_qr, n, m, [&](int nl, int) { return (size_t)2 * n + (n + 1) / 2 + (nl + 3) / 4; }, &q));
+  PQMC_CUDA(cudaMemsetAsync(work, 0xff, sizeof(cplx) * (size_t)m * n, s));
+  void* args[] = {&m, &n, &A, &d, &R, &lndet, &work, &q.in_smem, &q.nst, &err};
+  PQMC_CUDA(cudaLaunchCooperativeKernel((const void*)k_house_qr, q.grid, LT, args, q.smem, s));
   PQMC_LAUNCHED();
   return PQMC_OK;
 }
 
-int lu_factor(cudaStream_t s, int n, cplx* A, int* ipiv, int* info, cplx* lcol) {
-  int nb = coop_grid((const void*)k_lu, 256, n);
-  void* args[] = {&n, &A, &ipiv, &info, &lcol};
-  PQMC_CUDA(cudaLaunchCooperativeKernel((const void*)k_lu, nb, 256, args, 0, s));
+int lu_solve(cudaStream_t s, int n, cplx* A, int nrhs, cplx* B, int ldb, cplx* diag, int* perm, int* info, cplx* work,
+             int* err) {
+  PipeShape q;
+  PQMC_TRY(pipe_shape((const void*)k_lu_solve, n + nrhs, n,
+                      [&](int, int in) { return (size_t)n + (in ? 0 : n) + (2 * n + 3) / 4; }, &q));
+  PQMC_CUDA(cudaMemsetAsync(work, 0xff, sizeof(cplx) * (size_t)n * n, s));
+  void* args[] = {&n, &A, &nrhs, &B, &ldb, &diag, &perm, &info, &work, &q.in_smem, &q.nst, &err};
+  PQMC_CUDA(cudaLaunchCooperativeKernel((const void*)k_lu_solve, q.grid, LT, args, q.smem, s));
   PQMC_LAUNCHED();
   return PQMC_OK;
 }
 
-int lu_solve(cudaStream_t s, int n, int nrhs, const cplx* LU, const int* ipiv, cplx* B, int ldb) {
-  int wpb = 4;
-  k_lu_solve<<<(nrhs + wpb - 1) / wpb, 32 * wpb, 0, s>>>(n, nrhs, LU, ipiv, B, ldb);
-  PQMC_LAUNCHED();
-  return PQMC_OK;
-}
-
-int lu_logdet(cudaStream_t s, int n, const cplx* LU, const int* ipiv, cplx* out) {
-  k_lu_logdet<<<1, 32, 0, s>>>(n, LU, ipiv, out);
+int lu_logdet(cudaStream_t s, int n, const cplx* diag, const int* perm, cplx* out) {
+  k_lu_logdet<<<1, LT, 0, s>>>(n, diag, perm, out);
   PQMC_LAUNCHED();
   return PQMC_OK;
 }

@@ -82,17 +82,23 @@ extern "C" int pqmc_cal_g_and_det_noalloc(const double* x_left, const double* rm
   // P^H B P = X^H R  (cal_g_and_det_T0, src/mod_evolution.f90:344)
   PQMC_TRY(pqmc::zgemm(s, 'C', 'N', nelec, nelec, ns, mk(1.0), X, ns, R, ns, mk(0.0), pbp, nelec));
   // log det (:345) and the LU factors for the inverse (:347)
-  PQMC_TRY(pqmc::lu_factor(s, nelec, pbp, ipiv, info, lcol));
-  PQMC_TRY(pqmc::lu_logdet(s, nelec, pbp, ipiv, reinterpret_cast<cplx*>(logdet_out)));
-  // g_h = R (P^H B P)^-1 L with L = X^H  (:349-350)
+  // and L = X^H solved beside it; the caller's G is the factorisation's
+  // scratch until the product below fills it
   PQMC_TRY(pqmc::herm_t(s, ns, nelec, X, lmat));
-  PQMC_TRY(pqmc::lu_solve(s, nelec, ns, pbp, ipiv, lmat, nelec));
+  PQMC_CUDA(cudaMemsetAsync(info + 1, 0, sizeof(int), s));
+  PQMC_TRY(pqmc::lu_solve(s, nelec, pbp, ns, lmat, nelec, lcol, ipiv, info, G, info + 1));
+  PQMC_TRY(pqmc::lu_logdet(s, nelec, lcol, ipiv, reinterpret_cast<cplx*>(logdet_out)));
+  // g_h = R (P^H B P)^-1 L  (:349-350)
   PQMC_TRY(pqmc::zgemm(s, 'N', 'N', ns, ns, nelec, mk(1.0), R, ns, lmat, nelec, mk(0.0), G, ns));
-  int h_info = 0;
-  PQMC_CUDA(cudaMemcpyAsync(&h_info, info, sizeof(int), cudaMemcpyDeviceToHost, s));
+  int h_info[2] = {0, 0};
+  PQMC_CUDA(cudaMemcpyAsync(h_info, info, sizeof(h_info), cudaMemcpyDeviceToHost, s));
   PQMC_CUDA(cudaStreamSynchronize(s));
-  if (h_info != 0) {
-    pqmc::set_error("cal_g_and_det_noalloc: zero pivot %d in P^H B P", h_info);
+  if (h_info[1] != 0) {
+    pqmc::set_error("cal_g_and_det_noalloc: a wait inside the factorisation ran out");
+    return h_info[1];
+  }
+  if (h_info[0] != 0) {
+    pqmc::set_error("cal_g_and_det_noalloc: zero pivot %d in P^H B P", h_info[0]);
     return PQMC_ERR_SINGULAR;
   }
   return PQMC_OK;

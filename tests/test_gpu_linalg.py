@@ -1,0 +1,93 @@
+"""The FP64 factorisations at the edges of their column pipeline: fewer rows
+than threads, exactly a block of 128 and one past it, one and two columns
+per CTA, and right-hand sides beside the factored columns.
+
+Tolerances: backward-stable factorisations of matrices of condition ~10, so
+errors are a small multiple of eps * n; 1e-11 leaves two orders of room at
+the largest size.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tests.helpers import SEED_WORDS, epsocz_small, rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ns,ne", [(1, 1), (2, 1), (5, 3), (64, 31), (128, 127), (200, 128), (257, 129), (392, 196), (512, 256)])
+def test_lu_solve_through_the_allocation_free_entry(ns, ne):
+    """G = R (X^H R)^-1 X^H and log det(X^H R) against numpy."""
+    torch = pytest.importorskip("torch")
+    from pqmc_allinone_gb300.abi import load_library
+    rng = np.random.default_rng(1000 * ns + ne)
+
+    def orth():
+        return np.linalg.qr(rng.normal(size=(ns, ne)) + 1j * rng.normal(size=(ns, ne)))[0]
+
+    x = orth()
+    r = x @ (rng.permutation(np.eye(ne)) * np.exp(1j * rng.uniform(0, 6, ne))) + 0.2 * orth()
+    lib = load_library()
+    fn = lib.pqmc_cal_g_and_det_noalloc
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 3
+    fn.restype = ctypes.c_int
+    dev = [torch.from_numpy(np.asfortranarray(a).ravel(order="F").view(np.float64).copy()).cuda() for a in (x, r)]
+    g_d = torch.zeros(2 * ns * ns, dtype=torch.float64, device="cuda")
+    ld_d = torch.zeros(2, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert fn(dev[0].data_ptr(), dev[1].data_ptr(), ns, ne, g_d.data_ptr(), ld_d.data_ptr(), None) == 0, lib.pqmc_last_error()
+    g = g_d.cpu().numpy().view(np.complex128).reshape((ns, ns), order="F")
+    lr = x.conj().T @ r
+    assert rel_fro(g, r @ np.linalg.solve(lr, x.conj().T)) < 1e-11
+    sign, logabs = np.linalg.slogdet(lr)
+    ld = ld_d.cpu().numpy()
+    assert abs(ld[0] - logabs) < 1e-11 * max(1.0, ne)
+    assert abs(np.exp(1j * ld[1]) - sign) < 1e-10
+
+
+def test_singular_matrix_is_reported():
+    torch = pytest.importorskip("torch")
+    from pqmc_allinone_gb300.abi import load_library
+    lib = load_library()
+    x = torch.zeros(2 * 6 * 3, dtype=torch.float64, device="cuda")
+    out = torch.zeros(2 * 6 * 6 + 2, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    fn = lib.pqmc_cal_g_and_det_noalloc
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 3
+    fn.restype = ctypes.c_int
+    assert fn(x.data_ptr(), x.data_ptr(), 6, 3, out.data_ptr(), out[72:].data_ptr(), None) == 3   # PQMC_ERR_SINGULAR
+
+
+@pytest.mark.parametrize("L", [(4, 4), (4, 6), (8, 8), (6, 12), (12, 14)])
+def test_qr_strings_against_the_oracle(L):
+    """Q and D of every block (zgeqrf's signs): Ns = 32 .. 336, nelec = 16 .. 168."""
+    from oracle.oracle import OracleChain
+    from pqmc_allinone_gb300.engine import PqmcChain
+    m, f = epsocz_small(L=L, ntime=20, ngroup=10, alpha=0.3)
+    o = OracleChain(m, field=f, seed_words=SEED_WORDS, meas=False)
+    g = PqmcChain(m, field=f, rng_words=SEED_WORDS)
+    for c in (o, g):
+        c.init_expkv()
+        c.init_g(1)
+    for blk in range(1, m.nblock + 1):
+        (qo, do), (qg, dg) = o.qd(blk), g.qd(blk)
+        assert rel_fro(qg, qo) < 1e-10 and np.allclose(dg, do, rtol=1e-10, atol=1e-12), blk
+    assert rel_fro(g.g(), o.g()) < 1e-10
+
+
+def test_square_qr_with_two_columns_per_cta():
+    """Finite temperature at Ns = 320: 320 columns, R and det Q returned."""
+    from oracle.finite_t import dense_g_and_weight
+    from oracle.oracle import OracleChain
+    from pqmc_allinone_gb300.engine import PqmcChain
+    m, f = epsocz_small(L=(10, 16), ntime=10, ngroup=5, alpha=0.3)
+    o = OracleChain(m, field=f, seed_words=SEED_WORDS, meas=False)
+    o.init_expkv()
+    g = PqmcChain(m, field=f, rng_words=SEED_WORDS)
+    g.set_temperature(False)
+    g.init_expkv()
+    g.init_g(1)
+    gd, ld = dense_g_and_weight(o)
+    assert rel_fro(g.g(), gd) < 1e-10
+    assert abs(g.state()["ln_cw"].real - ld.real) <= 1e-9 * abs(ld.real)
