@@ -268,7 +268,7 @@ __global__ void k_scalars_zero(DevScalars* sc) {
 }
 
 // waits for the stream and reports a zero pivot or a wait that ran out inside
-// a factorisation
+// a kernel (factorisation or update)
 int check_factor(pqmc_chain* c, const char* what) {
   int h[2] = {0, 0};
   static_assert(offsetof(DevScalars, lin_err) == offsetof(DevScalars, lu_info) + sizeof(int), "read back together");
@@ -276,7 +276,7 @@ int check_factor(pqmc_chain* c, const char* what) {
   PQMC_CUDA(cudaStreamSynchronize(c->stream));
   if (h[1] != 0) {
     PQMC_CUDA(cudaMemsetAsync(&c->sc->lin_err, 0, sizeof(int), c->stream));
-    set_error("%s: a wait inside a factorisation ran out", what);
+    set_error("%s: a wait inside a kernel ran out", what);
     return h[1];
   }
   if (h[0] != 0) {
@@ -559,6 +559,8 @@ int chain_alloc(pqmc_chain* c, const pqmc_model* m, cudaStream_t s) {
   PQMC_TRY(dalloc(&c->lcol, (size_t)c->nelec + 2));
   PQMC_TRY(dalloc(&c->ipiv, (size_t)c->nelec));
   PQMC_TRY(dalloc(&c->ctl, 2));
+  PQMC_TRY(dalloc(&c->upd_sync, 1));
+  PQMC_CUDA(cudaMemset(c->upd_sync, 0, sizeof(UpdSync)));
   PQMC_TRY(dalloc(&c->sc, 1));
   PQMC_CUDA(cudaMemset(c->g, 0, sizeof(cplx) * (size_t)c->ns * c->ns));
   PQMC_CUDA(cudaMemset(c->field, 0, sizeof(double) * (size_t)c->n_bf * c->ntime));
@@ -623,7 +625,7 @@ int chain_free(pqmc_chain* c) {
   ft_free(c);
   void* ptrs[] = {c->d_logsum, c->pre, c->d_model_blob, c->field, c->expkv, c->expkv_inv, c->g, c->g_alt, c->q_string, c->d_string,
                   c->slater_q, c->slater_d, c->rmat, c->xmat, c->lmat, c->pbp, c->dtmp, c->lcol,
-                  c->ipiv, c->ctl, c->sc, c->m_cell_sites, c->m_cell_bf, c->m_cell_xnb, c->m_cell_ynb,
+                  c->ipiv, c->ctl, c->upd_sync, c->sc, c->m_cell_sites, c->m_cell_bf, c->m_cell_xnb, c->m_cell_ynb,
                   c->m_cell_cross, c->m_c2_of, c->m_kphase, c->m_acc, c->m_gtmp};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -847,8 +849,10 @@ int pqmc_update_phonon_field(pqmc_chain* c, int pf_id, int time) {
     return PQMC_ERR_ARG;
   }
   PQMC_TRY(launch_update(c, pf_id - 1, time));
+  int late = 0;
+  PQMC_CUDA(cudaMemcpyAsync(&late, &c->sc->lin_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   PQMC_CUDA(cudaStreamSynchronize(c->stream));
-  return PQMC_OK;
+  return late ? check_factor(c, "update_phonon_field") : PQMC_OK;
 }
 
 int pqmc_left_evolve_g(pqmc_chain* c, int time, int pf_id, int two_way) {

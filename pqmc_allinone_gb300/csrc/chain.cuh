@@ -23,17 +23,28 @@ struct DevScalars {
   long long neg_acc;
   int rng[5];
   int lu_info;
-  int lin_err;          // a wait inside a factorisation ran out (PQMC_ERR_TIMEOUT)
+  int lin_err;          // a wait inside a kernel ran out (PQMC_ERR_TIMEOUT)
   int status;
 };
 
-// Control record the proposer publishes at every grid barrier of the update
-// kernel: the accepted plaquette and T = Delta R^-1 of its rank-dim update.
+// Control record the proposer publishes for every accepted move of the update
+// kernel: the accepted plaquette (-1: the walk is over) and T = Delta R^-1 of
+// its rank-dim update, entry (i, j) at i + 4 j.
 struct UpdCtl {
   int p;
   int dim;
   int S[4];
   cplx T[16];
+};
+
+// Running counters of the update kernel's hand-over (on cache lines of their own).
+struct UpdSync {
+  unsigned seq;
+  unsigned pad0[31];
+  unsigned arrived;
+  unsigned pad1[31];
+  unsigned done;
+  unsigned pad2[31];
 };
 
 // Per-plaquette proposal data of one family step, computed in parallel
@@ -88,10 +99,11 @@ struct pqmc_chain {
   cplx* lcol = nullptr;             // (nelec)
   int* ipiv = nullptr;              // (nelec)
   pqmc::UpdCtl* ctl = nullptr;      // [2]
+  pqmc::UpdSync* upd_sync = nullptr;
   pqmc::PlaqPre* pre = nullptr;     // (max_pla)
   pqmc::DevScalars* sc = nullptr;
   std::vector<pqmc::WrapItems> wrap;
-  int upd_blocks = 0;
+  int upd_blocks = 0, upd_smem = 0;
   bool have_g = false;
   bool have_meas = false;
   cudaStream_t stream = nullptr;

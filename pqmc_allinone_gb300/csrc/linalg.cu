@@ -619,11 +619,11 @@ __global__ void __launch_bounds__(LT) k_lu_logdet(int n, const cplx* diag, const
   out[0] = mk(re, im);
 }
 
-int coop_grid(const void* fn, int threads, int want) {
+int coop_grid(const void* fn, int threads, int want, size_t smem) {
   int dev = 0, nsm = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem);
   int cap = nsm * (per > 0 ? per : 1);
   if (want > cap) want = cap;
   if (want > nsm) want = nsm;

@@ -20,5 +20,5 @@ int lu_solve(cudaStream_t s, int n, cplx* A, int nrhs, cplx* B, int ldb, cplx* d
 // log det A from lu_solve's pivots
 int lu_logdet(cudaStream_t s, int n, const cplx* diag, const int* perm, cplx* out);
 int herm_t(cudaStream_t s, int m, int n, const cplx* a, cplx* out);
-int coop_grid(const void* fn, int threads, int want);
+int coop_grid(const void* fn, int threads, int want, size_t smem = 0);
 }  // namespace pqmc

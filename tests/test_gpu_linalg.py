@@ -91,3 +91,25 @@ def test_square_qr_with_two_columns_per_cta():
     gd, ld = dense_g_and_weight(o)
     assert rel_fro(g.g(), gd) < 1e-10
     assert abs(g.state()["ln_cw"].real - ld.real) <= 1e-9 * abs(ld.real)
+
+
+@pytest.mark.parametrize("L", [(4, 6), (6, 6), (10, 10), (12, 18)])
+def test_update_shares(L):
+    """Rank-dim updates of G by shares of the entries: a few CTAs, all of
+    them, entries kept in registers (Ns <= 393) and read again (Ns = 432)."""
+    from oracle.oracle import OracleChain
+    from pqmc_allinone_gb300.engine import PqmcChain
+    m, f = epsocz_small(L=L, ntime=10, ngroup=5, alpha=0.3)
+    o = OracleChain(m, field=f, seed_words=SEED_WORDS, meas=False)
+    g = PqmcChain(m, field=f, rng_words=SEED_WORDS)
+    for c in (o, g):
+        c.init_expkv()
+        c.init_g(1)
+    for pf in (4, 3):
+        for c in (o, g):
+            c.right_evolve_g(m.ntime, pf)
+            c.update_phonon_field(pf, m.ntime)
+        so, sg = o.state(), g.state()
+        assert sg["rng"] == so["rng"] and np.array_equal(g.field(), o.field())
+        assert sg["positive_accept"] == so["positive_accept"] > 0
+        assert rel_fro(g.g(), o.g()) < 1e-10
