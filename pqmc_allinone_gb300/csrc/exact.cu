@@ -40,10 +40,10 @@ __device__ __forceinline__ dfc dfc_inv(dfc a) {
 
 // ---------------------------------------------------------------------------
 // M = Delta_S W^-1, W = I + G(S,S) Delta_S, in two launches:
-//   k_xinv  (one CTA per chain) forms W in double-float and inverts its
-//           FP32 rounding by Gauss-Jordan over the moves' dim x dim blocks
-//           (the block pivots are the moves' ratio matrices R_j, each
-//           inverted by its adjugate): V0 = W^-1 to ~1e-6;
+//   k_xinv  (one CTA per chain) inverts the FP32 rounding of W by
+//           Gauss-Jordan over the moves' dim x dim blocks (the block pivots
+//           are the moves' ratio matrices R_j, each inverted by its
+//           adjugate): V0 = W^-1 to ~1e-6;
 //   k_xres  (XR_CTAS per chain, a column slab each) one Newton step,
 //           V1 = V0 + V0 (I - W V0), with the residual I - W V0 formed in
 //           double-float from every product's exact parts, so V1 = W^-1 to
@@ -51,114 +51,125 @@ __device__ __forceinline__ dfc dfc_inv(dfc a) {
 //           columns (the B operand of X = G(:,S) M).
 // The rows of G(:,S) (the A operand of X) and the columns of Z = E_S - G(S,:)
 // (the B operand of the flush) depend on G and S only and are cut by
-// k_xslice, launched before both.
-constexpr int XC_THREADS = 1024;
+// k_xslice, launched before both, which forms W in double-float too.
+constexpr int XC_THREADS = 512;
 constexpr int XC_LD = UM_KP;   // leading dimension of the K x K matrices
 constexpr int XR_CTAS = 8;     // column slabs of the Newton step per chain
 constexpr int XR_W = UM_KP / XR_CTAS;
 constexpr int XR_THREADS = UM_KP * XR_W;   // one residual entry per thread
-constexpr size_t XI_SMEM = sizeof(float4) * 16 * UM_KP + sizeof(float2) * ((size_t)XC_LD * XC_LD + 8 * UM_KP) +
-                           sizeof(int) * UM_KP;
 constexpr size_t XR_SMEM = sizeof(float4) * ((size_t)XC_LD * XC_LD + 16 * UM_KP + (size_t)UM_KP * XR_W) +
                            sizeof(float2) * (size_t)XC_LD * XC_LD;
 
-__global__ void __launch_bounds__(XC_THREADS, 1) k_xinv(const XDesc* X, int dim, int parity) {
-  __shared__ XDesc sd;
-  __shared__ float2 s_pb[16];
-  extern __shared__ __align__(16) unsigned char xc_dyn[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) sd = X[blockIdx.y];
-  __syncthreads();
-  const XDesc& d = sd;
+// FP32 Gauss-Jordan of W's rounding, W in registers: eight threads per row,
+// eight adjacent columns each, four rows per warp.  A step needs its pivot
+// rows, the pivot columns and P^-1 in shared memory, two buffers in turn, and
+// one barrier: having updated its rows, every thread publishes what the next
+// step needs of them, and the warp that holds the next pivot rows (all of
+// them: DIM divides 4; DIM = 3 takes two more barriers) inverts the next pivot
+// block meanwhile.  Bound by issue (160 FP32 instructions per thread and
+// step) and that chain: 16 steps of W held in shared memory by 1024 threads,
+// each forming its row's multipliers anew, took 39 us at K = 64.
+template <int DIM>
+__global__ void __launch_bounds__(XC_THREADS, 1) k_xinv(const XDesc* X) {
+  const XDesc& d = X[blockIdx.y];
   const int K = *d.kcount;
   if (K == 0) return;
-  const int ns = d.ns;
-  const float4* G = parity ? d.g_alt : d.g;
-  {
-    float4* s_dl = reinterpret_cast<float4*>(xc_dyn);                 // [n_acc][16] Delta blocks
-    float2* Wf = reinterpret_cast<float2*>(s_dl + 16 * UM_KP);        // [K][XC_LD] FP32 W, inverted in place
-    float2* s_row = Wf + (size_t)XC_LD * XC_LD;                       // [dim][UM_KP] pivot rows
-    float2* s_col = s_row + 4 * UM_KP;                                // [dim][UM_KP] pivot columns
-    int* s_site = reinterpret_cast<int*>(s_col + 4 * UM_KP);
-    const int nb = K / dim;
-    for (int k = tid; k < K; k += XC_THREADS) s_site[k] = d.acc_site[k];
-    for (int e = tid; e < nb * 16; e += XC_THREADS) s_dl[e] = d.acc_delta[e];
+  __shared__ __align__(16) float2 s_row[2][DIM][UM_KP];
+  __shared__ float2 s_col[2][DIM][UM_KP];
+  __shared__ float2 s_pb[2][16];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int ri = tid >> 3, c0 = 8 * (tid & 7);   // row ri, columns c0 .. c0 + 7
+  const int nb = K / DIM;
+  float2 w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    w[j] = (ri < K && c0 + j < K) ? hi2(d.wdf[(size_t)(c0 + j) * XC_LD + ri]) : make_float2(0.f, 0.f);
+  // P^-1 by one warp, in place (column-major)
+  auto invert = [&](int par) {
+    __syncwarp();
+    const float2 det = wf_det(DIM, s_pb[par], lane);
+    if (lane == 0 && !(det.x * det.x + det.y * det.y > 0.f)) atomicExch(d.err, PQMC_ERR_SINGULAR);
+    wf_inverse(DIM, s_pb[par], det, lane);
+  };
+  // what step b needs: its pivot columns (left as zeros: the step writes them
+  // anew), and from the pivot rows (zeros likewise) the rows with the identity
+  // in place of the pivot block, and the block
+  auto publish = [&](int b) {
+    const int b0 = b * DIM, par = b & 1;
+    const bool piv = ri >= b0 && ri < b0 + DIM;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int c = c0 + j - b0;
+      if (c >= 0 && c < DIM) {
+        s_col[par][c][ri] = w[j];
+        if (piv) s_pb[par][ri - b0 + DIM * c] = w[j];
+        w[j] = piv && c == ri - b0 ? make_float2(1.f, 0.f) : make_float2(0.f, 0.f);
+      }
+    }
+    if (piv) {
+#pragma unroll
+      for (int j = 0; j < 8; j += 2)
+        *reinterpret_cast<float4*>(&s_row[par][ri - b0][c0 + j]) = make_float4(w[j].x, w[j].y, w[j + 1].x, w[j + 1].y);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = make_float2(0.f, 0.f);
+    }
+    if (DIM != 3) {
+      if (tid >> 5 == b0 >> 2) invert(par);
+    } else {
+      __syncthreads();
+      if (tid < 32) invert(par);
+      __syncthreads();
+    }
+  };
+  publish(0);
+  for (int b = 0; b < nb; ++b) {
     __syncthreads();
-    // W(i, jb*dim + jj) = delta_ij + sum_m G(S_i, S_{jb dim + m}) Delta_jb(m, jj)
-    for (int it = tid; it < K * nb; it += XC_THREADS) {
-      const int i = it % K, jb = it / K;
-      dfc gs[4];
+    const int b0 = b * DIM, par = b & 1;
+    if ((tid & ~31) < 8 * K) {   // the warp has rows
+      // f = row ri of P^-1 on the pivot rows, -W(ri, pivot columns) P^-1 elsewhere
+      const bool piv = ri >= b0 && ri < b0 + DIM;
+      float2 f[DIM];
+      if constexpr (DIM == 4) {   // a thread's share of its row's four, the rest by shuffles
+        const int n = tid & 3;
+        float2 own = make_float2(0.f, 0.f);
+        if (piv) {
+          own = s_pb[par][ri - b0 + 4 * n];
+        } else {
 #pragma unroll
-      for (int m = 0; m < 4; ++m)
-        if (m < dim) gs[m] = dg_dfc(G[s_site[i] + (size_t)ns * s_site[jb * dim + m]]);
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        if (jj >= dim) break;
-        const int j = jb * dim + jj;
-        dfc a = dfc{df{i == j ? 1.f : 0.f, 0.f}, df{0.f, 0.f}};
+          for (int m = 0; m < 4; ++m) own = fcfma(s_col[par][m][ri], s_pb[par][m + 4 * n], own);
+          own = make_float2(-own.x, -own.y);
+        }
 #pragma unroll
         for (int m = 0; m < 4; ++m)
-          if (m < dim) a = dfc_mac(a, gs[m], dg_dfc(s_dl[jb * 16 + m + dim * jj]));
-        d.wdf[j * XC_LD + i] = dfc_dg(a);   // column-major: k_xres reads W(i, k) for consecutive i
-        Wf[i * XC_LD + j] = make_float2(a.re.hi, a.im.hi);
-      }
-    }
-    __syncthreads();
-    // FP32 Gauss-Jordan in place by blocks of the moves: the pivot block P is
-    // inverted by its adjugate on 16 lanes, the multipliers F_i = W(i, bb)
-    // P^-1 are formed once per row
-    constexpr int CG = XC_THREADS / UM_KP;      // threads per row
-    const int ri = tid / CG, cg = tid % CG;   // row ri, columns cg, cg + CG, ...
-    for (int b = 0; b < nb; ++b) {
-      const int b0 = b * dim;
-      if (warp == 0) {
-        if (lane < dim * dim) s_pb[lane] = Wf[(b0 + lane % dim) * XC_LD + b0 + lane / dim];   // column-major P
-        __syncwarp();
-        const float2 det = wf_det(dim, s_pb, lane);
-        if (lane == 0 && !(det.x * det.x + det.y * det.y > 0.f)) atomicExch(d.err, PQMC_ERR_SINGULAR);
-        wf_inverse(dim, s_pb, det, lane);   // s_pb <- P^-1
-      }
-      for (int e = tid; e < dim * K; e += XC_THREADS) {   // pivot rows and pivot columns before the step
-        const int m = e / K, j = e % K;
-        s_row[m * UM_KP + j] = Wf[(b0 + m) * XC_LD + j];
-        s_col[m * UM_KP + j] = Wf[j * XC_LD + b0 + m];
-      }
-      __syncthreads();
-      if (ri < K) {
-        const bool piv_row = ri >= b0 && ri < b0 + dim;
-        float2 f[4];   // piv_row: row ri - b0 of P^-1; else F_ri = W(ri, bb) P^-1
+          f[m] = make_float2(__shfl_sync(0xffffffffu, own.x, (lane & 24) + m), __shfl_sync(0xffffffffu, own.y, (lane & 24) + m));
+      } else {
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
+        for (int n = 0; n < DIM; ++n) {
           f[n] = make_float2(0.f, 0.f);
-          if (n >= dim) continue;
-          if (piv_row) {
-            f[n] = s_pb[(ri - b0) + dim * n];
+          if (piv) {
+            f[n] = s_pb[par][ri - b0 + DIM * n];
           } else {
 #pragma unroll
-            for (int m = 0; m < 4; ++m)
-              if (m < dim) f[n] = fcfma(s_col[m * UM_KP + ri], s_pb[m + dim * n], f[n]);
+            for (int m = 0; m < DIM; ++m) f[n] = fcfma(s_col[par][m][ri], s_pb[par][m + DIM * n], f[n]);
+            f[n] = make_float2(-f[n].x, -f[n].y);
           }
-        }
-        for (int j = cg; j < K; j += CG) {
-          float2 v;
-          if (j >= b0 && j < b0 + dim) {
-            v = piv_row ? f[j - b0] : make_float2(-f[j - b0].x, -f[j - b0].y);
-          } else {
-            v = piv_row ? make_float2(0.f, 0.f) : Wf[ri * XC_LD + j];
-#pragma unroll
-            for (int m = 0; m < 4; ++m)
-              if (m < dim) {
-                const float2 r = s_row[m * UM_KP + j];
-                v = piv_row ? fcfma(f[m], r, v) : fsb(v, fm(f[m], r));
-              }
-          }
-          Wf[ri * XC_LD + j] = v;
         }
       }
-      __syncthreads();
+#pragma unroll
+      for (int m = 0; m < DIM; ++m)
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+          const float4 r = *reinterpret_cast<const float4*>(&s_row[par][m][c0 + j]);
+          w[j] = fcfma(f[m], make_float2(r.x, r.y), w[j]);
+          w[j + 1] = fcfma(f[m], make_float2(r.z, r.w), w[j + 1]);
+        }
     }
-    for (int e = tid; e < K * K; e += XC_THREADS) d.v0[(e / K) * XC_LD + e % K] = Wf[(e / K) * XC_LD + e % K];
-    return;
+    if (b + 1 < nb) publish(b + 1);
+  }
+  if (ri < K) {
+#pragma unroll
+    for (int j = 0; j < 8; j += 2)
+      *reinterpret_cast<float4*>(d.v0 + (size_t)ri * XC_LD + c0 + j) = make_float4(w[j].x, w[j].y, w[j + 1].x, w[j + 1].y);
   }
 }
 
@@ -170,12 +181,15 @@ __global__ void __launch_bounds__(XC_THREADS, 1) k_xinv(const XDesc* X, int dim,
 //   CTAs 0 .. XS_RCTAS-1 (per 16 rows): 16 threads per row, 4 k each; the
 //   row's exponent from the largest |hi| over its K entries (a max over the
 //   16 lanes of the row), then 8-byte stores of 4 BF16 per slice.
-//   CTAs past them (per 8 columns): a warp per column of Z, 2 k per lane,
+//   The next (per 8 columns): a warp per column of Z, 2 k per lane,
 //   into the column tiles of the flush kernel in use (64 or 32 columns).
+//   The last XS_WCTAS: W = I + G(S,S) Delta_S in double-float, a row's
+//   entries of one move per thread (on one CTA of k_xinv, 4 us of its time).
 constexpr int XS_THREADS = 256;
 constexpr int XS_ROWS = XS_THREADS / 16;   // rows of G(:,S) per CTA
 constexpr int XS_COLS = XS_THREADS / 32;   // columns of Z per CTA
-__global__ void __launch_bounds__(XS_THREADS, 4) k_xslice(const XDesc* X, int parity, int n_rcta, int ct) {
+constexpr int XS_WCTAS = 4;
+__global__ void __launch_bounds__(XS_THREADS, 4) k_xslice(const XDesc* X, int parity, int n_rcta, int ct, int dim) {
   const XDesc& d = X[blockIdx.y];
   const int K = *d.kcount;
   if (K == 0) return;
@@ -220,6 +234,29 @@ __global__ void __launch_bounds__(XS_THREADS, 4) k_xslice(const XDesc* X, int pa
       unsigned char* im = d.img + (size_t)oz_slot_a1(ns, t, sl) * UM_IMG;
       *reinterpret_cast<uint2*>(im + um_off(row, kg * 8, nrg) + half) = make_uint2(wr[sl][0], wr[sl][1]);
       *reinterpret_cast<uint2*>(im + um_off(row, UM_KP + kg * 8, nrg) + half) = make_uint2(wi[sl][0], wi[sl][1]);
+    }
+    return;
+  }
+  const int wb = (int)blockIdx.x - ((int)gridDim.x - XS_WCTAS);
+  if (wb >= 0) {
+    // ---- W(i, jb*dim + jj) = delta_ij + sum_m G(S_i, S_{jb dim + m}) Delta_jb(m, jj)
+    const int nb = K / dim;
+    for (int it = wb * XS_THREADS + tid; it < K * nb; it += XS_WCTAS * XS_THREADS) {
+      const int i = it % K, jb = it / K;
+      const float4* dl = d.acc_delta + (size_t)jb * 16;
+      dfc gs[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        if (m < dim) gs[m] = dg_dfc(G[S[i] + (size_t)ns * S[jb * dim + m]]);
+#pragma unroll 1
+      for (int jj = 0; jj < dim; ++jj) {
+        const int j = jb * dim + jj;
+        dfc a = dfc{df{i == j ? 1.f : 0.f, 0.f}, df{0.f, 0.f}};
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (m < dim) a = dfc_mac(a, gs[m], dg_dfc(dl[m + dim * jj]));
+        d.wdf[(size_t)j * XC_LD + i] = dfc_dg(a);   // column-major: k_xres reads W(i, k) for consecutive i
+      }
     }
     return;
   }
@@ -1011,7 +1048,6 @@ __global__ void __launch_bounds__(XP_THREADS, 1) k_xflushp(const XDesc* X, int p
 }
 
 int exact_setup() {
-  PQMC_CUDA(raise_dyn_smem(k_xinv, (int)XI_SMEM));
   PQMC_CUDA(raise_dyn_smem(k_xres, (int)XR_SMEM));
   PQMC_CUDA(raise_dyn_smem(k_xgemm<0>, XG_SMEM));
   PQMC_CUDA(raise_dyn_smem(k_xgemm<1>, XG_SMEM));
@@ -1024,9 +1060,15 @@ int exact_core(const XDesc* d_x, int C, int ns, int dim, int parity, int ct, cud
                int prio_hi) {
   const int n_r = (ns + XS_ROWS - 1) / XS_ROWS, n_c = (ns + XS_COLS - 1) / XS_COLS;
   const int zw = ct == 64 ? 64 : 32;   // Z's tile width: 64 for k_xgemm<1>, 32 for k_xflush2 and k_xflushp
-  PQMC_CUDA(launch_at(k_xslice, dim3(n_r + n_c, C), dim3(XS_THREADS), 0, st, prio, prio_hi, d_x, parity, n_r, zw));
+  PQMC_CUDA(launch_at(k_xslice, dim3(n_r + n_c + XS_WCTAS, C), dim3(XS_THREADS), 0, st, prio, prio_hi, d_x, parity, n_r, zw,
+                      dim));
   PQMC_LAUNCHED();
-  PQMC_CUDA(launch_at(k_xinv, dim3(1, C), dim3(XC_THREADS), XI_SMEM, st, prio, prio_hi, d_x, dim, parity));
+  switch (dim) {
+    case 1: PQMC_CUDA(launch_at(k_xinv<1>, dim3(1, C), dim3(XC_THREADS), 0, st, prio, prio_hi, d_x)); break;
+    case 2: PQMC_CUDA(launch_at(k_xinv<2>, dim3(1, C), dim3(XC_THREADS), 0, st, prio, prio_hi, d_x)); break;
+    case 3: PQMC_CUDA(launch_at(k_xinv<3>, dim3(1, C), dim3(XC_THREADS), 0, st, prio, prio_hi, d_x)); break;
+    default: PQMC_CUDA(launch_at(k_xinv<4>, dim3(1, C), dim3(XC_THREADS), 0, st, prio, prio_hi, d_x)); break;
+  }
   PQMC_LAUNCHED();
   PQMC_CUDA(launch_at(k_xres, dim3(XR_CTAS, C), dim3(XR_THREADS), XR_SMEM, st, prio, prio_hi, d_x, dim, parity));
   PQMC_LAUNCHED();

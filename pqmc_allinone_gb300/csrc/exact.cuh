@@ -12,8 +12,9 @@
 // are the sequential ratio matrices R_j = I + Geff_j(S_j,S_j) Delta_j of the
 // reference.)  The update is evaluated from the double-float G, never from
 // the scan's FP32 panels:
-//   k_xslice  the Ozaki slices of G(:,S) and of Z = E_S - G(S,:);
-//   k_xinv    W in double-float and the FP32 inverse V0 of its rounding;
+//   k_xslice  the Ozaki slices of G(:,S) and of Z = E_S - G(S,:), and W in
+//             double-float;
+//   k_xinv    the FP32 inverse V0 of W's rounding;
 //   k_xres    one Newton step V1 = V0 + V0 (I - W V0) with a double-float
 //             residual, M = Delta_S V1 and the Ozaki slices of M;
 //   k_xgemm   X = G(:,S) M, then G += X Z, on the tensor cores: every
