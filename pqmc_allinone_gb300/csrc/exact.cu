@@ -61,7 +61,9 @@ constexpr size_t XR_SMEM = sizeof(float4) * ((size_t)XC_LD * XC_LD + 16 * UM_KP 
                            sizeof(float2) * (size_t)XC_LD * XC_LD;
 
 // FP32 Gauss-Jordan of W's rounding, W in registers: eight threads per row,
-// eight adjacent columns each, four rows per warp.  A step needs its pivot
+// eight columns each (pairs 16 apart, so that a row's eight 16-byte reads of
+// a pivot row fall into different banks: eight adjacent columns each made
+// every read a four-way conflict, 3700 cycles a step), four rows per warp.  A step needs its pivot
 // rows, the pivot columns and P^-1 in shared memory, two buffers in turn, and
 // one barrier: having updated its rows, every thread publishes what the next
 // step needs of them, and the warp that holds the next pivot rows (all of
@@ -78,12 +80,13 @@ __global__ void __launch_bounds__(XC_THREADS, 1) k_xinv(const XDesc* X) {
   __shared__ float2 s_col[2][DIM][UM_KP];
   __shared__ float2 s_pb[2][16];
   const int tid = threadIdx.x, lane = tid & 31;
-  const int ri = tid >> 3, c0 = 8 * (tid & 7);   // row ri, columns c0 .. c0 + 7
+  const int ri = tid >> 3, c0 = 2 * (tid & 7);   // row ri, columns col(0) .. col(7)
+  auto col = [&](int j) { return c0 + 16 * (j >> 1) + (j & 1); };
   const int nb = K / DIM;
   float2 w[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j)
-    w[j] = (ri < K && c0 + j < K) ? hi2(d.wdf[(size_t)(c0 + j) * XC_LD + ri]) : make_float2(0.f, 0.f);
+    w[j] = (ri < K && col(j) < K) ? hi2(d.wdf[(size_t)col(j) * XC_LD + ri]) : make_float2(0.f, 0.f);
   // P^-1 by one warp, in place (column-major)
   auto invert = [&](int par) {
     __syncwarp();
@@ -99,7 +102,7 @@ __global__ void __launch_bounds__(XC_THREADS, 1) k_xinv(const XDesc* X) {
     const bool piv = ri >= b0 && ri < b0 + DIM;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int c = c0 + j - b0;
+      const int c = col(j) - b0;
       if (c >= 0 && c < DIM) {
         s_col[par][c][ri] = w[j];
         if (piv) s_pb[par][ri - b0 + DIM * c] = w[j];
@@ -109,7 +112,7 @@ __global__ void __launch_bounds__(XC_THREADS, 1) k_xinv(const XDesc* X) {
     if (piv) {
 #pragma unroll
       for (int j = 0; j < 8; j += 2)
-        *reinterpret_cast<float4*>(&s_row[par][ri - b0][c0 + j]) = make_float4(w[j].x, w[j].y, w[j + 1].x, w[j + 1].y);
+        *reinterpret_cast<float4*>(&s_row[par][ri - b0][col(j)]) = make_float4(w[j].x, w[j].y, w[j + 1].x, w[j + 1].y);
 #pragma unroll
       for (int j = 0; j < 8; ++j) w[j] = make_float2(0.f, 0.f);
     }
@@ -159,7 +162,7 @@ __global__ void __launch_bounds__(XC_THREADS, 1) k_xinv(const XDesc* X) {
       for (int m = 0; m < DIM; ++m)
 #pragma unroll
         for (int j = 0; j < 8; j += 2) {
-          const float4 r = *reinterpret_cast<const float4*>(&s_row[par][m][c0 + j]);
+          const float4 r = *reinterpret_cast<const float4*>(&s_row[par][m][col(j)]);
           w[j] = fcfma(f[m], make_float2(r.x, r.y), w[j]);
           w[j + 1] = fcfma(f[m], make_float2(r.z, r.w), w[j + 1]);
         }
@@ -169,7 +172,7 @@ __global__ void __launch_bounds__(XC_THREADS, 1) k_xinv(const XDesc* X) {
   if (ri < K) {
 #pragma unroll
     for (int j = 0; j < 8; j += 2)
-      *reinterpret_cast<float4*>(d.v0 + (size_t)ri * XC_LD + c0 + j) = make_float4(w[j].x, w[j].y, w[j + 1].x, w[j + 1].y);
+      *reinterpret_cast<float4*>(d.v0 + (size_t)ri * XC_LD + col(j)) = make_float4(w[j].x, w[j].y, w[j + 1].x, w[j + 1].y);
   }
 }
 
