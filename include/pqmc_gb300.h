@@ -449,9 +449,9 @@ int pqmc_batch_get_flush_tile(pqmc_batch* batch, int* ct);
  * agree to the products' rounding, not bit for bit.  Mixed batches only. */
 int pqmc_batch_set_gemm_engine(pqmc_batch* batch, int engine);
 int pqmc_batch_get_gemm_engine(pqmc_batch* batch, int* engine);
-/* Panel columns per streamed chunk of the scan (k_bscan's TMA stream of the
- * delayed panels through three shared-memory stages): 1 .. qc_max, the
- * largest chunk that fits (at most 8; the default).  The chunking does not
+/* Panel columns that a thread of the scan has in flight as it reads back
+ * those that do not stay in shared memory (in even numbers, at least 2):
+ * 1 .. qc_max, the most that fit (at most 8; the default).  It does not
  * change the arithmetic, so the chains are bit-identical whichever runs.
  * qc_max may be NULL.  Uneven batches: set for every class, get the first
  * class's. */

@@ -5,7 +5,7 @@
 // Mixed-precision family step (one launch per phase for all chains):
 //   k_bdraw   ran2 stream of every chain for the step
 //   k_bprep   per-plaquette proposal data (as phase 1 of k_update)
-//   k_bscan   one CTA per chain walks its plaquettes in Markov order; an
+//   k_bscan   one CTA (or a cluster) per chain walks its plaquettes in Markov order; an
 //             accepted move appends a rank-dim column block to the FP32
 //             delayed-update panels A (Ns x K) and B (K x Ns), so later
 //             ratios see G + A B without touching G (delayed updates)
@@ -49,16 +49,11 @@ struct BDesc {
   float2* A;     // (kmax, ldp): A[q*ldp + r]
   float2* B;     // (kmax, ldp): B[q*ldp + c]
   int kmax;
-  int ldp;       // panel leading dimension: Ns rounded up to even (16-byte columns)
+  int ldp;       // panel leading dimension: Ns rounded up to a multiple of 4 (whole row groups of a thread)
   int* err;      // batch-wide error word (PQMC_ERR_* of a device-side failure)
   PlaqPre* pre;
   DevScalars* sc;
   int* kcount;
-  // TMA tensor maps over the two G buffers (double-float, Ns rows x Ns
-  // columns, a row read as nrb boxes of rb columns)
-  const CUtensorMap* tm_g;
-  const CUtensorMap* tm_galt;
-  int rb, nrb;
   int t;         // 0-based time index of the slice in progress (k_bsettime)
   unsigned long long* nflush;   // flush rounds with work (for the roofline accounting)
   // the round's accepted moves for the exact update (exact.cuh)
@@ -206,7 +201,7 @@ __global__ void __launch_bounds__(256) k_bprep(const BDesc* D, int pf_first, int
 }
 
 // ---------------------------------------------------------------------------
-// Sequential scan with delayed updates, one CTA per chain.  The scan resumes
+// Sequential scan with delayed updates, one CTA or cluster per chain.  The scan resumes
 // at the chain's next plaquette and stops when the panels hold `kd` columns
 // (the delay depth); k_bflush then folds them into G and the next round
 // continues.  Ratios, R^-1 and T are FP32 (the panels are FP32); the weight
@@ -215,73 +210,161 @@ __global__ void __launch_bounds__(256) k_bprep(const BDesc* D, int pf_first, int
 // Latency design: at the start of a round (panels empty) the kernel stages
 // the family's site table, the FP32 Delta and thresholds, and
 // Geff(S_p,S_p) = G(S_p,S_p) for every plaquette still to come in shared
-// memory.  Every warp evaluates each ratio redundantly from shared memory,
-// so a rejected proposal costs no block barrier and no global access.  An
-// accepted move builds its rank-dim panel block (one pass over the panels)
-// and adds its contribution to the cached Geff blocks of the later
-// plaquettes.
-constexpr int SCAN_THREADS = 512;
+// memory.  Every warp evaluates one of the next proposals from shared memory,
+// so a rejected proposal costs no global access.  An accepted move builds its
+// rank-dim panel block (one pass over the panels) and adds its contribution
+// to the cached Geff blocks of the later plaquettes.
+//
+// What bounds it is the pass over the panels (28 columns on average at depth
+// 64).  The round's first `res` columns therefore stay in shared memory where
+// the CTA itself wrote them (all 64 up to Ns ~ 190, 16 at Ns = 392), and only
+// the later ones are read back, each thread its own rows through a private
+// ring of a few columns, so that no barrier is needed; the accepted
+// sites' entries of those columns are gathered once per move by the warps that
+// hold no row.  The same warps fetch G(:,S) and G(S,:) beside the pass, into
+// the place of the block to come.  Streaming every column through shared
+// memory with bulk copies cost 440 cycles a column at Ns = 392 and 210 at Ns =
+// 72, nearly all of it waiting for the copies; now a column costs 71 cycles at
+// Ns = 72, 130 at 160, 105 at 392 in a cluster of four CTAs, and 350 at 392 in
+// one CTA.  With all columns resident the row warps are doubled and the
+// sites halved between the two sets (SH = 2): a column at Ns = 160 cost 230.
+//
+// A chain's rows can be spread over a cluster of CTAs.  Each scans all
+// proposals alike, holds its rows of the panels, gathers the sites' entries
+// from the CTA that has them and writes its rows of a new block into every
+// CTA's copy (two copies in turn: one CTA may still read the last block as
+// another writes the next); one cluster barrier per accepted move.
+constexpr int SCAN_THREADS = 384;
 constexpr int SCAN_KSTAGE = 512;   // max delay depth (panel columns)
-
-constexpr int SCAN_NSTAGE = 3;   // panel chunks in flight
-constexpr int SCAN_RPT = 2;      // rows per thread: Ns <= SCAN_RPT * SCAN_THREADS
+constexpr int SCAN_GAT = 64;       // columns gathered at a time
+constexpr int SCAN_MAX_NS = 4 * (SCAN_THREADS - 128);   // 4 rows per thread and a spare warp
+constexpr int SCAN_SH_ROWS = 320;  // rows up to which two sets of row warps leave two spare ones
+constexpr int SCAN_RING = 8;       // columns read back that a thread has in flight, at most
+constexpr int SCAN_GLOAD = 2;      // items of G (two sites, column and row each) a thread has in flight
 
 __host__ __device__ __forceinline__ size_t al16(size_t b) { return (b + 15) & ~(size_t)15; }
 
-// dynamic shared memory of k_bscan (byte offsets, 16-byte aligned pieces)
+// dynamic shared memory of k_bscan (byte offsets, 16-byte aligned pieces):
+// `res` resident panel columns of A and B, a slot of 4 for a block past them,
+// and the ring where there can be such blocks
 struct ScanLayout {
-  size_t rows, stage, delta, geff, newA, newB, thr, site, accp, accd, total;
+  size_t pa, pb, ring, nw, delta, geff, gat, thr, site, accp, accd, total;
 };
-// rows first: the TMA tile destination wants a 128-byte aligned address
-__host__ __device__ __forceinline__ ScanLayout scan_layout(int npla, int ns, int ldp, int qc, int kd, int rows_bytes) {
+// rows of G of one CTA of a cluster of nc (a multiple of 4)
+__host__ __device__ __forceinline__ int scan_rows(int ns, int nc) { return ((ns + nc - 1) / nc + 3) & ~3; }
+__host__ __device__ __forceinline__ ScanLayout scan_layout(int npla, int ldp, int res, int kd, int nc, int ring) {
   ScanLayout L;
   size_t o = 0;
-  L.rows = o;  o += (size_t)((rows_bytes + 127) & ~127);
-  L.stage = o; o += al16(sizeof(float2) * (size_t)SCAN_NSTAGE * 2 * qc * ldp);
+  const int lr = nc > 1 ? scan_rows(ldp, nc) : ldp;
+  const int cols = res + (res < kd ? 4 : 0);
+  L.pa = o;    o += al16(sizeof(float2) * (size_t)cols * lr);
+  L.pb = o;    o += al16(sizeof(float2) * (size_t)cols * lr);
+  L.ring = o;  o += res < kd ? al16(sizeof(float2) * 2 * ring * (size_t)lr) : 0;
+  L.nw = o;    o += nc > 1 ? al16(sizeof(float2) * 2 * 8 * (size_t)ldp) : 0;
   L.delta = o; o += al16(sizeof(float2) * 16 * (size_t)npla);
   L.geff = o;  o += al16(sizeof(float2) * 16 * (size_t)npla);
-  L.newA = o;  o += al16(sizeof(float2) * 4 * (size_t)ns);
-  L.newB = o;  o += al16(sizeof(float2) * 4 * (size_t)ns);
-  L.thr = o;   o += al16(sizeof(double) * (size_t)npla);
+  L.gat = o;   o += al16(sizeof(float4) * 8 * SCAN_GAT);
+  L.thr = o;   o += al16(sizeof(float) * (size_t)npla);
   L.site = o;  o += al16(sizeof(int) * 4 * (size_t)npla);
   L.accp = o;  o += al16(sizeof(int) * (size_t)kd);
   L.accd = o;  o += al16(sizeof(float2) * (size_t)kd);
   L.total = o;
   return L;
 }
+// rows of G per thread, in adjacent pairs
+__host__ __device__ constexpr int scan_rpt(int ns) { return ns <= 2 * (SCAN_THREADS - 128) ? 2 : 4; }
 
-// thread 0: stream panel columns [c*qc, c*qc+nq) of A and B into stage c % NSTAGE
-__device__ __forceinline__ void scan_issue(float2* s_stage, uint64_t* s_full, const float2* A, const float2* B,
-                                           int ldp, int qc, int K, int c) {
-  const int st = c % SCAN_NSTAGE, q0 = c * qc, nq = min(qc, K - q0);
-  const uint32_t bytes = (uint32_t)(sizeof(float2) * (size_t)nq * ldp);
-  float2* dA = s_stage + (size_t)st * 2 * qc * ldp;
-  float2* dB = dA + (size_t)qc * ldp;
-  mbar_arrive_tx(&s_full[st], 2 * bytes);
-  bulk_g2s(dA, A + (size_t)q0 * ldp, bytes, &s_full[st]);
-  bulk_g2s(dB, B + (size_t)q0 * ldp, bytes, &s_full[st]);
+// Two FP32 values side by side, for the packed multiply-add (two IEEE
+// multiply-adds in one instruction; the panel pass is bound by their issue).
+struct f32x2 {
+  float a, b;
+};
+__device__ __forceinline__ f32x2 fma2(f32x2 x, f32x2 y, f32x2 z) {
+  unsigned long long r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%1, %2};\n mov.b64 y, {%3, %4};\n mov.b64 z, {%5, %6};\n"
+      " fma.rn.f32x2 %0, x, y, z;\n}"
+      : "=l"(r)
+      : "f"(x.a), "f"(x.b), "f"(y.a), "f"(y.b), "f"(z.a), "f"(z.b));
+  f32x2 o;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(o.a), "=f"(o.b) : "l"(r));
+  return o;
+}
+// The panel entries of a pair of rows, re and im apart: in shared memory the
+// four words of a pair are {x0, x1, y0, y1}.
+struct Pair {
+  f32x2 x, y;
+};
+__device__ __forceinline__ Pair pair_of(float4 v) { return Pair{{v.x, v.y}, {v.z, v.w}}; }
+__device__ __forceinline__ float4 pair_words(Pair p) { return make_float4(p.x.a, p.x.b, p.y.a, p.y.b); }
+__device__ __forceinline__ f32x2 neg2(f32x2 v) { return f32x2{-v.a, -v.b}; }
+// entry r of a column stored by pairs
+__device__ __forceinline__ float2 pair_entry(const float4* col, int r) {
+  const float* f = reinterpret_cast<const float*>(col + (r >> 1)) + (r & 1);
+  return make_float2(f[0], f[2]);
+}
+__device__ __forceinline__ void pair_put(float4* col, int r, float2 v) {
+  float* f = reinterpret_cast<float*>(col + (r >> 1)) + (r & 1);
+  f[0] = v.x;
+  f[2] = v.y;
 }
 
-template <int DIM, int RPT>
-__global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, int parity, int kd, int qc,
-                                                         int* next_p, int exact, int prof) {
+// a thread's own pair of rows of a global panel column into shared memory, asynchronously
+__device__ __forceinline__ void scan_fetch(float4* dst, const float2* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+// one panel column onto a thread's row pairs: gm += A(r, q) B(q, S), bl +=
+// A(S, q) B(q, r), each complex product as fcfma forms it.  gat: the sites'
+// entries as {x, x, y, y}, B(q, S) then A(S, q).
+template <int DIM, int NP>
+__device__ __forceinline__ void scan_col(const Pair (&ar)[NP], const Pair (&bc)[NP], const float4* gat,
+                                         Pair (&gm)[NP][DIM], Pair (&bl)[NP][DIM]) {
+  f32x2 nay[NP], nby[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    nay[k] = neg2(ar[k].y);
+    nby[k] = neg2(bc[k].y);
+  }
+#pragma unroll
+  for (int m = 0; m < DIM; ++m) {
+    const float4 gb = gat[m], ga = gat[4 + m];
+    const f32x2 bx{gb.x, gb.y}, by{gb.z, gb.w}, ax{ga.x, ga.y}, ay{ga.z, ga.w};
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      gm[k][m].x = fma2(ar[k].x, bx, fma2(nay[k], by, gm[k][m].x));
+      gm[k][m].y = fma2(ar[k].x, by, fma2(ar[k].y, bx, gm[k][m].y));
+      bl[k][m].x = fma2(ax, bc[k].x, fma2(ay, nby[k], bl[k][m].x));
+      bl[k][m].y = fma2(ax, bc[k].y, fma2(ay, bc[k].x, bl[k][m].y));
+    }
+  }
+}
+
+// shared memory of another CTA of the cluster
+__device__ __forceinline__ uint32_t mapa(const void* p, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// RPT rows per thread; SH = 2: the accepted sites are halved between two sets
+// of row warps (twice the warps, half the multiply-adds each)
+template <int DIM, int RPT, int SH>
+__global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, int parity, int kd, int res_max, int nc,
+                                                         int ring, int* next_p, int exact, int prof) {
   const long long t_start = prof ? clock64() : 0;
-  constexpr int NW = SCAN_THREADS / 32;
+  constexpr int NW = SCAN_THREADS / 32, NP = RPT / 2, DS = DIM / SH;
   __shared__ BDesc sd;
   __shared__ float2 s_R[NW][16];
   __shared__ float2 s_T[16];
   __shared__ float2 s_det[NW];
-  __shared__ int s_dec[NW];
-  __shared__ __align__(8) uint64_t s_full[SCAN_NSTAGE];
-  __shared__ __align__(8) uint64_t s_rowbar;
-  __shared__ int s_abort;
+  __shared__ unsigned s_mask[2];   // accepted proposals of a pass, two passes in turn
   extern __shared__ __align__(1024) unsigned char s_dyn[];
   if (threadIdx.x == 0) {
-    sd = D[blockIdx.x];
-    s_abort = 0;
-    for (int k = 0; k < SCAN_NSTAGE; ++k) mbar_init(&s_full[k], 1);
-    mbar_init(&s_rowbar, 1);
-    fence_mbar_init();
+    sd = D[blockIdx.x / nc];
+    s_mask[0] = s_mask[1] = 0;
   }
   __syncthreads();
   const BDesc& d = sd;
@@ -290,31 +373,37 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
   constexpr int dim = DIM, dd = DIM * DIM;
   const int ns = M.ns, npla = M.pf_npla[pf], pd = M.pdim, ldp = d.ldp;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int p0 = next_p[blockIdx.x];
-  // the thread that drives the copy engine: lane 0 of the last warp when that
-  // warp holds no row of G (its issue cost stays off the row workers' path)
-  if (p0 >= npla) {
-    if (tid == 0) *d.kcount = 0;
+  const int chain = blockIdx.x / nc, rank = blockIdx.x % nc;   // CTA `rank` of the chain's cluster
+  const int p0 = next_p[chain];
+  if (p0 >= npla) {   // the cluster's CTAs alike
+    if (tid == 0 && rank == 0) *d.kcount = 0;
     return;
   }
-  const int rb = d.rb, nrb = d.nrb;
-  const int io = (ns <= SCAN_THREADS - 32) ? SCAN_THREADS - 32 : 0;
-  const bool row_warp = warp * 32 < ns;   // holds a row of G (every warp when RPT = 2)
-  // a warp with no row of G that is not the copy-engine warp
-  const int inv_warp = (RPT == 1 && ns <= SCAN_THREADS - 64) ? SCAN_THREADS / 32 - 2 : -1;
-  const ScanLayout L = scan_layout(npla, ns, ldp, qc, kd, 4 * nrb * rb * (int)sizeof(float4));
-  float4* s_rows = reinterpret_cast<float4*>(s_dyn + L.rows);     // [dim][nrb*rb] rows of G at S
-  float2* s_stage = reinterpret_cast<float2*>(s_dyn + L.stage);
+  const int res = res_max - res_max % dim;   // whole blocks are resident or not
+  // the panels themselves are read by this kernel past `res`, and by the FP32 flushes
+  const bool to_global = !exact || kd > res;
+  // the CTA's rows lo .. hi - 1 of G, the thread's r0 ..
+  const int nr = nc > 1 ? scan_rows(ldp, nc) : ldp, lo = rank * nr, hi = min(ns, lo + nr);
+  const int n_w1 = max(0, hi - lo + 32 * RPT - 1) / (32 * RPT), n_rw = SH * n_w1;   // warps per set, row warps; the last warp is spare
+  const int set = SH > 1 && warp >= n_w1 ? 1 : 0, m0 = set * DS;   // the thread's sites m0 .. m0 + DS - 1
+  const int pt = tid - 32 * n_w1 * set;                            // its place in the set
+  const int r0 = lo + RPT * pt;
+  const bool row = warp < n_rw && r0 < hi;
+  constexpr int inv_warp = NW - 1;
+  const ScanLayout L = scan_layout(npla, ldp, res_max, kd, nc, ring);
+  const int lp = nr / 2;    // row pairs of a column here
+  float4* s_pa = reinterpret_cast<float4*>(s_dyn + L.pa);         // [res + 4][lp]
+  float4* s_pb = reinterpret_cast<float4*>(s_dyn + L.pb);
+  float4* s_ring = reinterpret_cast<float4*>(s_dyn + L.ring);     // [ring][A, B][lp], as in global memory
+  float4* s_nw = reinterpret_cast<float4*>(s_dyn + L.nw);         // nc > 1: [2][A, B][4][ldp / 2], new blocks of all rows
   float2* s_delta = reinterpret_cast<float2*>(s_dyn + L.delta);   // [npla][16]
   float2* s_geff = reinterpret_cast<float2*>(s_dyn + L.geff);     // [npla][16]
-  float2* s_newA = reinterpret_cast<float2*>(s_dyn + L.newA);     // [4][ns]
-  float2* s_newB = reinterpret_cast<float2*>(s_dyn + L.newB);     // [4][ns]
-  double* s_thr = reinterpret_cast<double*>(s_dyn + L.thr);
+  float4* s_gat = reinterpret_cast<float4*>(s_dyn + L.gat);       // [SCAN_GAT][8]: {x, x, y, y} of B(q, S), A(S, q)
+  float* s_thr = reinterpret_cast<float*>(s_dyn + L.thr);
   int* s_site = reinterpret_cast<int*>(s_dyn + L.site);           // [npla][4]
   int* s_accp = reinterpret_cast<int*>(s_dyn + L.accp);
   float2* s_accd = reinterpret_cast<float2*>(s_dyn + L.accd);
   const float4* G = reinterpret_cast<const float4*>(parity ? d.g_alt : d.g);   // double-float G
-  const CUtensorMap* tmG = parity ? d.tm_galt : d.tm_g;
   float2* A = d.A;
   float2* B = d.B;
   const PlaqPre* pre = d.pre + (size_t)pf * M.max_pla;
@@ -323,7 +412,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
     const int p = p0 + e / 4, m = e % 4;
     s_site[4 * p + m] = m < dim ? M.site[m + pd * (p + M.max_pla * pf)] : 0;
   }
-  for (int p = p0 + tid; p < npla; p += blockDim.x) s_thr[p] = pre[p].thr;
+  // x >= thr and x >= (thr rounded up to FP32) agree for every FP32 x, and an
+  // FP64 comparison per proposal would cost a pass 500 cycles
+  for (int p = p0 + tid; p < npla; p += blockDim.x) s_thr[p] = __double2float_ru(pre[p].thr);
   for (int e = tid; e < (npla - p0) * 16; e += blockDim.x) {
     const int p = p0 + e / 16, k = e % 16;
     if (k < dd) s_delta[16 * p + k] = pre[p].deltaf[k];
@@ -334,13 +425,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
     if (k < dd) s_geff[16 * p + k] = dg_f2(G[s_site[4 * p + k % dim] + (size_t)ns * s_site[4 * p + k / dim]]);
   }
   __syncthreads();
+  if (nc > 1) cluster_barrier();   // every CTA runs: its shared memory may be written
   int K = 0, n_acc = 0;
   long long na = 0;
-  uint32_t phase = 0;   // bit s: parity of the next completion of stage s
-  uint32_t rowphase = 0;
-  int npre = 0;         // panel chunks already in flight for the next accepted move
-  bool aborted = false;
-  int p = p0;
+  int p = p0, pass = 0;
   const int i = lane % dim, j = lane / dim;
   const bool act = lane < dd;
   while (p < npla && K + dim <= kd) {
@@ -348,8 +436,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
     //      Geff (valid for every proposal up to the first accepted one) ------
     {
       const int pw = p + warp;
-      int dec = 0;
-      float2 det = make_float2(0.f, 0.f);
       if (pw < npla) {
         const float2* ge = s_geff + 16 * pw;
         const float2* de = s_delta + 16 * pw;
@@ -360,33 +446,34 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
           s_R[warp][lane] = a;
         }
         __syncwarp();
-        det = wf_det(dim, s_R[warp], lane);
+        const float2 det = wf_det(dim, s_R[warp], lane);
         const float dm = det.x * det.x + det.y * det.y;
-        dec = ((double)dm >= s_thr[pw]) ? 1 : 0;
-      }
-      if (lane == 0) {
-        s_dec[warp] = dec;
-        s_det[warp] = det;
+        if (lane == 0) {
+          s_det[warp] = det;
+          if (dm >= s_thr[pw]) atomicOr(&s_mask[pass & 1], 1u << warp);
+        }
       }
     }
     __syncthreads();
-    int wa = -1;
-    for (int w = 0; w < NW && p + w < npla; ++w)
-      if (s_dec[w]) { wa = w; break; }
-    if (wa < 0) {   // all evaluated proposals rejected
+    const unsigned mask = s_mask[pass & 1];
+    if (tid == 0) s_mask[(pass & 1) ^ 1] = 0;   // read in the last pass, written in the next, a barrier from both
+    ++pass;
+    if (!mask) {   // all evaluated proposals rejected
       const int nrej = min(NW, npla - p);
       if (tid == 0) na += nrej;
       p += nrej;
-      __syncthreads();   // s_dec / s_R are rewritten by the next pass
+      __syncthreads();   // s_R is rewritten by the next pass
       continue;
     }
+    const int wa = __ffs(mask) - 1;
     if (tid == 0) na += wa;
     p += wa;
-    // ---- accepted move p: T = Delta R^-1, by a warp without rows of G when
-    //      there is one (its work then overlaps the row warps' panel loop),
-    //      else by the warp that evaluated the move -------------------------
-    const float2 det = s_det[wa];
-    if (warp == (inv_warp >= 0 ? inv_warp : wa)) {
+    int S[dim];
+#pragma unroll
+    for (int m = 0; m < dim; ++m) S[m] = s_site[4 * p + m];
+    // ---- accepted move p: T = Delta R^-1 by the spare warp, beside the panels
+    if (warp == inv_warp) {
+      const float2 det = s_det[wa];
       wf_inverse(dim, s_R[wa], det, lane);
       if (act) {
         const float2* de = s_delta + 16 * p;
@@ -401,145 +488,228 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
       }
     }
     ++n_acc;
-    const int* S = s_site + 4 * p;
-    const int nch = (K + qc - 1) / qc;
-    if (tid == io) {
-      // rows G(S_m, :) by the tensor engine (strided: one 16-byte element per column)
-      mbar_arrive_tx(&s_rowbar, (uint32_t)(dim * nrb * rb * sizeof(float4)));
-      for (int m = 0; m < dim; ++m)
-        for (int bx = 0; bx < nrb; ++bx) tma_load_2d(s_rows + (size_t)(m * nrb + bx) * rb, tmG, 4 * S[m], bx * rb, &s_rowbar);
-      if (nch > npre) {
-        if (npre == 0) fence_proxy_async_global();   // this round's panel columns were written by generic stores
-        for (int c = npre; c < nch && c < SCAN_NSTAGE; ++c) scan_issue(s_stage, s_full, A, B, ldp, qc, K, c);
-      }
-    }
-    npre = 0;
-    // rows of G at the accepted sites, loaded now and added after the panel
-    // loop (their latency overlaps it)
-    float4 gcol[RPT][dim];
-    float2 gm[RPT][dim], bl[RPT][dim];
+    const int n_res = min(K, res);
+    float4* new_a = s_pa + (size_t)(K < res ? K : res) * lp;   // the new block's columns in shared memory
+    float4* new_b = s_pb + (size_t)(K < res ? K : res) * lp;
+    // the block of all rows: the same, or this CTA's copy of it
+    const int lpa = ldp / 2;
+    float4* all_a = nc > 1 ? s_nw + (size_t)(n_acc & 1) * 8 * lpa : new_a;
+    float4* all_b = nc > 1 ? all_a + 4 * lpa : new_b;
+    // the thread's rows of the next `nb` columns into half `h` of the ring
+    auto fetch = [&](int q, int h, int nb) {
 #pragma unroll
-    for (int k = 0; k < RPT; ++k) {
-      const int r = tid + k * SCAN_THREADS;
+      for (int c = 0; c < SCAN_RING / 2; ++c)
+        if (c < nb && q + c < K)
 #pragma unroll
-      for (int m = 0; m < dim; ++m) {
-        gcol[k][m] = r < ns ? G[r + (size_t)ns * S[m]] : make_float4(0.f, 0.f, 0.f, 0.f);
-        gm[k][m] = make_float2(0.f, 0.f);
-        bl[k][m] = make_float2(0.f, 0.f);
-      }
-    }
-    for (int c = 0; c < nch; ++c) {
-      const int st = c % SCAN_NSTAGE;
-      if (!mbar_wait_bounded(&s_full[st], (phase >> st) & 1u)) s_abort = 1;
-      phase ^= 1u << st;
-      const float2* cA = s_stage + (size_t)st * 2 * qc * ldp;
-      const float2* cB = cA + (size_t)qc * ldp;
-      // warps without a row of G skip the column loop: the broadcast loads
-      // of the accepted sites' panel entries are its shared-memory bound
-      const int nq = row_warp ? min(qc, K - c * qc) : 0;
-#pragma unroll 2
-      for (int qq = 0; qq < nq; ++qq) {
-        float2 bs[dim], as[dim];
-#pragma unroll
-        for (int m = 0; m < dim; ++m) {
-          bs[m] = cB[(size_t)qq * ldp + S[m]];
-          as[m] = cA[(size_t)qq * ldp + S[m]];
-        }
-#pragma unroll
-        for (int k = 0; k < RPT; ++k) {
-          const int r = tid + k * SCAN_THREADS;
-          if (r < ns) {
-            const float2 ar = cA[(size_t)qq * ldp + r], bc = cB[(size_t)qq * ldp + r];
-#pragma unroll
-            for (int m = 0; m < dim; ++m) {
-              gm[k][m] = fcfma(ar, bs[m], gm[k][m]);
-              bl[k][m] = fcfma(as[m], bc, bl[k][m]);
-            }
+          for (int k = 0; k < NP; ++k) {
+            float4* dst = s_ring + (size_t)(2 * (nb * h + c)) * lp + NP * pt + k;
+            scan_fetch(dst, A + (size_t)(q + c) * ldp + r0 + 2 * k);
+            scan_fetch(dst + lp, B + (size_t)(q + c) * ldp + r0 + 2 * k);
           }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (SH == 1 && row && K > res) {   // the first columns to read back; with SH = 2 all are resident
+      fetch(res, 0, ring / 2);
+      fetch(res + ring / 2, 1, ring / 2);
+    }
+    Pair gm[NP][DS], bl[NP][DS];
+#pragma unroll
+    for (int k = 0; k < NP; ++k)
+#pragma unroll
+      for (int m = 0; m < DS; ++m) gm[k][m] = bl[k][m] = Pair{{0.f, 0.f}, {0.f, 0.f}};
+    int slot = 0;
+    for (int q0 = 0; q0 == 0 || q0 < K; q0 += SCAN_GAT) {
+      // the accepted sites' entries of the next columns
+      if (q0 > 0) __syncthreads();
+      const int qe = min(K, q0 + SCAN_GAT);
+      for (int e = tid; e < 8 * (qe - q0); e += SCAN_THREADS) {
+        const int q = q0 + (e >> 3), m = e & 3;
+        if (m < dim) {
+          const int sm = s_site[4 * p + m];
+          float2 v;
+          if (q >= res) {
+            v = __ldcg(((e & 4) ? A : B) + (size_t)q * ldp + sm);
+          } else if (nc == 1) {
+            v = pair_entry(((e & 4) ? s_pa : s_pb) + (size_t)q * lp, sm);
+          } else {
+            const int o = sm / nr, r = sm - o * nr;
+            const uint32_t at = mapa(((e & 4) ? s_pa : s_pb) + (size_t)q * lp + (r >> 1), o) + 4 * (r & 1);
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v.x) : "r"(at) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v.y) : "r"(at + 8) : "memory");
+          }
+          s_gat[e] = make_float4(v.x, v.x, v.y, v.y);
         }
       }
       __syncthreads();
-      if (s_abort) break;
-      if (tid == io && c + SCAN_NSTAGE < nch) scan_issue(s_stage, s_full, A, B, ldp, qc, K, c + SCAN_NSTAGE);
-    }
-    if (s_abort) {
-      aborted = true;
-      break;
-    }
-    if (nch == 0) __syncthreads();   // s_T visible
-    if (!mbar_wait_bounded(&s_rowbar, rowphase)) s_abort = 1;   // checked after the next barrier
-    rowphase ^= 1u;
+      // beside the panels, by the warps without rows (by all while the panels
+      // are short): G(:,S) and G(S,:), rounded to FP32, where the new block
+      // will be; two sites per item, as a pair's row entries share a sector
+      const int w0 = K >= 12 ? n_rw : 0;
+      if (q0 == 0 && warp >= w0) {
+        const int nt = SCAN_THREADS - 32 * w0, rows = hi - lo, ni = rows * ((dim + 1) / 2);
+        for (int e0 = tid - 32 * w0; e0 < ni; e0 += SCAN_GLOAD * nt) {
+          float4 gc[SCAN_GLOAD][2], gr[SCAN_GLOAD][2];
 #pragma unroll
-    for (int k = 0; k < RPT; ++k) {
-      const int r = tid + k * SCAN_THREADS;
-      if (r >= ns) continue;
+          for (int u = 0; u < SCAN_GLOAD; ++u) {
+            const int e = e0 + u * nt, h = e >= rows ? 1 : 0, r = lo + e - h * rows;
 #pragma unroll
-      for (int m = 0; m < dim; ++m) {
-        gm[k][m] = fa(gm[k][m], dg_f2(gcol[k][m]));
-        bl[k][m] = fa(bl[k][m], dg_f2(s_rows[(size_t)m * nrb * rb + r]));
+            for (int v = 0; v < 2; ++v)
+              if (e < ni && 2 * h + v < dim) {
+                const int sm = s_site[4 * p + 2 * h + v];
+                gc[u][v] = G[r + (size_t)ns * sm];
+                gr[u][v] = G[sm + (size_t)ns * r];
+              }
+          }
+#pragma unroll
+          for (int u = 0; u < SCAN_GLOAD; ++u) {
+            const int e = e0 + u * nt, h = e >= rows ? 1 : 0, r = lo + e - h * rows;
+#pragma unroll
+            for (int v = 0; v < 2; ++v)
+              if (e < ni && 2 * h + v < dim) {
+                pair_put(new_a + (size_t)(2 * h + v) * lp, r - lo, dg_f2(gc[u][v]));
+                pair_put(new_b + (size_t)(2 * h + v) * lp, r - lo, dg_f2(gr[u][v]));
+              }
+          }
+        }
       }
+      if (row) {
+        Pair ar[NP], bc[NP];
+#pragma unroll 4
+        for (int q = q0; q < min(qe, n_res); ++q) {
 #pragma unroll
-      for (int l = 0; l < dim; ++l) {
-        float2 a = make_float2(0.f, 0.f);
+          for (int k = 0; k < NP; ++k) {
+            ar[k] = pair_of(s_pa[(size_t)q * lp + NP * pt + k]);
+            bc[k] = pair_of(s_pb[(size_t)q * lp + NP * pt + k]);
+          }
+          scan_col<DS, NP>(ar, bc, s_gat + 8 * (q - q0) + m0, gm, bl);
+        }
+        // half a ring of columns at a time, so that their loads overlap
+        auto read_back = [&](int nb) {
+#pragma unroll 1
+          for (int q = max(q0, res); q < qe; q += nb) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");   // all but the batch behind this one
+            float4* rg = s_ring + (size_t)(2 * nb * slot) * lp + NP * pt;
+            constexpr int CB = RPT == 2 ? 4 : 2;   // columns in registers
 #pragma unroll
-        for (int m = 0; m < dim; ++m) a = fcfma(gm[k][m], s_T[m + dim * l], a);
-        float2 bv = make_float2(-bl[k][l].x, -bl[k][l].y);
-        if (r == S[l]) bv.x += 1.f;
-        A[(size_t)(K + l) * ldp + r] = a;
-        B[(size_t)(K + l) * ldp + r] = bv;
-        s_newA[(size_t)l * ns + r] = a;
-        s_newB[(size_t)l * ns + r] = bv;
+            for (int c0 = 0; c0 < SCAN_RING / 2; c0 += CB) {
+              if (c0 >= nb || q + c0 >= qe) break;
+              float4 u[CB][NP], v[CB][NP];
+#pragma unroll
+              for (int c = 0; c < CB; ++c)
+#pragma unroll
+                for (int k = 0; k < NP; ++k) {
+                  if (c0 + c >= nb) break;
+                  u[c][k] = rg[(size_t)(2 * (c0 + c)) * lp + k];
+                  v[c][k] = rg[(size_t)(2 * (c0 + c) + 1) * lp + k];
+                }
+#pragma unroll
+              for (int c = 0; c < CB; ++c) {
+                if (c0 + c >= nb || q + c0 + c >= qe) break;
+#pragma unroll
+                for (int k = 0; k < NP; ++k) {
+                  ar[k] = Pair{{u[c][k].x, u[c][k].z}, {u[c][k].y, u[c][k].w}};
+                  bc[k] = Pair{{v[c][k].x, v[c][k].z}, {v[c][k].y, v[c][k].w}};
+                }
+                scan_col<DS, NP>(ar, bc, s_gat + 8 * (q + c0 + c - q0) + m0, gm, bl);
+              }
+            }
+            fetch(q + 2 * nb, slot, nb);   // into the batch that this thread alone has read
+            slot ^= 1;
+          }
+        };
+        if (SH == 1) {
+          if (ring == SCAN_RING) read_back(SCAN_RING / 2);   // unrolled
+          else read_back(ring / 2);
+        }
       }
     }
-    __syncthreads();
-    if (s_abort) {
-      aborted = true;
-      break;
+    __syncthreads();   // s_T, G(:,S), G(S,:)
+    // ---- the new block: a = Geff(:,S) T, b = (I - Geff)(S,:) ----------------
+    if (row) {
+#pragma unroll
+      for (int k = 0; k < NP; ++k)
+#pragma unroll
+        for (int m = 0; m < DS; ++m) {
+          float4* pa_ = new_a + (size_t)(m0 + m) * lp + NP * pt + k;
+          const float4 ga = *pa_, gb = new_b[(size_t)(m0 + m) * lp + NP * pt + k];
+          gm[k][m] = Pair{{gm[k][m].x.a + ga.x, gm[k][m].x.b + ga.y}, {gm[k][m].y.a + ga.z, gm[k][m].y.b + ga.w}};
+          bl[k][m] = Pair{{bl[k][m].x.a + gb.x, bl[k][m].x.b + gb.y}, {bl[k][m].y.a + gb.z, bl[k][m].y.b + gb.w}};
+          if (SH > 1) *pa_ = pair_words(gm[k][m]);   // the other set needs Geff(r, S) of these sites
+        }
     }
+    if (SH > 1) __syncthreads();
+    float4 out_a[NP][DS];
+    if (row) {
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        float2 g0[dim], g1[dim];   // Geff(r, S) of the two rows
+#pragma unroll
+        for (int m = 0; m < dim; ++m) {
+          const Pair g = SH > 1 ? pair_of(new_a[(size_t)m * lp + NP * pt + k]) : gm[k][m % DS];
+          g0[m] = make_float2(g.x.a, g.y.a);
+          g1[m] = make_float2(g.x.b, g.y.b);
+        }
+#pragma unroll
+        for (int l = 0; l < DS; ++l) {
+          float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+#pragma unroll
+          for (int m = 0; m < dim; ++m) {
+            const float2 tm = s_T[m + dim * (m0 + l)];
+            a0 = fcfma(g0[m], tm, a0);
+            a1 = fcfma(g1[m], tm, a1);
+          }
+          out_a[k][l] = make_float4(a0.x, a1.x, a0.y, a1.y);
+        }
+      }
+    }
+    if (SH > 1) __syncthreads();   // Geff(r, S) is read
+    if (row) {
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        const int rk = r0 + 2 * k;
+#pragma unroll
+        for (int l = 0; l < DS; ++l) {
+          const int sl = s_site[4 * p + m0 + l];
+          const float4 wa4 = out_a[k][l];
+          float4 wb4 = make_float4(-bl[k][l].x.a, -bl[k][l].x.b, -bl[k][l].y.a, -bl[k][l].y.b);
+          if (rk == sl) wb4.x += 1.f;
+          if (rk + 1 == sl) wb4.y += 1.f;
+          // rows past Ns land in the columns' padding
+          if (to_global) {
+            *reinterpret_cast<float4*>(A + (size_t)(K + m0 + l) * ldp + rk) = make_float4(wa4.x, wa4.z, wa4.y, wa4.w);
+            *reinterpret_cast<float4*>(B + (size_t)(K + m0 + l) * ldp + rk) = make_float4(wb4.x, wb4.z, wb4.y, wb4.w);
+          }
+          new_a[(size_t)(m0 + l) * lp + NP * pt + k] = wa4;
+          new_b[(size_t)(m0 + l) * lp + NP * pt + k] = wb4;
+          if (nc > 1)   // to every CTA's copy of the block; two in turn, a CTA may still read the last one
+            for (int o = 0; o < nc; ++o) {
+              const uint32_t at_ = mapa(all_a + (size_t)(m0 + l) * lpa + (rk >> 1), o);
+              asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at_), "f"(wa4.x), "f"(wa4.y),
+                           "f"(wa4.z), "f"(wa4.w)
+                           : "memory");
+              asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at_ + 64 * (uint32_t)lpa),
+                           "f"(wb4.x), "f"(wb4.y), "f"(wb4.z), "f"(wb4.w)
+                           : "memory");
+            }
+        }
+      }
+    }
+    if (nc > 1) cluster_barrier();
+    else __syncthreads();
     // ---- the new block's contribution to the cached Geff of later plaquettes
     for (int e = tid; e < (npla - p - 1) * dd; e += blockDim.x) {
       const int pq = p + 1 + e / dd, k = e % dd;
       const int si = s_site[4 * pq + k % dim], sj = s_site[4 * pq + k / dim];
       float2 a = s_geff[16 * pq + k];
 #pragma unroll
-      for (int l = 0; l < dim; ++l) a = fcfma(s_newA[(size_t)l * ns + si], s_newB[(size_t)l * ns + sj], a);
+      for (int l = 0; l < dim; ++l) a = fcfma(pair_entry(all_a + (size_t)l * lpa, si), pair_entry(all_b + (size_t)l * lpa, sj), a);
       s_geff[16 * pq + k] = a;
     }
     K += dim;
     ++p;
     __syncthreads();
-    // the next accepted move of this round streams columns [0, K): start it now
-    if (p < npla && K + dim <= kd) {
-      npre = min((K + qc - 1) / qc, SCAN_NSTAGE);
-      if (tid == io) {
-        fence_proxy_async_global();
-        for (int c = 0; c < npre; ++c) scan_issue(s_stage, s_full, A, B, ldp, qc, K, c);
-      }
-    }
   }
-  // chunks started for an accepted move that did not come: drain them
-  if (!aborted && npre > 0) {
-    for (int c = 0; c < npre; ++c) {
-      if (!mbar_wait_bounded(&s_full[c], (phase >> c) & 1u)) s_abort = 1;
-      phase ^= 1u << c;
-    }
-    __syncthreads();
-    aborted = s_abort != 0;
-  }
-  if (aborted) {
-    // a panel chunk never arrived: give the copies still in flight a bounded
-    // wait, flag the chain and stop (the host reports PQMC_ERR_TIMEOUT)
-    if (tid == io) {
-      for (int st = 0; st < SCAN_NSTAGE; ++st) mbar_wait_bounded(&s_full[st], (phase >> st) & 1u);
-      mbar_wait_bounded(&s_rowbar, rowphase);
-      d.sc->status = PQMC_ERR_TIMEOUT;
-      atomicExch(d.err, PQMC_ERR_TIMEOUT);
-      *d.kcount = 0;
-      next_p[blockIdx.x] = npla;
-    }
-    return;
-  }
-  __syncthreads();
+  if (rank != 0) return;   // nothing of another CTA is touched after the last move's barrier
   // ---- bookkeeping of the round's accepted moves (field, expKV, ln_cw) -----
   for (int e = tid; e < n_acc * pd * pd; e += blockDim.x) {
     const int ja = e / (pd * pd), k = e % (pd * pd);
@@ -589,7 +759,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
     }
     if (lane == 0) {
       *d.kcount = K;
-      next_p[blockIdx.x] = p;
+      next_p[chain] = p;
       if (n_acc > 0) {
         const double l = (mant > 0.0) ? log(mant) + (double)ex * 0.69314718055994530942 : log(mant);
         d.sc->ln_cw = cadd(d.sc->ln_cw, mk(l));
@@ -1361,8 +1531,10 @@ struct pqmc_batch {
   std::vector<int*> kcounts;
   int parity = 0;
   int kd = 64;            // delay depth (panel columns per flush)
-  int qc = 8;             // panel columns per streamed chunk of the scan
-  int qc_max = 8;         // the largest chunk whose staging fits in shared memory
+  int scan_nc = 1;        // CTAs per chain of the scan
+  int scan_res = 0;       // panel columns of a round that stay in shared memory
+  int qc = 8;             // panel columns past those that the scan's threads have in flight as they read them back
+  int qc_max = 8;
   // 2: exact round update (exact.cuh; delay depth <= 64), 1: tcgen05 flush of
   // the scan's FP32 panels (delay depth <= 64), 0: mma.sync flush of them
   int flush_mode = 2;
@@ -1376,9 +1548,6 @@ struct pqmc_batch {
   // scan, bit 1: the split and flush); slice graphs then use node priorities
   int prio_mask = 3, prio_hi = 0;
   unsigned char* d_img = nullptr;   // split operand tile images of the tcgen05 flush
-  CUtensorMap* d_tmaps = nullptr;   // per chain: maps of its two G buffers
-  int rb = 0, nrb = 0;              // row box of the maps (columns) and boxes per row
-  std::vector<cplx*> tm_buf;        // per chain x 2: the buffer each map describes
   int* d_err = nullptr;   // device error word shared by all chains
   int* d_next = nullptr;  // per chain: next plaquette of the current family step
   cudaStream_t stream = nullptr;   // the stream of group 0, the batch's public stream
@@ -1474,11 +1643,6 @@ static int batch_refresh(pqmc_batch* b) {
   for (size_t i = 0; i < b->chains.size(); ++i) {
     b->h_desc[i].g = b->chains[i]->g;
     b->h_desc[i].g_alt = b->chains[i]->g_alt;
-    if (b->d_tmaps) {
-      const bool same = b->tm_buf[2 * i] == b->chains[i]->g;
-      b->h_desc[i].tm_g = b->d_tmaps + 2 * i + (same ? 0 : 1);
-      b->h_desc[i].tm_galt = b->d_tmaps + 2 * i + (same ? 1 : 0);
-    }
   }
   b->parity = 0;
   PQMC_CUDA(cudaMemcpyAsync(b->d_desc, b->h_desc.data(), sizeof(BDesc) * b->h_desc.size(), cudaMemcpyHostToDevice,
@@ -1510,6 +1674,23 @@ static int batch_sync_parity(pqmc_batch* b) {
 static cudaEvent_t gphase_begin(pqmc_batch* b, int g) { return g == 0 ? phase_begin(b) : nullptr; }
 static void gphase_end(pqmc_batch* b, int g, int phase, cudaEvent_t a) {
   if (g == 0) phase_end(b, phase, a);
+}
+
+// the dynamic shared-memory limit of the scan of one family dimension
+template <int DM>
+static cudaError_t scan_smem_dm(int ns, int sm) {
+  cudaError_t e = raise_dyn_smem(k_bscan<DM, 2, 1>, sm);
+  if (e == cudaSuccess && DM % 2 == 0) e = raise_dyn_smem(k_bscan<DM, 2, (DM % 2 ? 1 : 2)>, sm);
+  if (e == cudaSuccess && scan_rpt(ns) == 4) e = raise_dyn_smem(k_bscan<DM, 4, 1>, sm);
+  return e;
+}
+static cudaError_t scan_smem(int dim, int ns, int sm) {
+  switch (dim) {
+    case 1: return scan_smem_dm<1>(ns, sm);
+    case 2: return scan_smem_dm<2>(ns, sm);
+    case 3: return scan_smem_dm<3>(ns, sm);
+    default: return scan_smem_dm<4>(ns, sm);
+  }
 }
 
 // the dynamic shared-memory limit of every k_bwrap_cols variant of one
@@ -1638,18 +1819,26 @@ static int bupdate(pqmc_batch* b, int g, int pf, int parity) {
   unsigned char* img = b->d_img ? b->d_img + um_chain_bytes(ns) * c_first : nullptr;
   for (int r = 0; r < rounds; ++r) {
     const BDesc& h0 = b->h_desc[0];
-    const size_t smem = scan_layout(npla, ns, h0.ldp, b->qc, kd, 4 * h0.nrb * h0.rb * (int)sizeof(float4)).total;
+    const int nc = kd <= UM_KP ? b->scan_nc : 1, res = nc > 1 ? UM_KP : std::min(b->scan_res, kd);
+    const int ring = std::max(2, b->qc & ~1);
+    const size_t smem = scan_layout(npla, h0.ldp, res, kd, nc, ring).total;
+    const int nr = nc > 1 ? scan_rows(h0.ldp, nc) : ns;
+    const bool two = dim % 2 == 0 && res - res % dim >= kd - kd % dim && nr <= SCAN_SH_ROWS;
     cudaEvent_t ts = gphase_begin(b, g);
-    const bool one = ns <= SCAN_THREADS;
-#define PQMC_SCAN(DM, R)                                                                                         \
-  PQMC_CUDA(launch_at(k_bscan<DM, R>, dim3(C), dim3(SCAN_THREADS), smem, st, (b->prio_mask & 1) != 0, b->prio_hi, Dg, \
-                      pf, parity, kd, b->qc, next, exact ? 1 : 0, b->timing ? 1 : 0))
+#define PQMC_SCANR(DM, R, H)                                                                                        \
+  PQMC_CUDA(launch_cluster_at(k_bscan<DM, R, H>, nc, dim3(C * nc), dim3(SCAN_THREADS), smem, st, (b->prio_mask & 1) != 0, b->prio_hi, Dg, \
+                      pf, parity, kd, res, nc, ring, next, exact ? 1 : 0, b->timing ? 1 : 0))
+#define PQMC_SCAN(DM)                                                                                           \
+  if (two) { PQMC_SCANR(DM, 2, (DM % 2 ? 1 : 2)); }                                                             \
+  else if (scan_rpt(nr) == 2) { PQMC_SCANR(DM, 2, 1); }                                                          \
+  else { PQMC_SCANR(DM, 4, 1); }
     switch (dim) {
-      case 1: if (one) PQMC_SCAN(1, 1); else PQMC_SCAN(1, 2); break;
-      case 2: if (one) PQMC_SCAN(2, 1); else PQMC_SCAN(2, 2); break;
-      case 3: if (one) PQMC_SCAN(3, 1); else PQMC_SCAN(3, 2); break;
-      default: if (one) PQMC_SCAN(4, 1); else PQMC_SCAN(4, 2); break;
+      case 1: PQMC_SCAN(1); break;
+      case 2: PQMC_SCAN(2); break;
+      case 3: PQMC_SCAN(3); break;
+      default: PQMC_SCAN(4); break;
     }
+#undef PQMC_SCANR
 #undef PQMC_SCAN
     PQMC_LAUNCHED();
     gphase_end(b, g, PQMC_PHASE_SCAN, ts);
@@ -1884,7 +2073,8 @@ static bool same_geometry(const pqmc_model* a, const pqmc_model* b) {
 }
 
 extern "C" int pqmc_batch_destroy(pqmc_batch* b);
-extern "C" int pqmc_batch_create(const pqmc_model* const* models, int n_chains, int precision, pqmc_batch** out);
+static int create_batch(const pqmc_model* const* models, int n_chains, int all_chains, int precision,
+                        pqmc_batch** out);
 
 // an uneven mixed batch: one homogeneous batch per geometry class, each with
 // its own streams, chain groups, delay depth and graphs
@@ -1903,7 +2093,7 @@ static int create_uneven(const pqmc_model* const* models, int n_chains, const st
         sub.push_back(models[i]);
       }
     pqmc_batch* part = nullptr;
-    const int st = pqmc_batch_create(sub.data(), (int)sub.size(), PQMC_PREC_MIXED, &part);
+    const int st = create_batch(sub.data(), (int)sub.size(), n_chains, PQMC_PREC_MIXED, &part);
     if (st != PQMC_OK) {
       pqmc_batch_destroy(b);
       return st;
@@ -1923,9 +2113,9 @@ static int create_uneven(const pqmc_model* const* models, int n_chains, const st
   return PQMC_OK;
 }
 
-extern "C" {
-
-int pqmc_batch_create(const pqmc_model* const* models, int n_chains, int precision, pqmc_batch** out) {
+// all_chains: chains that run beside each other, those of an uneven batch's other classes too
+static int create_batch(const pqmc_model* const* models, int n_chains, int all_chains, int precision,
+                        pqmc_batch** out) {
   if (!models || !out || n_chains < 1) { set_error("batch_create: bad arguments"); return PQMC_ERR_ARG; }
   if (precision != PQMC_PREC_FP64 && precision != PQMC_PREC_MIXED) {
     set_error("batch_create: unknown precision %d", precision);
@@ -1996,10 +2186,10 @@ int pqmc_batch_create(const pqmc_model* const* models, int n_chains, int precisi
     pqmc_batch_destroy(b);
     return PQMC_ERR_ARG;
   }
-  const int ldp = (c0->ns + 1) & ~1;
+  const int ldp = (c0->ns + 3) & ~3;
   if (precision == PQMC_PREC_MIXED) {
-    if (c0->ns > SCAN_RPT * SCAN_THREADS) {
-      set_error("batch_create: mixed precision supports Ns <= %d", SCAN_RPT * SCAN_THREADS);
+    if (c0->ns > SCAN_MAX_NS) {
+      set_error("batch_create: mixed precision supports Ns <= %d", SCAN_MAX_NS);
       pqmc_batch_destroy(b);
       return PQMC_ERR_ARG;
     }
@@ -2007,59 +2197,47 @@ int pqmc_batch_create(const pqmc_model* const* models, int n_chains, int precisi
     for (int f = 0; f < c0->n_pf; ++f) max_pla = std::max(max_pla, c0->h_pf_npla[f]);
     PQMC_CUDA(cudaGetDevice(&dev));
     PQMC_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const size_t stat = 4096;   // static shared memory of k_bscan (descriptor, per-warp R and T, barriers)
-    // rows of G by TMA boxes of rb columns (rb a multiple of 8: 128-byte aligned boxes)
-    const int nrb = (c0->ns + 255) / 256;
-    const int rb = (((c0->ns + nrb - 1) / nrb) + 7) & ~7;
-    const int rows_bytes = 4 * nrb * rb * (int)sizeof(float4);
-    int qc = 8;
-    while (qc > 1 && scan_layout(max_pla, c0->ns, ldp, qc, SCAN_KSTAGE, rows_bytes).total + stat > (size_t)optin) --qc;
-    const size_t need = scan_layout(max_pla, c0->ns, ldp, qc, SCAN_KSTAGE, rows_bytes).total;
-    if (need + stat > (size_t)optin) {
-      set_error("batch_create: scan staging needs %zu bytes of shared memory, the device offers %d", need + stat,
-                optin);
+    const size_t stat = 4096;   // static shared memory of k_bscan (descriptor, per-warp R and T)
+    int res = UM_KP;            // panel columns that stay in shared memory: as many as fit, whole blocks of 4
+    int ring = SCAN_RING;       // ... and the ring as deep as fits where none does
+    const auto need_of = [&](int r, int q) { return scan_layout(max_pla, ldp, r, SCAN_KSTAGE, 1, q).total; };
+    while (res > 0 && need_of(res, ring) + stat > (size_t)optin) res -= 4;
+    while (ring > 2 && need_of(res, ring) + stat > (size_t)optin) ring -= 2;
+    const size_t need = need_of(res, ring);
+    // The sizes taken do not depend on what the scan stages: those for which
+    // eight rows of G, a short stream of panel columns and the family's tables
+    // fit (need never exceeds this where it does).
+    const size_t ns_ = c0->ns, boxes = (ns_ + 255) / 256, rows = boxes * (((ns_ + boxes - 1) / boxes + 7) & ~(size_t)7);
+    const size_t bound = 64 * rows + 48 * ((ns_ + 1) & ~(size_t)1) + 64 * ns_ + 2 * al16(140 * (size_t)max_pla) + 12 * SCAN_KSTAGE;
+    if (std::max(need, bound) + stat > (size_t)optin) {
+      set_error("batch_create: scan staging needs %zu bytes of shared memory, the device offers %d",
+                std::max(need, bound) + stat, optin);
       pqmc_batch_destroy(b);
       return PQMC_ERR_ARG;
     }
-    b->qc = qc;
-    b->qc_max = qc;
-    // tensor maps over every chain's two G buffers (double-float: 4 FP32 per element)
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn) {
-      set_error("batch_create: cuTensorMapEncodeTiled unavailable");
-      pqmc_batch_destroy(b);
-      return PQMC_ERR_CUDA;
-    }
-    auto encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    std::vector<CUtensorMap> maps(2 * (size_t)n_chains);
-    b->tm_buf.resize(2 * (size_t)n_chains);
-    for (int i = 0; i < n_chains; ++i)
-      for (int k = 0; k < 2; ++k) {
-        cplx* buf = k == 0 ? b->chains[i]->g : b->chains[i]->g_alt;
-        b->tm_buf[2 * i + k] = buf;
-        const cuuint64_t dims[2] = {4ull * (cuuint64_t)c0->ns, (cuuint64_t)c0->ns};
-        const cuuint64_t strides[1] = {16ull * (cuuint64_t)c0->ns};
-        const cuuint32_t box[2] = {4u, (cuuint32_t)rb};
-        const cuuint32_t estr[2] = {1u, 1u};
-        const CUresult r = encode(&maps[2 * i + k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)buf, dims, strides, box,
-                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                  CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) {
-          set_error("batch_create: cuTensorMapEncodeTiled failed (%d)", (int)r);
-          pqmc_batch_destroy(b);
-          return PQMC_ERR_CUDA;
-        }
+    b->scan_res = res;
+    // One CTA per chain, or a cluster with about 100 of the rows in each: a
+    // column then costs its latency and no longer its bytes and multiply-adds,
+    // and the panels fit in the CTAs' shared memory, for an exchange of the new
+    // block and a wider gather per acceptance. Below 161 rows that costs more
+    // than it saves (8 chains of 128 rows: 11.5 ms in one CTA, 11.7 in two;
+    // of 200: 19.9 and 18.4; of 288: 34.3 in one and 28.8 in three for 16
+    // chains; of 392: 55.6 and 46.5 in four), and once every chain's cluster
+    // no longer has its SMs to itself the extra CTAs only take time from the
+    // flushes (64 chains of 392 rows: 108.5 ms in one CTA, 118.6 in four).
+    b->scan_nc = 1;
+    size_t most = need;
+    int sms = 0;
+    PQMC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (const int nc = std::min((ldp + 99) / 100, 4); c0->ns > 160 && nc * all_chains <= sms) {
+      const size_t nd = scan_layout(max_pla, ldp, UM_KP, UM_KP, nc, ring).total;
+      if (nd + stat <= (size_t)optin && scan_rows(ldp, nc) * (nc - 1) < c0->ns && scan_rpt(scan_rows(ldp, nc)) == 2) {
+        b->scan_nc = nc;
+        most = std::max(most, nd);
       }
-    PQMC_CUDA(cudaMalloc((void**)&b->d_tmaps, sizeof(CUtensorMap) * maps.size()));
-    PQMC_CUDA(cudaMemcpy(b->d_tmaps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice));
-    b->rb = rb;
-    b->nrb = nrb;
-#define PQMC_SMEM(DM, R) PQMC_CUDA(raise_dyn_smem(k_bscan<DM, R>, (int)need))
-    PQMC_SMEM(1, 1); PQMC_SMEM(2, 1); PQMC_SMEM(3, 1); PQMC_SMEM(4, 1);
-    PQMC_SMEM(1, 2); PQMC_SMEM(2, 2); PQMC_SMEM(3, 2); PQMC_SMEM(4, 2);
-#undef PQMC_SMEM
+    }
+    b->qc = b->qc_max = ring;
+    for (int f = 0; f < c0->n_pf; ++f) PQMC_CUDA(scan_smem(c0->h_pf_dim[f], c0->ns, (int)most));
   }
   PQMC_CUDA(cudaMalloc((void**)&b->d_err, sizeof(int)));
   PQMC_CUDA(cudaMemset(b->d_err, 0, sizeof(int)));
@@ -2112,8 +2290,6 @@ int pqmc_batch_create(const pqmc_model* const* models, int n_chains, int precisi
     h.g_alt = c->g_alt;
     h.kmax = kmax;
     h.ldp = ldp;
-    h.rb = b->rb;
-    h.nrb = b->nrb;
     h.err = b->d_err;
     h.pre = c->pre;
     if (precision == PQMC_PREC_MIXED) {
@@ -2218,6 +2394,12 @@ int pqmc_batch_create(const pqmc_model* const* models, int n_chains, int precisi
   return PQMC_OK;
 }
 
+extern "C" {
+
+int pqmc_batch_create(const pqmc_model* const* models, int n_chains, int precision, pqmc_batch** out) {
+  return create_batch(models, n_chains, n_chains, precision, out);
+}
+
 int pqmc_batch_destroy(pqmc_batch* b) {
   if (!b) return PQMC_OK;
   if (!b->parts.empty() || !b->part_of.empty()) {
@@ -2250,7 +2432,6 @@ int pqmc_batch_destroy(pqmc_batch* b) {
   if (b->d_wtab) cudaFree(b->d_wtab);
   if (b->d_ximg) cudaFree(b->d_ximg);
   if (b->d_acc) cudaFree(b->d_acc);
-  if (b->d_tmaps) cudaFree(b->d_tmaps);
   for (int g = 1; g < pqmc_batch::MAX_GROUPS; ++g)
     if (b->g_stream[g]) {
       cudaStreamSynchronize(b->g_stream[g]);

@@ -42,14 +42,6 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-// 2-D tiled TMA load of the box at (x, y) of the tensor map into shared memory
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* b) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_addr(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_addr(b))
-      : "memory");
-}
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
 __device__ __forceinline__ void bulk_s2g(void* gdst, const void* ssrc, uint32_t bytes) {
@@ -157,6 +149,30 @@ static cudaError_t launch_at(void (*k)(P...), dim3 grid, dim3 block, size_t smem
     at[0].val.priority = prio;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
+// the same in clusters of nc CTAs
+template <typename... P, typename... A>
+static cudaError_t launch_cluster_at(void (*k)(P...), int nc, dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool use, int prio,
+                             A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  cfg.attrs = at;
+  if (use) {
+    at[cfg.numAttrs].id = cudaLaunchAttributePriority;
+    at[cfg.numAttrs++].val.priority = prio;
+  }
+  if (nc > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = nc;
+    at[cfg.numAttrs].val.clusterDim.y = 1;
+    at[cfg.numAttrs++].val.clusterDim.z = 1;
   }
   return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }

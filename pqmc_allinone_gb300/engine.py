@@ -420,11 +420,11 @@ class PqmcBatch:
         return int(v.value)
 
     def set_scan_chunk(self, qc: int):
-        """Panel columns per streamed chunk of the scan (1 .. the largest that fits)."""
+        """Panel columns a thread of the scan has in flight as it reads them back (1 .. the most that fit)."""
         check(self.lib, self.lib.pqmc_batch_set_scan_chunk(self.h, qc), "pqmc_batch_set_scan_chunk")
 
     def scan_chunk(self, with_max: bool = False):
-        """The scan's panel chunk (and, with_max, the largest that fits)."""
+        """Panel columns in flight per thread of the scan (and, with_max, the most that fit)."""
         v, mx = ctypes.c_int(0), ctypes.c_int(0)
         check(self.lib, self.lib.pqmc_batch_get_scan_chunk(self.h, ctypes.byref(v), ctypes.byref(mx)),
               "pqmc_batch_get_scan_chunk")

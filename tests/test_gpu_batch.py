@@ -7,12 +7,14 @@ products, double-float wraps, double-float recompute): G within 1e-8 of the
 oracle throughout.  Flush modes 1 and 0 (the scan's FP32 panels folded in
 by tcgen05 or mma.sync split-BF16 products, FP32 wrap corrections) keep
 their looser bounds."""
+from dataclasses import replace
+
 import numpy as np
 import pytest
 
 from pqmc_allinone_gb300 import model as M
 from pqmc_allinone_gb300.rng import seed_words
-from tests.helpers import epsocz_small, rel_fro
+from tests.helpers import epsocz_small, general_bond_model, rel_fro
 
 pytestmark = pytest.mark.gpu
 
@@ -341,6 +343,48 @@ def test_scan_chunks_bit_identical():
     b = PqmcBatch([m for m, _, _ in ms], [f for _, f, _ in ms], [w for _, _, w in ms], precision=1)
     with pytest.raises(RuntimeError, match="shared memory"):
         b.set_scan_chunk(10 ** 6)
+    b.close()
+
+
+@pytest.mark.parametrize("make,L,many", [(epsocz_small, 10, 77), (epsocz_small, 12, 51), (epsocz_small, 14, 39),
+                                         (general_bond_model, 14, 77)])
+def test_scan_clusters_bit_identical(make, L, many):
+    """A chain's rows spread over a cluster of 2, 3 or 4 CTAs (200 / 196, 288
+    and 392 rows; few chains) or held by one (more chains than the SMs have
+    clusters): the sums run in the same order, so the chain is bit-identical."""
+    from pqmc_allinone_gb300.engine import PqmcBatch
+    m, f = make(L=L, ntime=4, ngroup=2, seed=31)
+    runs = []
+    for n in (1, many):
+        b = PqmcBatch([m] * n, [f] * n, [seed_words(900 + i) for i in range(n)], precision=1)
+        b.init()
+        for loop in (1, 2):
+            b.sweep(loop)
+        runs.append((b.chains[0].field(), b.chains[0].g(), b.chains[0].state()))
+        b.close()
+    (f0, g0, s0), (f1, g1, s1) = runs
+    assert s0["positive_accept"] + s0["negative_accept"] > 0
+    assert np.array_equal(f0, f1) and np.array_equal(g0, g1) and s0["ln_cw"] == s1["ln_cw"]
+
+
+def test_mixed_batch_1024_rows():
+    """Four rows per thread, no resident panel column, and a ring shorter than
+    its eight columns: the G that the moves leave drifts from the recompute no
+    further than at smaller sizes."""
+    from pqmc_allinone_gb300.engine import PqmcBatch
+    spec = general_bond_model(L=4)[0].spec   # an eighth of the bonds: families of 128 plaquettes
+    pfs = [replace(pf, tsl=[8, 0, 4, 1], offset=[o, 0], n_cover=0.25, bf_index=1 + i)
+           for i, (pf, o) in enumerate((pf, o) for pf in spec.pfs[:3:2] for o in range(8))]
+    m = M.build_model(replace(spec, lat_size=[32, 32], pfs=pfs, bf_sets=16, beta=0.4, ngroup=2), twist_seed=3,
+                      twist=1e-3)
+    f = M.field_gaussian(m, 33)
+    b = PqmcBatch([m], [f], [seed_words(950)], precision=1)
+    assert b.scan_chunk(with_max=True)[1] < 8
+    b.init()
+    b.sweep(1)
+    s = b.chains[0].state()
+    assert s["positive_accept"] > 0 and s["negative_accept"] > 0
+    assert 0.0 < s["err_g_rel_max"] < MIXED_DRIFT_TOL[2], s
     b.close()
 
 
