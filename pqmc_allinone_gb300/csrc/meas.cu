@@ -2,10 +2,11 @@
 // src/mod_meas.f90:210-544; helpers :64-208; k-space :546-566; window
 // averaging :729-763) and the fused sweep driver (src/Main_PQMC.f90:81-156).
 //
-// One CTA per relative displacement `ind`; its threads cover the cells c1,
-// each evaluating every Wick contraction of the pair (c1, c2) with
-// rel(c1,c2) = ind, then a fixed-order tree reduction per observable.  The
-// per-cell phonon scalars are a separate single-thread pass in cell order.
+// One CTA per part of the observables and relative displacement `ind`; its
+// threads cover the cells c1, each evaluating its part of the Wick
+// contractions of the pair (c1, c2) with rel(c1,c2) = ind, then a fixed-order
+// sum per observable.  The per-cell phonon scalars are one more CTA.
+#include <algorithm>
 #include <string.h>
 #include <vector>
 #include "chain.cuh"
@@ -28,211 +29,317 @@ struct MeasView {
   double hop, ep;
 };
 
-__device__ __forceinline__ cplx GH(const MeasView& V, int i, int j) { return V.gh[i + (size_t)V.ns * j]; }
+__device__ __forceinline__ cplx GH(const MeasView& V, int i, int j) {
+  const double2 v = __ldg(reinterpret_cast<const double2*>(V.gh) + i + (size_t)V.ns * j);
+  return mk(v.x, v.y);
+}
 __device__ __forceinline__ cplx GG(const MeasView& V, int i, int j) {
-  cplx v = cneg(V.gh[i + (size_t)V.ns * j]);
+  cplx v = cneg(GH(V, i, j));
   if (i == j) v = cadd(v, mk(1.0));
   return v;
 }
 
-// cal_wick_contraction (:165-183): mat(i,j) = gh(l2,l1) gh(r2,r1) [+ gh(r2,l1) g(l2,r1)]
-template <int N>
-__device__ inline void wick(const MeasView& V, const int (*ls)[2], const int (*rs)[2], bool hartree, cplx* mat) {
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < N; ++j) {
-      cplx m = mk(0.0);
-      m = cfma(GH(V, ls[i][1], ls[i][0]), GH(V, rs[j][1], rs[j][0]), m);
-      if (!hartree) m = cfma(GH(V, rs[j][1], ls[i][0]), GG(V, ls[i][1], rs[j][0]), m);
-      mat[i + N * j] = m;
-    }
+// ---------------------------------------------------------------------------
+// The Wick contractions of a pair of cells (cal_wick_contraction, :165-183):
+//   mat(i,j) = gh(l2,l1) gh(r2,r1) + gh(r2,l1) g(l2,r1)
+// between site pairs (l1,l2) of a bond at c1 and (r1,r2) of one at c2, and
+// sums vl(i) mat(i,j) vr(j) over them.  FP64 issue bounds the kernel, so the
+// sums are factored.  The first term is a product of one sum over i and one
+// over j (the Hartree observables are that product alone).  A bond's four
+// spin-flipping pairs carry the coefficients (b, sb, -b', -sb') (s = +1 or
+// -1, b the boundary phase, b' its conjugate, :199-208), so the second term
+// is four block sums of the 16 products, with signs only; and with the four
+// spin-conserving pairs of the physical current it is the trace of P VL Q VR,
+// P = gh between the bonds' sites, Q = g, VL and VR with two entries per row.
+// That is ~1.3k FP64 operations per pair instead of the ~4.2k of the plain
+// contractions.  The division by N_cell is done on the sums.
+// ---------------------------------------------------------------------------
+struct Bond {     // a cell's two sites and its neighbour's, the phase of the bond
+  int s[4];
+  cplx b;
+};
+__device__ __forceinline__ Bond bond(const MeasView& V, int c, int dir) {
+  const int n = dir ? V.ynb[c] : V.xnb[c];
+  Bond B;
+  B.s[0] = V.sites[2 * c];
+  B.s[1] = V.sites[2 * c + 1];
+  B.s[2] = V.sites[2 * n];
+  B.s[3] = V.sites[2 * n + 1];
+  B.b = V.cross[2 * c + dir] ? V.bc[dir] : mk(1.0);
+  return B;
+}
+__device__ __forceinline__ double boson(const MeasView& V, int c, int dir) {
+  return V.field[V.bfi[2 * c + dir] + (size_t)V.n_bf * V.t];
 }
 
-__device__ inline void spin_current(const MeasView& V, int p1, int p2, int p3, int p4, bool h, cplx* mat) {
-  auto s = [&](int c, int k) { return V.sites[k + 2 * c]; };
-  int ls[4][2] = {{s(p1, 0), s(p2, 1)}, {s(p1, 1), s(p2, 0)}, {s(p2, 0), s(p1, 1)}, {s(p2, 1), s(p1, 0)}};
-  int rs[4][2] = {{s(p3, 0), s(p4, 1)}, {s(p3, 1), s(p4, 0)}, {s(p4, 0), s(p3, 1)}, {s(p4, 1), s(p3, 0)}};
-  wick<4>(V, ls, rs, h, mat);
+// b1 (b2 t00 + b2' t01) + b1' (b2 t10 + b2' t11)
+__device__ __forceinline__ cplx phases(cplx b1, cplx b2, const cplx (&t)[2][2]) {
+  const cplx u = cfma(b2, t[0][0], cmul(cconj(b2), t[0][1]));
+  const cplx w = cfma(b2, t[1][0], cmul(cconj(b2), t[1][1]));
+  return cfma(b1, u, cmul(cconj(b1), w));
+}
+__device__ __forceinline__ cplx times_i(cplx z, double f) { return mk(-f * z.y, f * z.x); }
+
+// sum of v(i) gh(l2,l1) over a bond's spin-flipping pairs; vx: i hop (b, b,
+// -b', -b'), vy: hop (b, -b, -b', b')
+__device__ __forceinline__ void spin_sums(const MeasView& V, const Bond& B, cplx* vx, cplx* vy) {
+  const cplx a0 = GH(V, B.s[3], B.s[0]), a1 = GH(V, B.s[2], B.s[1]);
+  const cplx a2 = GH(V, B.s[1], B.s[2]), a3 = GH(V, B.s[0], B.s[3]);
+  *vx = times_i(csub(cmul(B.b, cadd(a0, a1)), cmul(cconj(B.b), cadd(a2, a3))), V.hop);
+  const cplx y = csub(cmul(B.b, csub(a0, a1)), cmul(cconj(B.b), csub(a2, a3)));
+  *vy = mk(V.hop * y.x, V.hop * y.y);
 }
 
-__device__ inline void spin_momentum(const MeasView& V, int p1, int p2, cplx* mat) {
-  auto s = [&](int c, int k) { return V.sites[k + 2 * c]; };
-  int ls[4][2] = {{s(p1, 0), s(p1, 0)}, {s(p1, 0), s(p1, 1)}, {s(p1, 1), s(p1, 0)}, {s(p1, 1), s(p1, 1)}};
-  int rs[4][2] = {{s(p2, 0), s(p2, 0)}, {s(p2, 0), s(p2, 1)}, {s(p2, 1), s(p2, 0)}, {s(p2, 1), s(p2, 1)}};
-  wick<4>(V, ls, rs, false, mat);
-}
-
-__device__ inline void phys_current(const MeasView& V, int p1, int p2, int p3, int p4, cplx* mat) {
-  auto s = [&](int c, int k) { return V.sites[k + 2 * c]; };
-  int ls[8][2] = {{s(p1, 0), s(p2, 1)}, {s(p1, 1), s(p2, 0)}, {s(p2, 0), s(p1, 1)}, {s(p2, 1), s(p1, 0)},
-                  {s(p1, 0), s(p2, 0)}, {s(p1, 1), s(p2, 1)}, {s(p2, 0), s(p1, 0)}, {s(p2, 1), s(p1, 1)}};
-  int rs[8][2] = {{s(p3, 0), s(p4, 1)}, {s(p3, 1), s(p4, 0)}, {s(p4, 0), s(p3, 1)}, {s(p4, 1), s(p3, 0)},
-                  {s(p3, 0), s(p4, 0)}, {s(p3, 1), s(p4, 1)}, {s(p4, 0), s(p3, 0)}, {s(p4, 1), s(p3, 1)}};
-  wick<8>(V, ls, rs, false, mat);
-}
-
-__device__ __forceinline__ void bphase(const MeasView& V, cplx* v, bool cross, int dir) {
-  // add_boundary_phase (:199-208)
-  if (!cross) return;
-  cplx bc = V.bc[dir];
-  v[0] = cmul(v[0], bc); v[1] = cmul(v[1], bc); v[2] = cmul(v[2], cconj(bc)); v[3] = cmul(v[3], cconj(bc));
-}
-
-template <int N>
-__device__ __forceinline__ cplx contract(const cplx* vl, const cplx* m, const cplx* vr) {
-  cplx tot = mk(0.0);
-  for (int i = 0; i < N; ++i) {
-    cplx w = mk(0.0);
-    for (int j = 0; j < N; ++j) w = cfma(m[i + N * j], vr[j], w);
-    tot = cfma(vl[i], w, tot);
-  }
-  return tot;
-}
-
-// all field observables of one cell pair, already divided by N_cell
-__device__ void pair_obs(const MeasView& V, int c1, int c2, cplx* F) {
-  const double N = (double)V.nc;
-  const int t = V.t;
-  auto X = [&](int b) { return V.field[b + (size_t)V.n_bf * t]; };
-  const int c1x = V.xnb[c1], c1y = V.ynb[c1], c2x = V.xnb[c2], c2y = V.ynb[c2];
-  const bool cr1[2] = {V.cross[2 * c1] != 0, V.cross[2 * c1 + 1] != 0};
-  const bool cr2[2] = {V.cross[2 * c2] != 0, V.cross[2 * c2 + 1] != 0};
-  const double x1x = X(V.bfi[2 * c1]), x1y = X(V.bfi[2 * c1 + 1]);
-  const double x2x = X(V.bfi[2 * c2]), x2y = X(V.bfi[2 * c2 + 1]);
-  F[PQMC_F_BFX_BFX] = mk((x1x * x2x) / N);
-  F[PQMC_F_BFX_BFY] = mk((x1x * x2y) / N);
-  F[PQMC_F_BFY_BFY] = mk((x1y * x2y) / N);
-  F[PQMC_F_BFXY_BFXY] = mk((x1x * x1y * x2x * x2y) / N);
-  const cplx vx[4] = {mk(-0.0, V.hop), mk(-0.0, V.hop), mk(0.0, -V.hop), mk(0.0, -V.hop)};
-  const cplx vy[4] = {mk(V.hop), mk(-V.hop), mk(-V.hop), mk(V.hop)};
-  cplx m[64], vl[8], vr[8];
-  auto cur = [&](int f, const cplx* lv, int ld, const cplx* rv, int rd, bool quirk) {
-    for (int k = 0; k < 4; ++k) { vl[k] = lv[k]; vr[k] = rv[k]; }
-    bphase(V, vl, cr1[ld], ld);
-    bphase(V, vr, cr2[rd], rd);
-    cplx r = contract<4>(vl, m, quirk ? vl : vr);
-    F[f] = mk(r.x / N, r.y / N);
-  };
-  spin_current(V, c1, c1x, c2, c2x, false, m);
-  cur(PQMC_F_JXX_JXX, vx, 0, vx, 0, false);
-  cur(PQMC_F_JXY_JXY, vy, 0, vy, 0, false);
-  spin_current(V, c1, c1y, c2, c2y, false, m);
-  cur(PQMC_F_JYX_JYX, vx, 1, vx, 1, false);
-  cur(PQMC_F_JYY_JYY, vy, 1, vy, 1, true);     // :353 contracts with vec_l twice
-  spin_current(V, c1, c1x, c2, c2y, false, m);
-  cur(PQMC_F_JXX_JYX, vx, 0, vx, 1, false);
-  cur(PQMC_F_JXY_JYY, vy, 0, vy, 1, false);
-  spin_current(V, c1, c1x, c2, c2x, true, m);
-  cur(PQMC_F_JXXH_JXXH, vx, 0, vx, 0, false);
-  cur(PQMC_F_JXYH_JXYH, vy, 0, vy, 0, false);
-  spin_current(V, c1, c1y, c2, c2y, true, m);
-  cur(PQMC_F_JYXH_JYXH, vx, 1, vx, 1, false);
-  cur(PQMC_F_JYYH_JYYH, vy, 1, vy, 1, true);   // :417
-  spin_current(V, c1, c1x, c2, c2y, true, m);
-  cur(PQMC_F_JXXH_JYXH, vx, 0, vx, 1, false);
-  cur(PQMC_F_JXYH_JYYH, vy, 0, vy, 1, false);
-  cur(PQMC_F_JXXH_JYYH, vx, 0, vy, 1, false);
-  cur(PQMC_F_JXYH_JYXH, vy, 0, vx, 1, false);
-  spin_momentum(V, c1, c2, m);
-  {
-    const cplx dn[4] = {mk(0.5), mk(0), mk(0), mk(0.5)};
-    const cplx sz[4] = {mk(0.5), mk(0), mk(0), mk(-0.5)};
-    const cplx sx[4] = {mk(0), mk(0.5), mk(0.5), mk(0)};
-    const cplx sy[4] = {mk(0), mk(-0.0, -0.5), mk(0.0, 0.5), mk(0)};
-    cplx r = contract<4>(dn, m, dn);
-    F[PQMC_F_DEN_DEN] = mk(r.x / N, r.y / N);
-    int s1u = V.sites[2 * c1], s1d = V.sites[2 * c1 + 1], s2u = V.sites[2 * c2], s2d = V.sites[2 * c2 + 1];
-    cplx sc = csub(cmul(GH(V, s2u, s1u), GH(V, s2d, s1d)), cmul(GH(V, s2d, s1u), GH(V, s2u, s1d)));
-    F[PQMC_F_SC_SC] = mk(sc.x / N, sc.y / N);
-    r = contract<4>(sz, m, sz);
-    F[PQMC_F_SZ_SZ] = mk(r.x / N, r.y / N);
-    r = contract<4>(sx, m, sx);
-    F[PQMC_F_SX_SX] = mk(r.x / N, r.y / N);
-    r = contract<4>(sy, m, sy);
-    F[PQMC_F_SY_SY] = mk(r.x / N, r.y / N);
-  }
-  auto phys = [&](int f, const cplx* cv, double xl, double xr, int dir) {
-    for (int k = 0; k < 4; ++k) vl[k] = cneg(cv[k]);
-    for (int k = 0; k < 4; ++k) vl[4 + k] = mk(V.ep * xl * 1.0);
-    for (int k = 0; k < 4; ++k) vr[k] = vl[k];
-    for (int k = 0; k < 4; ++k) vr[4 + k] = mk(V.ep * xr * 1.0);
-    bphase(V, vl, cr1[dir], dir);
-    bphase(V, vr, cr2[dir], dir);
-    bphase(V, vl + 4, cr1[dir], dir);
-    bphase(V, vr + 4, cr2[dir], dir);
-    cplx r = contract<8>(vl, m, vr);
-    F[f] = mk(r.x / N, r.y / N);
-  };
-  phys_current(V, c1, c1y, c2, c2y, m);
-  phys(PQMC_F_CJYX_CJYX, vx, x1y, x2y, 1);
-  phys_current(V, c1, c1x, c2, c2x, m);
-  phys(PQMC_F_CJXY_CJXY, vy, x1x, x2x, 0);
-}
-
-constexpr int MEAS_THREADS = 128;
-
-__global__ void __launch_bounds__(MEAS_THREADS) k_meas_pairs(MeasView V, cplx* acc) {
-  __shared__ double red[MEAS_THREADS];
-  const int ind = blockIdx.x;
-  cplx part[PQMC_N_FIELD];
-  for (int f = 0; f < PQMC_N_FIELD; ++f) part[f] = mk(0.0);
-  cplx F[PQMC_N_FIELD];
-  for (int c1 = threadIdx.x; c1 < V.nc; c1 += blockDim.x) {
-    int c2 = V.c2_of[c1 + (size_t)V.nc * ind];
-    pair_obs(V, c1, c2, F);
-    for (int f = 0; f < PQMC_N_FIELD; ++f) part[f] = cadd(part[f], F[f]);
-  }
-  for (int f = 0; f < PQMC_N_FIELD; ++f) {
-    for (int comp = 0; comp < 2; ++comp) {
-      red[threadIdx.x] = comp ? part[f].y : part[f].x;
-      __syncthreads();
-      for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
+// the second term of the spin currents of two bonds, (vx, vx) and (vy, vy);
+// bq: the phase that stands for the right bond's in (vy, vy)
+__device__ __forceinline__ void spin_exchange(const MeasView& V, const Bond& L, const Bond& R, cplx bq, cplx* xx,
+                                              cplx* yy) {
+  cplx pp[2][2], mm[2][2];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      cplx e[2][2];   // site pairs (l1, l2) = (i, 3 - i), (r1, r2) = (j, 3 - j)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int l = 2 * a + i, r = 2 * b + j;
+          e[i][j] = cmul(GH(V, R.s[3 - r], L.s[l]), GG(V, L.s[3 - l], R.s[r]));
+        }
+      pp[a][b] = cadd(cadd(e[0][0], e[0][1]), cadd(e[1][0], e[1][1]));
+      mm[a][b] = cadd(csub(e[0][0], e[0][1]), csub(e[1][1], e[1][0]));
+      if (a != b) {
+        pp[a][b] = cneg(pp[a][b]);
+        mm[a][b] = cneg(mm[a][b]);
       }
-      if (threadIdx.x == 0) {
-        cplx* dst = acc + PQMC_N_SCALAR + (size_t)f * V.nc + ind;
-        if (comp) dst->y += red[0];
-        else dst->x += red[0];
-      }
-      __syncthreads();
     }
+  const double h2 = V.hop * V.hop;
+  const cplx x = phases(L.b, R.b, pp), y = phases(L.b, bq, mm);
+  *xx = mk(-h2 * x.x, -h2 * x.y);
+  *yy = mk(h2 * y.x, h2 * y.y);
+}
+
+// k z + e w, k the coefficient of a spin-flipping pair in the physical
+// current: -i hop (X) or -hop, times sg
+template <bool X>
+__device__ __forceinline__ cplx flip_keep(double hop, double sg, cplx z, double e, cplx w) {
+  const double k = -sg * hop;
+  return X ? mk(fma(e, w.x, -k * z.y), fma(e, w.y, k * z.x)) : mk(fma(e, w.x, k * z.x), fma(e, w.y, k * z.y));
+}
+
+// sum of v(i) gh(l2,l1) over a bond's eight pairs, e the spin-conserving coefficient
+template <bool X>
+__device__ __forceinline__ cplx phys_sum(const MeasView& V, const Bond& B, double e) {
+  auto g = [&](int l2, int l1) { return GH(V, B.s[l2], B.s[l1]); };
+  const cplx f0 = X ? cadd(g(3, 0), g(2, 1)) : csub(g(3, 0), g(2, 1));
+  const cplx f1 = X ? cadd(g(1, 2), g(0, 3)) : csub(g(1, 2), g(0, 3));
+  const cplx u = flip_keep<X>(V.hop, 1.0, f0, e, cadd(g(2, 0), g(3, 1)));
+  const cplx w = flip_keep<X>(V.hop, -1.0, f1, e, cadd(g(0, 2), g(1, 3)));
+  return cfma(B.b, u, cmul(cconj(B.b), w));
+}
+
+// physical current-current of two bonds along one direction; X: the spin
+// part is vx, else vy; e1, e2: ep x of the bonds
+template <bool X>
+__device__ __forceinline__ cplx phys_pair(const MeasView& V, const Bond& L, const Bond& R, double e1, double e2) {
+  cplx t[2][2];
+  // columns of P VL and Q VR by the second site, 3 and 2 with the phase, 1
+  // and 0 with its conjugate; a column takes two of P's (Q's)
+  const double s1 = X ? 1.0 : -1.0;
+  cplx y[4][4];   // [l2][r2]
+#pragma unroll
+  for (int l2 = 0; l2 < 4; ++l2) {
+    cplx q[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) q[r] = GG(V, L.s[l2], R.s[r]);
+    y[l2][3] = flip_keep<X>(V.hop, 1.0, q[0], e2, q[1]);
+    y[l2][2] = flip_keep<X>(V.hop, s1, q[1], e2, q[0]);
+    y[l2][1] = flip_keep<X>(V.hop, -1.0, q[2], e2, q[3]);
+    y[l2][0] = flip_keep<X>(V.hop, -s1, q[3], e2, q[2]);
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) t[a][b] = mk(0.0);
+#pragma unroll
+  for (int r2 = 0; r2 < 4; ++r2) {
+    cplx q[4], x[4];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) q[l] = GH(V, R.s[r2], L.s[l]);
+    x[3] = flip_keep<X>(V.hop, 1.0, q[0], e1, q[1]);
+    x[2] = flip_keep<X>(V.hop, s1, q[1], e1, q[0]);
+    x[1] = flip_keep<X>(V.hop, -1.0, q[2], e1, q[3]);
+    x[0] = flip_keep<X>(V.hop, -s1, q[3], e1, q[2]);
+    const int b = r2 < 2 ? 1 : 0;
+#pragma unroll
+    for (int l2 = 0; l2 < 4; ++l2) t[l2 < 2 ? 1 : 0][b] = cfma(x[l2], y[l2][r2], t[l2 < 2 ? 1 : 0][b]);
+  }
+  return cfma(phys_sum<X>(V, L, e1), phys_sum<X>(V, R, e2), phases(L.b, R.b, t));
+}
+
+// The observables of a pair in five parts of about equal work (the current
+// correlations along y and x, the spin currents along y, x and crossed) and
+// a light one (density, spin, pairing, phonons).  One CTA per part and
+// relative displacement: the longest CTA is then 1/5 of a pair, and the
+// 6 n_cell CTAs spread evenly.
+constexpr int MEAS_PARTS = 6;
+constexpr int MEAS_MAX = 9;   // observables of a part, at most
+__device__ __constant__ const signed char meas_field[MEAS_PARTS][MEAS_MAX] = {
+    {PQMC_F_CJYX_CJYX, -1},
+    {PQMC_F_CJXY_CJXY, -1},
+    {PQMC_F_JXX_JYX, PQMC_F_JXY_JYY, PQMC_F_JXXH_JYXH, PQMC_F_JXYH_JYYH, PQMC_F_JXXH_JYYH, PQMC_F_JXYH_JYXH, -1},
+    {PQMC_F_JYX_JYX, PQMC_F_JYY_JYY, PQMC_F_JYXH_JYXH, PQMC_F_JYYH_JYYH, -1},
+    {PQMC_F_JXX_JXX, PQMC_F_JXY_JXY, PQMC_F_JXXH_JXXH, PQMC_F_JXYH_JXYH, -1},
+    {PQMC_F_DEN_DEN, PQMC_F_SZ_SZ, PQMC_F_SX_SX, PQMC_F_SY_SY, PQMC_F_SC_SC, PQMC_F_BFX_BFX, PQMC_F_BFX_BFY,
+     PQMC_F_BFY_BFY, PQMC_F_BFXY_BFXY}};
+__device__ __constant__ const int meas_count[MEAS_PARTS] = {1, 1, 6, 4, 4, 9};
+
+// adds one pair's observables of `part` (uniform over the CTA) to f
+__device__ __forceinline__ void pair_obs(const MeasView& V, int part, int c1, int c2, cplx (&f)[MEAS_MAX]) {
+  if (part == 0) {
+    f[0] = cadd(f[0], phys_pair<true>(V, bond(V, c1, 1), bond(V, c2, 1), V.ep * boson(V, c1, 1),
+                                      V.ep * boson(V, c2, 1)));
+  } else if (part == 1) {
+    f[0] = cadd(f[0], phys_pair<false>(V, bond(V, c1, 0), bond(V, c2, 0), V.ep * boson(V, c1, 0),
+                                       V.ep * boson(V, c2, 0)));
+  } else if (part < 5) {
+    const Bond L = bond(V, c1, part == 3 ? 1 : 0), R = bond(V, c2, part == 4 ? 0 : 1);
+    const bool quirk = part == 3;   // (vy, vy) along y takes the left phases twice (:353, :417)
+    cplx lx, ly, rx, ry, xx, yy;
+    spin_exchange(V, L, R, quirk ? L.b : R.b, &xx, &yy);
+    spin_sums(V, L, &lx, &ly);
+    spin_sums(V, R, &rx, &ry);
+    cplx rq = ry;
+    if (quirk) {
+      Bond Q = R;
+      Q.b = L.b;
+      cplx unused;
+      spin_sums(V, Q, &unused, &rq);
+    }
+    const cplx hx = cmul(lx, rx), hy = cmul(ly, rq);
+    f[0] = cadd(f[0], cadd(hx, xx));
+    f[1] = cadd(f[1], cadd(hy, yy));
+    f[2] = cadd(f[2], hx);
+    f[3] = cadd(f[3], hy);
+    if (part == 2) {
+      f[4] = cfma(lx, ry, f[4]);
+      f[5] = cfma(ly, rx, f[5]);
+    }
+  } else {
+    const int u1 = V.sites[2 * c1], d1 = V.sites[2 * c1 + 1], u2 = V.sites[2 * c2], d2 = V.sites[2 * c2 + 1];
+    const cplx puu = GH(V, u2, u1), pud = GH(V, u2, d1), pdu = GH(V, d2, u1), pdd = GH(V, d2, d1);   // gh(r, l)
+    const cplx quu = GG(V, u1, u2), qud = GG(V, u1, d2), qdu = GG(V, d1, u2), qdd = GG(V, d1, d2);   // g(l, r)
+    const cplx a0 = GH(V, u1, u1), a1 = GH(V, d1, u1), a2 = GH(V, u1, d1), a3 = GH(V, d1, d1);       // gh(l2, l1)
+    const cplx b0 = GH(V, u2, u2), b1 = GH(V, d2, u2), b2 = GH(V, u2, d2), b3 = GH(V, d2, d2);
+    // pairs (u,u), (d,d) on both sides: mat(i,j) for density and s_z
+    const cplx s = cadd(cmul(puu, quu), cmul(pdd, qdd)), o = cadd(cmul(pdu, qud), cmul(pud, qdu));
+    const cplx den = cadd(cmul(cadd(a0, a3), cadd(b0, b3)), cadd(s, o));
+    const cplx sz = cadd(cmul(csub(a0, a3), csub(b0, b3)), csub(s, o));
+    // pairs (u,d), (d,u): s_x = (1 + 2) / 2, s_y = (-i 1 + i 2) / 2
+    const cplx e11 = cmul(pdu, qdu), e12 = cmul(puu, qdd), e21 = cmul(pdd, quu), e22 = cmul(pud, qud);
+    const cplx d = cadd(e11, e22), x = cadd(e12, e21);
+    const cplx sx = cadd(cmul(cadd(a1, a2), cadd(b1, b2)), cadd(d, x));
+    const cplx sy = csub(csub(x, d), cmul(csub(a1, a2), csub(b1, b2)));
+    const cplx sc = csub(cmul(puu, pdd), cmul(pdu, pud));
+    f[0] = mk(fma(0.25, den.x, f[0].x), fma(0.25, den.y, f[0].y));
+    f[1] = mk(fma(0.25, sz.x, f[1].x), fma(0.25, sz.y, f[1].y));
+    f[2] = mk(fma(0.25, sx.x, f[2].x), fma(0.25, sx.y, f[2].y));
+    f[3] = mk(fma(0.25, sy.x, f[3].x), fma(0.25, sy.y, f[3].y));
+    f[4] = cadd(f[4], sc);
+    const double x1x = boson(V, c1, 0), x1y = boson(V, c1, 1), x2x = boson(V, c2, 0), x2y = boson(V, c2, 1);
+    f[5].x = fma(x1x, x2x, f[5].x);
+    f[6].x = fma(x1x, x2y, f[6].x);
+    f[7].x = fma(x1y, x2y, f[7].x);
+    f[8].x = fma(x1x * x1y, x2x * x2y, f[8].x);
   }
 }
 
-// BF_KE, BF_PE, BF_X per cell in cell order (:249-268)
-__global__ void k_meas_scalars(MeasView V, double D, double M, double biased, double delt, cplx* acc) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+constexpr int MEAS_THREADS = 224;   // at most; a lattice of 14 x 14 cells fills them
+
+// the sums over the CTA of n values per thread, in a fixed order; sum v is
+// returned by lane 0 of warp v % warps in `out`
+template <class F>
+__device__ __forceinline__ void meas_sum(int n, double (*s)[MEAS_THREADS], F out) {
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int v = warp; v < n; v += nw) {
+    double a = s[v][lane];
+    for (int k = lane + 32; k < blockDim.x; k += 32) a += s[v][k];
+    for (int m = 16; m > 0; m >>= 1) a += __shfl_xor_sync(~0u, a, m);
+    if (lane == 0) out(v, a);
+  }
+}
+
+// CTAs 0 .. 6 n_cell - 1: a part of the pair observables at one relative
+// displacement `ind`, each thread the pairs (c1, c2) with rel(c1, c2) = ind of
+// its cells c1.  The last CTA: BF_KE, BF_PE, BF_X (:249-268).  Measured at
+// 196 cells 167 us, of which FP64 issue alone is ~85 (one CTA per
+// displacement with all observables as written out: 594 us, and 337 for the
+// scalars by one thread); at 16 cells 23 us (196 and 29).
+__global__ void __launch_bounds__(MEAS_THREADS) k_meas_pairs(MeasView V, double D, double M, double biased, double delt,
+                                                             cplx* acc) {
+  __shared__ double s[2 * MEAS_MAX][MEAS_THREADS];
+  const int tid = threadIdx.x;
   const double N = (double)V.nc;
-  const int t = V.t;
-  for (int c1 = 0; c1 < V.nc; ++c1) {
-    int bx = V.bfi[2 * c1], by = V.bfi[2 * c1 + 1];
-    double x1x = V.field[bx + (size_t)V.n_bf * t], x1y = V.field[by + (size_t)V.n_bf * t];
-    double o = (0.5 * D) * (x1x * x1x + x1y * x1y) - biased * (x1x + x1y);
-    acc[PQMC_OBS_BF_KE] = cadd(acc[PQMC_OBS_BF_KE], mk(o / N));
-    double d1 = x1x - V.field[bx + (size_t)V.n_bf * (t + 1)], d2 = x1y - V.field[by + (size_t)V.n_bf * (t + 1)];
-    double q = 0.0 - ((0.5 * M) * (d1 * d1 + d2 * d2)) / (delt * delt);
-    q = q + (1.0 / (2.0 * delt)) * 2.0;
-    acc[PQMC_OBS_BF_PE] = cadd(acc[PQMC_OBS_BF_PE], mk(q / N));
-    acc[PQMC_OBS_BF_X] = cadd(acc[PQMC_OBS_BF_X], mk((x1x + x1y) / N));
+  if (blockIdx.x == MEAS_PARTS * V.nc) {
+    double ke = 0.0, pe = 0.0, xs = 0.0;
+    for (int c = tid; c < V.nc; c += blockDim.x) {
+      const double* x = V.field + (size_t)V.n_bf * V.t;
+      const int bx = V.bfi[2 * c], by = V.bfi[2 * c + 1];
+      const double x1x = x[bx], x1y = x[by], d1 = x1x - x[bx + V.n_bf], d2 = x1y - x[by + V.n_bf];
+      ke += (0.5 * D) * (x1x * x1x + x1y * x1y) - biased * (x1x + x1y);
+      pe += (1.0 / (2.0 * delt)) * 2.0 - ((0.5 * M) * (d1 * d1 + d2 * d2)) / (delt * delt);
+      xs += x1x + x1y;
+    }
+    s[PQMC_OBS_BF_KE][tid] = ke;
+    s[PQMC_OBS_BF_PE][tid] = pe;
+    s[PQMC_OBS_BF_X][tid] = xs;
+    meas_sum(PQMC_N_SCALAR, s, [&](int v, double a) { acc[v].x += a / N; });
+    return;
   }
+  const int part = blockIdx.x / V.nc, ind = blockIdx.x % V.nc;
+  cplx f[MEAS_MAX];
+#pragma unroll
+  for (int k = 0; k < MEAS_MAX; ++k) f[k] = mk(0.0);
+  for (int c1 = tid; c1 < V.nc; c1 += blockDim.x) pair_obs(V, part, c1, V.c2_of[c1 + (size_t)V.nc * ind], f);
+  const int n = meas_count[part];
+#pragma unroll
+  for (int k = 0; k < MEAS_MAX; ++k)
+    if (k < n) {
+      s[2 * k][tid] = f[k].x;
+      s[2 * k + 1][tid] = f[k].y;
+    }
+  meas_sum(2 * n, s, [&](int v, double a) {
+    cplx* dst = acc + PQMC_N_SCALAR + (size_t)meas_field[part][v >> 1] * V.nc + ind;
+    if (v & 1) dst->y += a / N;
+    else dst->x += a / N;
+  });
 }
 
-// window average + ms_k_space_obs
-__global__ void k_meas_finish(int nc, double div, const cplx* __restrict__ kphase, cplx* acc) {
-  // divide r-space part (block 0 does it first, others wait through a second launch)
-  const int f = blockIdx.x, ik = threadIdx.x + blockIdx.y * blockDim.x;
-  if (ik >= nc) return;
+// ms_k_space_obs of the averaged real-space part: sixteen k per CTA, the sum
+// over the cells in MEAS_KSPLIT shares.  FP64 issue bounds it (4 n_cell
+// multiply-adds per output); the window's average was divided out of each
+// term here before (two divisions per four multiply-adds): 263 us at 196 cells,
+// now 13.
+constexpr int MEAS_KSPLIT = 8;
+__global__ void __launch_bounds__(16 * MEAS_KSPLIT) k_meas_finish(int nc, const cplx* __restrict__ kphase, cplx* acc) {
+  __shared__ cplx part[MEAS_KSPLIT][16];
+  const int f = blockIdx.x, k = threadIdx.x & 15, h = threadIdx.x >> 4, ik = k + 16 * blockIdx.y;
   const cplx* r = acc + PQMC_N_SCALAR + (size_t)f * nc;
   cplx s = mk(0.0);
-  for (int i = 0; i < nc; ++i) {
-    cplx rv = r[i];
-    rv = mk(rv.x / div, rv.y / div);
-    s = cfma(kphase[ik + (size_t)nc * i], rv, s);
+  if (ik < nc)
+    for (int i = h; i < nc; i += MEAS_KSPLIT) s = cfma(kphase[ik + (size_t)nc * i], r[i], s);
+  part[h][k] = s;
+  __syncthreads();
+  if (h == 0 && ik < nc) {
+    for (int j = 1; j < MEAS_KSPLIT; ++j) s = cadd(s, part[j][k]);
+    cplx* kd = acc + PQMC_N_SCALAR + (size_t)(PQMC_N_FIELD + f) * nc;
+    kd[ik] = cadd(kd[ik], mk(s.x / (double)nc, s.y / (double)nc));
   }
-  cplx* kd = acc + PQMC_N_SCALAR + (size_t)(PQMC_N_FIELD + f) * nc;
-  kd[ik] = cadd(kd[ik], mk(s.x / (double)nc, s.y / (double)nc));
 }
 
+// window average
 __global__ void k_meas_divide(int n, double div, cplx* acc) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     acc[i] = mk(acc[i].x / div, acc[i].y / div);
@@ -261,20 +368,19 @@ static MeasView view(pqmc_chain* c, int time) {
 
 int do_measure(pqmc_chain* c, int time) {
   MeasView V = view(c, time);
-  k_meas_scalars<<<1, 1, 0, c->stream>>>(V, c->M.stiff, c->M.mass, c->M.biased, c->M.delt, c->m_acc);
-  PQMC_LAUNCHED();
-  k_meas_pairs<<<c->n_cell, MEAS_THREADS, 0, c->stream>>>(V, c->m_acc);
+  const int threads = std::min(MEAS_THREADS, (c->n_cell + 31) / 32 * 32);
+  k_meas_pairs<<<MEAS_PARTS * c->n_cell + 1, threads, 0, c->stream>>>(V, c->M.stiff, c->M.mass, c->M.biased, c->M.delt,
+                                                                      c->m_acc);
   PQMC_LAUNCHED();
   return PQMC_OK;
 }
 
 int do_finish_record(pqmc_chain* c, int meas_number) {
-  const int nc = c->n_cell;
-  double div = (double)(2 * meas_number + 1);
-  dim3 g(PQMC_N_FIELD, (nc + 127) / 128);
-  k_meas_finish<<<g, 128, 0, c->stream>>>(nc, div, c->m_kphase, c->m_acc);
+  const int nc = c->n_cell, n = PQMC_N_SCALAR + PQMC_N_FIELD * nc;
+  k_meas_divide<<<(n + 127) / 128, 128, 0, c->stream>>>(n, (double)(2 * meas_number + 1), c->m_acc);
   PQMC_LAUNCHED();
-  k_meas_divide<<<8, 256, 0, c->stream>>>(PQMC_N_SCALAR + PQMC_N_FIELD * nc, div, c->m_acc);
+  dim3 g(PQMC_N_FIELD, (nc + 15) / 16);
+  k_meas_finish<<<g, 16 * MEAS_KSPLIT, 0, c->stream>>>(nc, c->m_kphase, c->m_acc);
   PQMC_LAUNCHED();
   return PQMC_OK;
 }

@@ -134,6 +134,22 @@ def test_measurement(engine):
     assert np.allclose(rg, ro, rtol=1e-10, atol=1e-12)
 
 
+@pytest.mark.parametrize("L,meas_number", [((4, 2), 0), ((6, 6), 1), ((16, 16), 0)])
+def test_measurement_of_a_given_g(L, meas_number):
+    """Fewer cells than a warp, a remainder, and more cells than the CTA has
+    threads, with twisted boundary phases, on the oracle's own G: entries of
+    order one in sums of n_cell terms, so errors stay below n_cell eps ~ 6e-14;
+    1e-12 leaves an order of room."""
+    m, o, g = _pair(epsocz_small, L=L, ntime=8, ngroup=4, lam=0.8, alpha=0.3, bc=(0.3, 0.7))
+    o.init_expkv(); o.init_g(1)
+    g.init_expkv(); g.set_g(o.g())
+    half = m.ntime // 2
+    for t in range(half - meas_number, half + meas_number + 1):
+        ro, rg = o.begin_measure(True, t, meas_number), g.begin_measure(True, t, meas_number)
+    assert np.abs(ro).max() > 0.1
+    assert np.allclose(rg, ro, rtol=1e-12, atol=1e-12)
+
+
 def _c1_model():
     """The 4x4 configuration with phonon-modulated bonds t(1 - lambda x_b),
     lambda = 0.8, 32 bonds, spin 1/2 as ncopy = 2 (weight det^ncopy,
