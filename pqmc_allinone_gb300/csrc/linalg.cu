@@ -12,65 +12,92 @@ namespace pqmc {
 
 // ---------------------------------------------------------------------------
 // C = alpha * op(A) * op(B) + beta * C, op in {N, C (conjugate transpose)}.
-// 32x32 output tile per CTA, 256 threads, 2x2 outputs per thread, k-tiles of
-// 16 staged in shared memory.
+//
+// FP64 issue bounds it: a multiply-add holds an SM quarter for 64 cycles, so
+// one warp per quarter is enough and operands come straight from L1 (two
+// 16-byte loads per four multiply-adds).  What is left is to give every
+// quarter the same work: a warp makes 32, 16, 8 or 4 outputs with the sum over
+// k in 1, 2, 4 or 8 shares, whichever leaves the fullest quarter the least.
+// Measured for 196 x 196 x 392, 392 x 392 x 196 and 32 x 32 x 8: 111, 207 and
+// 2.6 us (FP64 issue alone 103 and 206); as 32 x 32 tiles through shared
+// memory, 49 and 169 CTAs, 432, 428 and 19.
+constexpr int ZG_AHEAD = 4;   // elements of the sum in flight
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_zgemm(int m, int n, int k, cplx alpha, const cplx* __restrict__ A,
-                                                int lda, const cplx* __restrict__ B, int ldb, cplx beta,
-                                                cplx* __restrict__ C, int ldc) {
-  __shared__ cplx sA[16][33];
-  __shared__ cplx sB[16][33];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int row0 = blockIdx.x * 32, col0 = blockIdx.y * 32;
-  cplx acc[2][2] = {{mk(0), mk(0)}, {mk(0), mk(0)}};
-  for (int kk = 0; kk < k; kk += 16) {
-    // A tile: rows row0..row0+31, k kk..kk+15 -> sA[k][row]
-    for (int e = threadIdx.x; e < 16 * 32; e += 256) {
-      int r = e & 31, q = e >> 5;
-      int gr = row0 + r, gk = kk + q;
-      cplx v = mk(0);
-      if (gr < m && gk < k) v = TA ? cconj(A[gk + (size_t)lda * gr]) : A[gr + (size_t)lda * gk];
-      sA[q][r] = v;
-    }
-    for (int e = threadIdx.x; e < 16 * 32; e += 256) {
-      int q = e & 15, c = e >> 4;
-      int gc = col0 + c, gk = kk + q;
-      cplx v = mk(0);
-      if (gc < n && gk < k) v = TB ? cconj(B[gc + (size_t)ldb * gk]) : B[gk + (size_t)ldb * gc];
-      sB[q][c] = v;
-    }
-    __syncthreads();
+__global__ void __launch_bounds__(128) k_zgemm(int m, int n, int k, int ls, cplx alpha, const cplx* __restrict__ A,
+                                               int lda, const cplx* __restrict__ B, int ldb, cplx beta,
+                                               cplx* __restrict__ C, int ldc) {
+  // a warp's outputs: 2^lr x 2^lc of them, 2^ls shares of the sum
+  const int lr = (6 - ls) >> 1, lc = (5 - ls) >> 1;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int o = lane & ((32 >> ls) - 1), h = lane >> (5 - ls);
+  const int r = ((2 * blockIdx.x + (w & 1)) << lr) + (o & ((1 << lr) - 1));
+  const int c = ((2 * blockIdx.y + (w >> 1)) << lc) + (o >> lr);
+  if (((2 * blockIdx.x + (w & 1)) << lr) >= m || ((2 * blockIdx.y + (w >> 1)) << lc) >= n) return;   // the whole warp
+  const int kl = (k + (1 << ls) - 1) >> ls, k0 = min(k, h * kl), k1 = min(k, k0 + kl);
+  const int ra = min(r, m - 1), cb = min(c, n - 1);
+  const size_t da = TA ? 1 : lda, db = TB ? ldb : 1;
+  const double2* a = reinterpret_cast<const double2*>(A) + (TA ? (size_t)lda * ra : (size_t)ra) + da * k0;
+  const double2* b = reinterpret_cast<const double2*>(B) + (TB ? (size_t)cb : (size_t)ldb * cb) + db * k0;
+  const double2 zero = make_double2(0.0, 0.0);
+  double2 va[ZG_AHEAD], vb[ZG_AHEAD];
+  cplx acc = mk(0.0);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      cplx a0 = sA[q][tx], a1 = sA[q][tx + 16];
-      cplx b0 = sB[q][ty], b1 = sB[q][ty + 16];
-      acc[0][0] = cfma(a0, b0, acc[0][0]);
-      acc[1][0] = cfma(a1, b0, acc[1][0]);
-      acc[0][1] = cfma(a0, b1, acc[0][1]);
-      acc[1][1] = cfma(a1, b1, acc[1][1]);
-    }
-    __syncthreads();
+  for (int e = 0; e < ZG_AHEAD; ++e) {
+    va[e] = k0 + e < k1 ? __ldg(a + da * e) : zero;
+    vb[e] = k0 + e < k1 ? __ldg(b + db * e) : zero;
   }
-  for (int i = 0; i < 2; ++i)
-    for (int j = 0; j < 2; ++j) {
-      int r = row0 + tx + 16 * i, c = col0 + ty + 16 * j;
-      if (r < m && c < n) {
-        cplx* p = C + r + (size_t)ldc * c;
-        cplx v = cmul(alpha, acc[i][j]);
-        if (beta.x != 0.0 || beta.y != 0.0) v = cfma(beta, *p, v);
-        *p = v;
-      }
+  for (int q = 0; q < kl; q += ZG_AHEAD) {   // the same number of steps in every lane
+    a += da * ZG_AHEAD;
+    b += db * ZG_AHEAD;
+#pragma unroll
+    for (int e = 0; e < ZG_AHEAD; ++e) {
+      if (q + e >= kl) break;
+      cplx x = mk(va[e].x, va[e].y), y = mk(vb[e].x, vb[e].y);
+      const bool more = k0 + q + e + ZG_AHEAD < k1;
+      va[e] = more ? __ldg(a + da * e) : zero;
+      vb[e] = more ? __ldg(b + db * e) : zero;
+      if (TA) x = cconj(x);
+      if (TB) y = cconj(y);
+      acc = cfma(x, y, acc);
     }
+  }
+  for (int d = 16; d >= (32 >> ls); d >>= 1) {
+    acc.x += __shfl_xor_sync(~0u, acc.x, d);
+    acc.y += __shfl_xor_sync(~0u, acc.y, d);
+  }
+  if (h == 0 && r < m && c < n) {
+    cplx* p = C + r + (size_t)ldc * c;
+    cplx v = cmul(alpha, acc);
+    if (beta.x != 0.0 || beta.y != 0.0) v = cfma(beta, *p, v);
+    *p = v;
+  }
 }
 
 int zgemm(cudaStream_t s, char ta, char tb, int m, int n, int k, cplx alpha, const cplx* A, int lda,
           const cplx* B, int ldb, cplx beta, cplx* C, int ldc) {
-  dim3 grid((m + 31) / 32, (n + 31) / 32);
+  int dev = 0, nsm = 0;
+  PQMC_CUDA(cudaGetDevice(&dev));
+  PQMC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  // shares of the sum: FP64 instructions of the fullest SM quarter, a CTA
+  // being a warp on each; the largest share that is no worse
+  int ls = 0;
+  long best = 0;
+  dim3 grid;
+  for (int l = 0; l <= 3; ++l) {
+    const int th = 2 << ((6 - l) >> 1), tw = 2 << ((5 - l) >> 1);
+    const dim3 g((m + th - 1) / th, (n + tw - 1) / tw);
+    const long rounds = ((long)g.x * g.y + nsm - 1) / nsm, cost = rounds * (4L * ((k + (1 << l) - 1) >> l) + 2 * l + 8);
+    if (l == 0 || cost < best) {
+      best = cost;
+      ls = l;
+      grid = g;
+    }
+  }
   bool TA = (ta == 'C'), TB = (tb == 'C');
-  if (!TA && !TB) k_zgemm<false, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-  else if (TA && !TB) k_zgemm<true, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-  else if (!TA && TB) k_zgemm<false, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-  else k_zgemm<true, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+  if (!TA && !TB) k_zgemm<false, false><<<grid, 128, 0, s>>>(m, n, k, ls, alpha, A, lda, B, ldb, beta, C, ldc);
+  else if (TA && !TB) k_zgemm<true, false><<<grid, 128, 0, s>>>(m, n, k, ls, alpha, A, lda, B, ldb, beta, C, ldc);
+  else if (!TA && TB) k_zgemm<false, true><<<grid, 128, 0, s>>>(m, n, k, ls, alpha, A, lda, B, ldb, beta, C, ldc);
+  else k_zgemm<true, true><<<grid, 128, 0, s>>>(m, n, k, ls, alpha, A, lda, B, ldb, beta, C, ldc);
   PQMC_LAUNCHED();
   return PQMC_OK;
 }
