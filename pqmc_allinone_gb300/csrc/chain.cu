@@ -95,44 +95,94 @@ int launch_wrap(pqmc_chain* c, int pf, int time, bool left) {
 // ascending, families 1..n_pf, X(S,:) <- E X(S,:).  backward: right_evolve
 // (.false.) on lmat = X^H, slices descending, families n_pf..1,
 // X(S,:) <- E^H X(S,:).  One CTA per column; the column lives in shared memory.
-__global__ void k_propagate(DevModel M, cplx* X, int ldx, int t_from, int t_to, int forward,
-                            const cplx* __restrict__ expkv) {
+//
+// FP64 issue bounds it (a multiply-add holds an SM quarter for 64 cycles with
+// however few lanes), so a plaquette takes eight lanes, one per real component
+// of its result and eight multiply-adds in a row in each; a lane's row of
+// expKV for its next item is loaded beside them.  One thread per plaquette
+// left most lanes idle.  Ten slices of four families, before and now: 212 and
+// 160 us at 392 rows (two CTAs on some SMs, hence the bound on registers: 188
+// with one at a time), 186 and 93 at 288, 165 and 29 at 32.
+constexpr int PROP_THREADS = 512;   // at most; 64 plaquettes at a time
+// v with `sgn`'s sign bit turned: no FP64 instruction
+__device__ __forceinline__ double flip_sign(double v, int sgn) {
+  return __hiloint2double(__double2hiint(v) ^ sgn, __double2loint(v));
+}
+struct PropItem {
+  double2 e[4];
+  int S[4];
+};
+// item `i` (plaquette i / 8, component i % 8) of family pf at slice t
+__device__ __forceinline__ void prop_load(const DevModel& M, const cplx* expkv, int i, int pf, int t, bool forward,
+                                          PropItem& it) {
+  const int p = i >> 3, a = (i >> 1) & 3, pd = M.pdim, dim = M.pf_dim[pf];
+  if (p >= M.pf_npla[pf] || a >= dim) return;
+  const int* S = M.site + pd * (p + M.max_pla * pf);
+  const double2* E = reinterpret_cast<const double2*>(expkv + M.kv_base(p, pf, t));
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (k < dim) {
+      it.S[k] = __ldg(S + k);
+      it.e[k] = __ldg(E + (forward ? a + pd * k : k + pd * a));
+    }
+}
+__global__ void __launch_bounds__(PROP_THREADS, 2) k_propagate(DevModel M, cplx* X, int ldx, int t_from, int t_to,
+                                                            int forward, const cplx* __restrict__ expkv) {
   extern __shared__ cplx col[];
-  const int ns = M.ns, pd = M.pdim;
+  const int ns = M.ns, tid = threadIdx.x, nth = blockDim.x;
   cplx* x = X + (size_t)ldx * blockIdx.x;
-  for (int r = threadIdx.x; r < ns; r += blockDim.x) col[r] = x[r];
-  __syncthreads();
+  for (int r = tid; r < ns; r += nth) col[r] = x[r];
   const int nt = forward ? (t_to - t_from + 1) : (t_from - t_to + 1);
-  for (int it = 0; it < nt; ++it) {
-    const int t = (forward ? t_from + it : t_from - it) - 1;
+  const int comp = tid & 1, a = (tid >> 1) & 3;
+  double* out = reinterpret_cast<double*>(col) + comp;
+  const int sgn = comp != (forward ? 0 : 1) ? 0 : (int)0x80000000;   // of ey below
+  auto family = [&](int f) { return forward ? f : M.n_pf - 1 - f; };
+  auto slice = [&](int it) { return (forward ? t_from + it : t_from - it) - 1; };
+  PropItem cur;
+  if (nt > 0 && M.n_pf > 0) prop_load(M, expkv, tid, family(0), slice(0), forward, cur);
+  __syncthreads();
+  for (int it = 0; it < nt; ++it)
     for (int f = 0; f < M.n_pf; ++f) {
-      const int pf = forward ? f : M.n_pf - 1 - f;
-      const int dim = M.pf_dim[pf], npla = M.pf_npla[pf];
-      for (int p = threadIdx.x; p < npla; p += blockDim.x) {
-        int S[4];
-        cplx v[4];
-        for (int k = 0; k < dim; ++k) {
-          S[k] = M.site[k + pd * (p + M.max_pla * pf)];
-          v[k] = col[S[k]];
-        }
-        const cplx* E = expkv + M.kv_base(p, pf, t);
-        for (int a = 0; a < dim; ++a) {
-          cplx s = mk(0.0);
-          for (int k = 0; k < dim; ++k) {
-            cplx e = forward ? E[a + pd * k] : cconj(E[k + pd * a]);
-            s = cfma(e, v[k], s);
+      const int pf = family(f), dim = M.pf_dim[pf], ni = 8 * M.pf_npla[pf];
+      for (int i0 = 0; i0 < ni; i0 += nth) {
+        const int i = i0 + tid;
+        const bool on = i < ni && a < dim;
+        PropItem nxt;
+        // the lane's next item: of this family, else the first of the next one
+        if (i0 + nth < ni) prop_load(M, expkv, i + nth, pf, slice(it), forward, nxt);
+        else if (f + 1 < M.n_pf) prop_load(M, expkv, tid, family(f + 1), slice(it), forward, nxt);
+        else if (it + 1 < nt) prop_load(M, expkv, tid, family(0), slice(it + 1), forward, nxt);
+        if (i0 + (tid & ~31) < ni) {   // any item in the warp
+          double s = 0.0;
+          if (on)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (k < dim) {
+                const cplx v = col[cur.S[k]];
+                const double ey = flip_sign(cur.e[k].y, sgn);
+                // real: ex vx - ey vy, imaginary: ex vy + ey vx (ey's sign turned for E^H)
+                s = fma(cur.e[k].x, comp ? v.y : v.x, fma(ey, comp ? v.x : v.y, s));
+              }
+          __syncwarp();   // a plaquette's eight lanes have read its rows
+          if (on) {
+            int row = cur.S[0];
+#pragma unroll
+            for (int k = 1; k < 4; ++k)
+              if (a == k) row = cur.S[k];
+            out[2 * row] = s;
           }
-          col[S[a]] = s;
         }
+        cur = nxt;
       }
       __syncthreads();
     }
-  }
-  for (int r = threadIdx.x; r < ns; r += blockDim.x) x[r] = col[r];
+  for (int r = tid; r < ns; r += nth) x[r] = col[r];
 }
 
 int launch_propagate(pqmc_chain* c, cplx* X, int n, int t_from, int t_to, bool forward) {
-  int threads = 128;
+  int items = 1;
+  for (int f = 0; f < c->n_pf; ++f) items = std::max(items, 8 * c->h_pf_npla[f]);
+  const int threads = std::min(PROP_THREADS, (items + 127) / 128 * 128);   // a warp on each SM quarter
   size_t smem = sizeof(cplx) * (size_t)c->ns;
   k_propagate<<<n, threads, smem, c->stream>>>(c->M, X, c->ns, t_from, t_to, forward ? 1 : 0, c->expkv);
   PQMC_LAUNCHED();

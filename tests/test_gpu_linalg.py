@@ -11,7 +11,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from tests.helpers import SEED_WORDS, epsocz_small, rel_fro
+from tests.helpers import SEED_WORDS, epsocz_small, general_bond_model, rel_fro
 
 pytestmark = pytest.mark.gpu
 
@@ -113,3 +113,21 @@ def test_update_shares(L):
         assert sg["rng"] == so["rng"] and np.array_equal(g.field(), o.field())
         assert sg["positive_accept"] == so["positive_accept"] > 0
         assert rel_fro(g.g(), o.g()) < 1e-10
+
+
+@pytest.mark.parametrize("build,L", [(epsocz_small, (12, 12)), (general_bond_model, 12), (epsocz_small, (16, 16))])
+def test_propagation_in_passes(build, L):
+    """Families of 72 and 128 plaquettes of four and two sites: more items than
+    the CTA has lanes, with and without a remainder, in both directions."""
+    from oracle.oracle import OracleChain
+    from pqmc_allinone_gb300.engine import PqmcChain
+    m, f = build(L=L, ntime=4, ngroup=2, lam=0.8)
+    o = OracleChain(m, field=f, seed_words=SEED_WORDS, meas=False)
+    g = PqmcChain(m, field=f, rng_words=SEED_WORDS, meas=False)
+    for c in (o, g):
+        c.init_expkv()
+    for t in (1, 3):   # through every slice from the right, and from both sides
+        for c in (o, g):
+            c.init_g(t)
+        assert rel_fro(g.g(), o.g()) < 1e-11
+    g.close()
