@@ -104,10 +104,6 @@ int launch_wrap(pqmc_chain* c, int pf, int time, bool left) {
 // 160 us at 392 rows (two CTAs on some SMs, hence the bound on registers: 188
 // with one at a time), 186 and 93 at 288, 165 and 29 at 32.
 constexpr int PROP_THREADS = 512;   // at most; 64 plaquettes at a time
-// v with `sgn`'s sign bit turned: no FP64 instruction
-__device__ __forceinline__ double flip_sign(double v, int sgn) {
-  return __hiloint2double(__double2hiint(v) ^ sgn, __double2loint(v));
-}
 struct PropItem {
   double2 e[4];
   int S[4];
@@ -135,7 +131,7 @@ __global__ void __launch_bounds__(PROP_THREADS, 2) k_propagate(DevModel M, cplx*
   const int nt = forward ? (t_to - t_from + 1) : (t_from - t_to + 1);
   const int comp = tid & 1, a = (tid >> 1) & 3;
   double* out = reinterpret_cast<double*>(col) + comp;
-  const int sgn = comp != (forward ? 0 : 1) ? 0 : (int)0x80000000;   // of ey below
+  const bool minus = comp == (forward ? 0 : 1);   // of ey below
   auto family = [&](int f) { return forward ? f : M.n_pf - 1 - f; };
   auto slice = [&](int it) { return (forward ? t_from + it : t_from - it) - 1; };
   PropItem cur;
@@ -159,7 +155,7 @@ __global__ void __launch_bounds__(PROP_THREADS, 2) k_propagate(DevModel M, cplx*
             for (int k = 0; k < 4; ++k)
               if (k < dim) {
                 const cplx v = col[cur.S[k]];
-                const double ey = flip_sign(cur.e[k].y, sgn);
+                const double ey = flip_sign(cur.e[k].y, minus);
                 // real: ex vx - ey vy, imaginary: ex vy + ey vx (ey's sign turned for E^H)
                 s = fma(cur.e[k].x, comp ? v.y : v.x, fma(ey, comp ? v.x : v.y, s));
               }

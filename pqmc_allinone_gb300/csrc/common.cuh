@@ -13,7 +13,21 @@ typedef double2 cplx;
 __host__ __device__ __forceinline__ cplx mk(double r, double i = 0.0) { return make_double2(r, i); }
 __host__ __device__ __forceinline__ cplx cadd(cplx a, cplx b) { return mk(a.x + b.x, a.y + b.y); }
 __host__ __device__ __forceinline__ cplx csub(cplx a, cplx b) { return mk(a.x - b.x, a.y - b.y); }
-__host__ __device__ __forceinline__ cplx cneg(cplx a) { return mk(-a.x, -a.y); }
+#ifdef __CUDACC__
+// v, or -v where `neg`, by its sign bit.  A negation that does not end up as
+// an operand of a multiply-add is an FP64 instruction of its own otherwise,
+// 64 cycles of an SM quarter like any other.
+__device__ __forceinline__ double flip_sign(double v, bool neg) {
+  return __hiloint2double(__double2hiint(v) ^ (neg ? (int)0x80000000 : 0), __double2loint(v));
+}
+#endif
+__host__ __device__ __forceinline__ cplx cneg(cplx a) {
+#ifdef __CUDA_ARCH__
+  return mk(flip_sign(a.x, true), flip_sign(a.y, true));
+#else
+  return mk(-a.x, -a.y);
+#endif
+}
 __host__ __device__ __forceinline__ cplx cmul(cplx a, cplx b) {
   return mk(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }

@@ -221,7 +221,7 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
   h.beta = __longlong_as_double(__double_as_longlong(sqrt(n2)) | sign);
   h.z = mk(alpha.x - h.beta, alpha.y);
   const double den = h.beta * fma(h.z.x, h.z.x, h.z.y * h.z.y);
-  const double r = ((threadIdx.x & 1) ? -h.z.y : h.z.x) / den;   // both components in one division
+  const double r = flip_sign((threadIdx.x & 1) ? h.z.y : h.z.x, threadIdx.x & 1) / den;   // both components in one division
   h.c = mk(__shfl_sync(0xffffffffu, r, 0), __shfl_sync(0xffffffffu, r, 1));
   if (__double_as_longlong(ss) == 0 && (__double_as_longlong(alpha.y) << 1) == 0) {   // nothing below the diagonal: H = I
     h.z = h.c = mk(0.0);

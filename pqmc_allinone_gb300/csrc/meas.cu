@@ -33,9 +33,10 @@ __device__ __forceinline__ cplx GH(const MeasView& V, int i, int j) {
   const double2 v = __ldg(reinterpret_cast<const double2*>(V.gh) + i + (size_t)V.ns * j);
   return mk(v.x, v.y);
 }
-__device__ __forceinline__ cplx GG(const MeasView& V, int i, int j) {
-  cplx v = cneg(GH(V, i, j));
-  if (i == j) v = cadd(v, mk(1.0));
+// -g = gh - 1 (its sign goes into the sums)
+__device__ __forceinline__ cplx GN(const MeasView& V, int i, int j) {
+  cplx v = GH(V, i, j);
+  if (i == j) v.x -= 1.0;
   return v;
 }
 
@@ -105,7 +106,7 @@ __device__ __forceinline__ void spin_exchange(const MeasView& V, const Bond& L, 
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int l = 2 * a + i, r = 2 * b + j;
-          e[i][j] = cmul(GH(V, R.s[3 - r], L.s[l]), GG(V, L.s[3 - l], R.s[r]));
+          e[i][j] = cmul(GH(V, R.s[3 - r], L.s[l]), GN(V, L.s[3 - l], R.s[r]));
         }
       pp[a][b] = cadd(cadd(e[0][0], e[0][1]), cadd(e[1][0], e[1][1]));
       mm[a][b] = cadd(csub(e[0][0], e[0][1]), csub(e[1][1], e[1][0]));
@@ -116,8 +117,8 @@ __device__ __forceinline__ void spin_exchange(const MeasView& V, const Bond& L, 
     }
   const double h2 = V.hop * V.hop;
   const cplx x = phases(L.b, R.b, pp), y = phases(L.b, bq, mm);
-  *xx = mk(-h2 * x.x, -h2 * x.y);
-  *yy = mk(h2 * y.x, h2 * y.y);
+  *xx = mk(h2 * x.x, h2 * x.y);
+  *yy = mk(-h2 * y.x, -h2 * y.y);
 }
 
 // k z + e w, k the coefficient of a spin-flipping pair in the physical
@@ -152,7 +153,7 @@ __device__ __forceinline__ cplx phys_pair(const MeasView& V, const Bond& L, cons
   for (int l2 = 0; l2 < 4; ++l2) {
     cplx q[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) q[r] = GG(V, L.s[l2], R.s[r]);
+    for (int r = 0; r < 4; ++r) q[r] = GN(V, L.s[l2], R.s[r]);
     y[l2][3] = flip_keep<X>(V.hop, 1.0, q[0], e2, q[1]);
     y[l2][2] = flip_keep<X>(V.hop, s1, q[1], e2, q[0]);
     y[l2][1] = flip_keep<X>(V.hop, -1.0, q[2], e2, q[3]);
@@ -175,7 +176,7 @@ __device__ __forceinline__ cplx phys_pair(const MeasView& V, const Bond& L, cons
 #pragma unroll
     for (int l2 = 0; l2 < 4; ++l2) t[l2 < 2 ? 1 : 0][b] = cfma(x[l2], y[l2][r2], t[l2 < 2 ? 1 : 0][b]);
   }
-  return cfma(phys_sum<X>(V, L, e1), phys_sum<X>(V, R, e2), phases(L.b, R.b, t));
+  return csub(cmul(phys_sum<X>(V, L, e1), phys_sum<X>(V, R, e2)), phases(L.b, R.b, t));
 }
 
 // The observables of a pair in five parts of about equal work (the current
@@ -229,18 +230,18 @@ __device__ __forceinline__ void pair_obs(const MeasView& V, int part, int c1, in
   } else {
     const int u1 = V.sites[2 * c1], d1 = V.sites[2 * c1 + 1], u2 = V.sites[2 * c2], d2 = V.sites[2 * c2 + 1];
     const cplx puu = GH(V, u2, u1), pud = GH(V, u2, d1), pdu = GH(V, d2, u1), pdd = GH(V, d2, d1);   // gh(r, l)
-    const cplx quu = GG(V, u1, u2), qud = GG(V, u1, d2), qdu = GG(V, d1, u2), qdd = GG(V, d1, d2);   // g(l, r)
+    const cplx quu = GN(V, u1, u2), qud = GN(V, u1, d2), qdu = GN(V, d1, u2), qdd = GN(V, d1, d2);   // -g(l, r)
     const cplx a0 = GH(V, u1, u1), a1 = GH(V, d1, u1), a2 = GH(V, u1, d1), a3 = GH(V, d1, d1);       // gh(l2, l1)
     const cplx b0 = GH(V, u2, u2), b1 = GH(V, d2, u2), b2 = GH(V, u2, d2), b3 = GH(V, d2, d2);
     // pairs (u,u), (d,d) on both sides: mat(i,j) for density and s_z
     const cplx s = cadd(cmul(puu, quu), cmul(pdd, qdd)), o = cadd(cmul(pdu, qud), cmul(pud, qdu));
-    const cplx den = cadd(cmul(cadd(a0, a3), cadd(b0, b3)), cadd(s, o));
-    const cplx sz = cadd(cmul(csub(a0, a3), csub(b0, b3)), csub(s, o));
+    const cplx den = csub(cmul(cadd(a0, a3), cadd(b0, b3)), cadd(s, o));
+    const cplx sz = csub(cmul(csub(a0, a3), csub(b0, b3)), csub(s, o));
     // pairs (u,d), (d,u): s_x = (1 + 2) / 2, s_y = (-i 1 + i 2) / 2
     const cplx e11 = cmul(pdu, qdu), e12 = cmul(puu, qdd), e21 = cmul(pdd, quu), e22 = cmul(pud, qud);
     const cplx d = cadd(e11, e22), x = cadd(e12, e21);
-    const cplx sx = cadd(cmul(cadd(a1, a2), cadd(b1, b2)), cadd(d, x));
-    const cplx sy = csub(csub(x, d), cmul(csub(a1, a2), csub(b1, b2)));
+    const cplx sx = csub(cmul(cadd(a1, a2), cadd(b1, b2)), cadd(d, x));
+    const cplx sy = csub(csub(d, x), cmul(csub(a1, a2), csub(b1, b2)));
     const cplx sc = csub(cmul(puu, pdd), cmul(pdu, pud));
     f[0] = mk(fma(0.25, den.x, f[0].x), fma(0.25, den.y, f[0].y));
     f[1] = mk(fma(0.25, sz.x, f[1].x), fma(0.25, sz.y, f[1].y));
@@ -274,9 +275,9 @@ __device__ __forceinline__ void meas_sum(int n, double (*s)[MEAS_THREADS], F out
 // CTAs 0 .. 6 n_cell - 1: a part of the pair observables at one relative
 // displacement `ind`, each thread the pairs (c1, c2) with rel(c1, c2) = ind of
 // its cells c1.  The last CTA: BF_KE, BF_PE, BF_X (:249-268).  Measured at
-// 196 cells 167 us, of which FP64 issue alone is ~85 (one CTA per
+// 196 cells 142 us, of which FP64 issue alone is ~80 (one CTA per
 // displacement with all observables as written out: 594 us, and 337 for the
-// scalars by one thread); at 16 cells 23 us (196 and 29).
+// scalars by one thread); at 16 cells 22 us (196 and 29).
 __global__ void __launch_bounds__(MEAS_THREADS) k_meas_pairs(MeasView V, double D, double M, double biased, double delt,
                                                              cplx* acc) {
   __shared__ double s[2 * MEAS_MAX][MEAS_THREADS];

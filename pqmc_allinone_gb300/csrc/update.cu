@@ -24,7 +24,7 @@
 // from the twelve 2x2 minors of the row pairs, and no separate FP32 screen.
 // The other CTAs need Ns^2 dim complex multiply-adds per accepted move, 4.3 us
 // of the whole chip at Ns = 392 (8.6 us a move with the hand-over).  A family
-// step at 4x4 with Gaussian proposals takes 52 us (413 with one worker CTA
+// step at 4x4 with Gaussian proposals takes 49 us (413 with one worker CTA
 // and 16 complex lanes), at 14x14 0.53 ms (0.91).
 #include <cooperative_groups.h>
 #include "chain.cuh"
@@ -57,7 +57,7 @@ __device__ __forceinline__ double accept_threshold(const DevModel& M, double dE,
 
 // real component c (0 re, 1 im) of acc + x*y, the two products of cfma in its order
 __device__ __forceinline__ double cfma_part(cplx x, cplx y, double acc, int c) {
-  const double bx = c ? y.y : y.x, by = c ? y.x : -y.y;
+  const double bx = c ? y.y : y.x, by = flip_sign(c ? y.x : y.y, !c);
   return fma(x.x, bx, fma(x.y, by, acc));
 }
 __device__ __forceinline__ double ldg_part(const cplx* p, int c) { return __ldcg(reinterpret_cast<const double*>(p) + c); }
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
               double dt = 0.0;
               if (dq < 6) {
                 dt = cfma_part(B.min[dq], B.min[11 - dq], 0.0, dc);
-                if (dq == 1 || dq == 4) dt = -dt;
+                dt = flip_sign(dt, dq == 1 || dq == 4);
               }
 #pragma unroll
               for (int o = 4; o > 0; o >>= 1) dt += __shfl_xor_sync(0xffffffffu, dt, o);
@@ -449,9 +449,9 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
               double cof = cfma_part(B.r[io + 4 * c0], B.min[mo + pair_index(c1, c2)], 0.0, part);
               cof = cfma_part(cneg(B.r[io + 4 * c1]), B.min[mo + pair_index(c0, c2)], cof, part);
               cof = cfma_part(B.r[io + 4 * c2], B.min[mo + pair_index(c0, c1)], cof, part);
-              if ((i4 + j4) & 1) cof = -cof;
+              cof = flip_sign(cof, (i4 + j4) & 1);
               st_part(&B.g1[at], part, cof);
-              const double rd = (part ? -det.y : det.x) / (det.x * det.x + det.y * det.y);
+              const double rd = flip_sign(part ? det.y : det.x, part) / (det.x * det.x + det.y * det.y);
               const cplx rdet = mk(__shfl_sync(0xffffffffu, rd, 0), __shfl_sync(0xffffffffu, rd, 16));
               __syncwarp();
               st_part(&B.w[j4 + 4 * i4], part, cfma_part(B.g1[at], rdet, 0.0, part));
