@@ -150,6 +150,21 @@ __device__ __forceinline__ bool poll_col(const cplx* src, cplx* dst, int k0, int
   return true;
 }
 
+// two published words to dst, by a whole warp
+__device__ __forceinline__ bool poll_pair(const cplx* src, cplx* dst) {
+  const long long t0 = clock64();
+  const int w = threadIdx.x & 1;
+  for (;;) {
+    unsigned long long x, y;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(src + w) : "memory");
+    if (__all_sync(0xffffffffu, x != LA_EMPTY && y != LA_EMPTY)) {
+      if ((threadIdx.x & 31) < 2) dst[w] = mk(__longlong_as_double((long long)x), __longlong_as_double((long long)y));
+      return true;
+    }
+    if (__any_sync(0xffffffffu, clock64() - t0 > (4LL << 30))) return false;
+  }
+}
+
 // own rows k >= k0 (k % LT == threadIdx.x) of a column whose words this thread
 // has seen published (or published itself), asynchronously
 __device__ __forceinline__ void fetch_col(const cplx* src, cplx* dst, int k0, int m) {
@@ -190,6 +205,62 @@ __device__ __forceinline__ void cta_sum4(double& a, double& b, double& c, double
   half ^= 1;
 }
 
+// The sum of v over the warp, to every lane, as 58-bit integers in units of
+// 2^-57 of the largest, each rounded to the nearest: errors of 0.36e-16 of sum
+// |v| rms over a wide range of magnitudes, 0.74e-16 for a tree of FP64
+// additions.  Five levels of a tree cost 140 cycles each, 64 of them the
+// addition; this is four warp-wide integer reductions and some thirty integer
+// instructions, 300 cycles.  A NaN or infinity makes it NaN; a sum below
+// 2^-1022 is 0.
+__device__ __forceinline__ double warp_sum(double v) {
+  const unsigned full = 0xffffffffu;
+  const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
+  const int top = __reduce_max_sync(full, e);
+  unsigned long long f = (((unsigned long long)(unsigned)((hi & 0xfffff) | (e ? 0x100000 : 0))) << 32) | (unsigned)__double2loint(v);
+  f = (((f << 5) >> min(top - e, 63)) + 1) >> 1;
+  const long long g = hi < 0 ? -(long long)f : (long long)f;
+  const unsigned lo = __reduce_add_sync(full, (unsigned)g & 0xffffffu);
+  const unsigned mid = __reduce_add_sync(full, (unsigned)(g >> 24) & 0xffffffu);
+  const int up = __reduce_add_sync(full, (int)(g >> 48));
+  const double t = (double)((long long)lo + ((long long)mid << 24) + ((long long)up << 48));
+  const int ht = __double2hiint(t), et = ((ht >> 20) & 0x7ff) + top - 1079;   // units of 2^(top - 1075 - 4)
+  if (top == 0x7ff) return __hiloint2double(0x7ff80000, 0);
+  if (et <= 0) return 0.0;   // t = 0 too: its exponent field is 0
+  if (et >= 0x7ff) return __hiloint2double((ht & (int)0x80000000) | 0x7ff00000, 0);
+  return __hiloint2double(ht + ((top - 1079) << 20), __double2loint(t));
+}
+// Sums over the CTA in two halves: the warps' shares to `red`, and after a
+// barrier c (sum - beta a) with one real component per lane.
+__device__ __forceinline__ void cta_part2(double a, double b, double (*red)[4]) {
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = a;
+    red[1][threadIdx.x >> 5] = b;
+  }
+}
+__device__ __forceinline__ double cta_total(const double* r) { return (r[0] + r[1]) + (r[2] + r[3]); }
+// component (lane >> 2) & 1 of value (lane >> 3) & (NV - 1): c (sum - beta a)
+template <int NV, bool BETA>
+__device__ __forceinline__ double cta_coef(const double (*red)[4], cplx c, double beta, cplx a) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, im = (lane >> 2) & 1;
+  double r = cta_total(red[(lane >> 2) & (2 * NV - 1)]);
+  if (BETA) r = fma(-beta, im ? a.y : a.x, r);
+  const double o = __shfl_xor_sync(full, r, 4);
+  return fma(flip_sign(c.y, !im), o, c.x * r);
+}
+__device__ __forceinline__ cplx cta_value(double f, int v) {
+  return mk(__shfl_sync(0xffffffffu, f, 8 * v), __shfl_sync(0xffffffffu, f, 8 * v + 4));
+}
+// a sum over the CTA to every thread, one barrier
+__device__ __forceinline__ double cta_sum1(double a, double (*red)[4]) {
+  a = warp_sum(a);
+  if ((threadIdx.x & 31) == 0) red[0][threadIdx.x >> 5] = a;
+  __syncthreads();
+  return cta_total(red[0]);
+}
+
 // power of two as a double, |e| <= 1022
 __device__ __forceinline__ double pow2i(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
 // biased exponent of the larger component
@@ -206,23 +277,49 @@ __device__ __forceinline__ int cta_max(int v, int* red) {
   return v;
 }
 
+// Square root and reciprocal of a normal positive double from the hardware's
+// 32-bit-wide first guess by one step of Householder's third-order iteration
+// (A. S. Householder, The Numerical Treatment of a Single Nonlinear Equation,
+// 1970: x' = x (1 + e/2 + 3 e^2/8) for 1/sqrt(a), e = 1 - a x^2, and x' = x (1
+// + e + e^2) for 1/a, e = 1 - a x), which leaves e^3 < 2^-56 of a guess good to
+// 2^-19, and a Newton correction of the root.  11 FP64 instructions for the two.
+__device__ __forceinline__ double root_pos(double a) {
+  double x;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  const double e = fma(-(a * x), x, 1.0);
+  x = fma(x * e, fma(0.375, e, 0.5), x);
+  const double r = a * x;
+  const double hx = __hiloint2double(__double2hiint(x) - (1 << 20), __double2loint(x));   // x / 2
+  return fma(fma(-r, r, a), hx, r);
+}
+__device__ __forceinline__ double recip_pos(double a) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  const double e = fma(-a, x, 1.0);
+  return fma(x, fma(e, e, e), x);
+}
+
 // zlarfg for the column [alpha; x], ss = sum |x|^2, kept as the vector
 // u = [z; x], z = alpha - beta, that is z times zlarfg's v: then
 // H^H = I + c u u^H with c = 1/(beta z), and tau = -z/beta.  One square root
-// and one division, and two products fewer in a step's chain than with v.
+// and one reciprocal, and two products fewer in a step's chain than with v.
+// n2 = |alpha|^2 + ss in 2^-664 .. 2^530, or ss = 0.
 struct Reflector {
   cplx z, c;
   double beta;
 };
-__device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2) {   // n2 = |alpha|^2 + ss
+__device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2) {
   Reflector h;
   // signs and zeros are looked at as bits: an FP64 comparison costs what a multiplication costs
-  const long long sign = ~__double_as_longlong(alpha.x) & (1ll << 63);
-  h.beta = __longlong_as_double(__double_as_longlong(sqrt(n2)) | sign);
+  const int sign = ~__double2hiint(alpha.x) & (int)0x80000000;
+  const double root = root_pos(n2);   // |beta|
+  h.beta = __hiloint2double(__double2hiint(root) | sign, __double2loint(root));
   h.z = mk(alpha.x - h.beta, alpha.y);
-  const double den = h.beta * fma(h.z.x, h.z.x, h.z.y * h.z.y);
-  const double r = flip_sign((threadIdx.x & 1) ? h.z.y : h.z.x, threadIdx.x & 1) / den;   // both components in one division
-  h.c = mk(__shfl_sync(0xffffffffu, r, 0), __shfl_sync(0xffffffffu, r, 1));
+  // 1 / (|beta| |z|^2); c = conj(z) / (beta |z|^2)
+  const double r = recip_pos(root * fma(h.z.x, h.z.x, h.z.y * h.z.y));
+  const bool im = threadIdx.x & 1;   // a component per lane
+  const double q = flip_sign((im ? h.z.y : h.z.x) * r, im != (sign != 0));
+  h.c = mk(__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1));
   if (__double_as_longlong(ss) == 0 && (__double_as_longlong(alpha.y) << 1) == 0) {   // nothing below the diagonal: H = I
     h.z = h.c = mk(0.0);
     h.beta = alpha.x;
@@ -239,11 +336,15 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
 // ln det Q = sum over the reflectors of ln det(I - tau v v^H)
 // = ln(-z / conj(z)) (a phase; 0 for z = 0).
 //
-// What is published is the raw column (rows >= i after the reflectors before
-// it), so its norm is off the critical path: every CTA forms it beside its
-// own dot product, and the chain of a step is one poll, one reduction, a
-// square root, a division and the update of the next column, which its CTA
-// publishes before it turns to its others.  Q's columns need only reflectors
+// What is published is the raw column x (rows >= i after the reflectors
+// before it), and by its CTA alone, as soon as it has the norm, beta and c.
+// The others form x^H a of their next column meanwhile: with u = x - beta e_i,
+// u^H a = x^H a - beta a_i, so the reflector is not needed before the last
+// three instructions of the coefficient, and the chain of a step is two
+// overlapping halves of one column's passage.  The next column comes first
+// and is published row by row.  (Every CTA with the norm and reflector of its
+// own, 2 of 6 multiply-adds a row and 2.1k cycles of root and division in the
+// chain: 875 us at 288 x 144, 1.35 ms at 392 x 196; now 733 us and 1.16 ms.)  Q's columns need only reflectors
 // that their CTA has already seen, so their formation starts without waiting
 // for the rest.  Bound by that chain (n steps) and, in a step, by the FP64
 // pipe.  A column whose entries pass 2^+-256 is held times a power of two
@@ -251,14 +352,18 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
 // norm is taken, as LAPACK's dznrm2 avoids overflow (the graded
 // finite-temperature strings pass 1e154).
 //
+// Rows 0 .. QR_SELF - 1 of a later column are not published; they take
+// QR_COPIES copies of {c, (beta, up)}, so that not every CTA polls one sector.
+//
 // dynamic shared memory: nst columns of the ring, z and c of n reflectors, the local columns' exponents, the local columns if `in_smem`
 // (else they stay in A).
+constexpr int QR_COPIES = 4, QR_SELF = 2 * QR_COPIES;
 __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d, cplx* Rout, cplx* lndet, cplx* pub,
                                                  int in_smem, int nst, int* err) {
   extern __shared__ cplx qr_dyn[];
   __shared__ double red[2][4][4];
   __shared__ int redi[4];
-  __shared__ cplx s_al[2], s_aj[2][2];
+  __shared__ cplx s_al[2], s_aj[2], s_sc[2][2];
   __shared__ int s_fail;
   const int tid = threadIdx.x, b = blockIdx.x, G = gridDim.x;
   const int nl = (n - b + G - 1) / G;   // local columns b, b + G, ...
@@ -293,81 +398,115 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
   for (int i = 0; i < n; ++i) {
     const bool own = i == jown;
     const int l0 = own ? li + 1 : li;   // first local column right of i
-    cplx* x = xs;
-    if (own) {
-      for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) x[k] = col(li)[k];
-    } else if (!poll_col(pub + (size_t)m * i, x, i, m)) {
-      s_fail = 1;
-    }
+    cplx* x = own ? col(li) : xs;
+    if (!own && !poll_col(pub + (size_t)m * i, x, i, m)) s_fail = 1;
     const bool row_i = tid == (i & (LT - 1));
     cplx* c0 = l0 < nl ? col(l0) : nullptr;
-    double ss = 0.0, zero = 0.0;
-    cplx w = mk(0.0);
-    for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) {
-      const cplx v = x[k];
-      ss = fma(v.x, v.x, fma(v.y, v.y, ss));
-      if (c0) w = cfma(cconj(v), c0[k], w);
-    }
-    const int h0 = half;
-    if (row_i) {
-      s_al[h0] = x[i];
-      if (c0) s_aj[h0][0] = c0[i];
-    }
-    cta_sum4(w.x, w.y, ss, zero, red, half);
-    if (s_fail) {
-      if (tid == 0) atomicExch(err, PQMC_ERR_TIMEOUT);
-      return;
-    }
-    const cplx alpha = s_al[h0], aj0 = c0 ? s_aj[h0][0] : mk(0.0);
-    Reflector h;
-    double up_x = 1.0, beta_x;
-    const double n2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
-    if (__double2hiint(n2) < (1023 - 664) << 20) {   // below 2^-664 squares may have vanished: scale up
-      int e = 0;
-      for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) e = max(e, top_exp(x[k]));
-      e = cta_max(e, redi);
-      const int up = e ? min(1023 - e, 1000) : 1000;
-      up_x = pow2i(up);
-      double s2 = 0.0, z1 = 0.0;
-      w = mk(0.0);
+    // its CTA forms the reflector, and every CTA where the published column has no free rows for it
+    const bool self = own || i < QR_SELF;
+    cplx alpha = mk(0.0), c = mk(0.0);
+    double beta = 0.0, up_x = 1.0, beta_x = 0.0;
+    if (self) {
+      double ss = 0.0;
       for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) {
-        const cplx v = cscale(x[k], up_x);
-        x[k] = v;
-        s2 += cabs2(v);
-        if (c0) w = cfma(cconj(v), c0[k], w);
+        const cplx v = x[k];
+        ss = fma(v.x, v.x, fma(v.y, v.y, ss));
       }
-      cta_sum4(w.x, w.y, s2, z1, red, half);
-      const cplx al = cscale(alpha, up_x);
-      h = reflector(al, s2, s2 + cabs2(al));
-      beta_x = h.beta * pow2i(-up);
-    } else {
-      h = reflector(alpha, ss, n2);
-      beta_x = h.beta;
+      const int h0 = half;
+      half ^= 1;
+      if (row_i) s_al[h0] = x[i];
+      ss = cta_sum1(ss, red[h0]);
+      if (s_fail) {
+        if (tid == 0) atomicExch(err, PQMC_ERR_TIMEOUT);
+        return;
+      }
+      alpha = s_al[h0];
+      double n2 = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
+      int up = 0;
+      if (__double2hiint(n2) < (1023 - 664) << 20) {   // below 2^-664 squares may have vanished: scale up
+        int e = 0;
+        for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) e = max(e, top_exp(x[k]));
+        e = cta_max(e, redi);
+        up = e ? min(1023 - e, 1000) : 1000;
+        up_x = pow2i(up);
+        ss = 0.0;
+        for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
+          const cplx v = cscale(x[k], up_x);
+          x[k] = v;
+          if (k > i) ss += cabs2(v);
+        }
+        ss = cta_sum1(ss, red[half]);
+        half ^= 1;
+        alpha = cscale(alpha, up_x);
+        n2 = ss + cabs2(alpha);
+      }
+      const Reflector h = reflector(alpha, ss, n2);
+      c = h.c;
+      beta = h.beta;
+      beta_x = beta * pow2i(-up);
+      if (own && i >= QR_SELF && tid < 2 * QR_COPIES) publish(pub + (size_t)m * i + tid, tid & 1 ? mk(beta, up_x) : c);
     }
-    if (tid == 0) {
-      s_z[i] = h.z;
-      s_c[i] = h.c;
+    cplx f = mk(0.0);
+    if (c0) {
+      cplx w = mk(0.0);
+      for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) w = cfma(cconj(x[k]), c0[k], w);
+      int h0 = half;
+      half ^= 1;
+      if (row_i) {
+        if (!self) s_al[h0] = x[i];
+        s_aj[h0] = c0[i];
+      }
+      cta_part2(w.x, w.y, red[h0]);
+      if (!self && tid < 32 && !poll_pair(pub + (size_t)m * i + 2 * (b & (QR_COPIES - 1)), s_sc[h0])) s_fail = 1;
+      __syncthreads();
+      if (s_fail) {
+        if (tid == 0) atomicExch(err, PQMC_ERR_TIMEOUT);
+        return;
+      }
+      const cplx aj = s_aj[h0];
+      if (!self) {
+        alpha = s_al[h0];
+        c = s_sc[h0][0];
+        beta = s_sc[h0][1].x;
+        up_x = s_sc[h0][1].y;
+        if (__double2hiint(up_x) != 0x3ff00000) {   // not 1: the dot product of the scaled column
+          w = mk(0.0);
+          for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
+            const cplx v = cscale(x[k], up_x);
+            x[k] = v;
+            w = cfma(cconj(v), c0[k], w);
+          }
+          alpha = cscale(alpha, up_x);
+          h0 = half;
+          half ^= 1;
+          cta_part2(w.x, w.y, red[h0]);
+          __syncthreads();
+        }
+      }
+      f = cta_value(cta_coef<1, true>(red[h0], c, beta, aj), 0);   // c u^H a
+    }
+    if (row_i) {
+      const cplx z = mk(alpha.x - beta, alpha.y);
+      x[i] = z;   // u
+      s_z[i] = z;
+      s_c[i] = c;
       s_up[i] = up_x;
     }
-    if (row_i) x[i] = h.z;   // u
     // H_i^H on the local columns right of i, the next column first
     for (int l = l0; l < nl; ++l) {
-      cplx* c = col(l);
-      cplx aj = aj0;
+      cplx* cl = col(l);
       if (l != l0) {
-        w = mk(0.0);
-        double z1 = 0.0, z2 = 0.0;
-        for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) w = cfma(cconj(x[k]), c[k], w);
-        const int h1 = half;
-        if (row_i) s_aj[h1][0] = c[i];
-        cta_sum4(w.x, w.y, z1, z2, red, half);
-        aj = s_aj[h1][0];
+        cplx w = mk(0.0);
+        for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) w = cfma(cconj(x[k]), cl[k], w);
+        cta_part2(w.x, w.y, red[half]);
+        __syncthreads();
+        f = cta_value(cta_coef<1, false>(red[half], c, 0.0, mk(0.0)), 0);
+        half ^= 1;
       }
-      const cplx f = cmul(h.c, cfma(cconj(h.z), aj, w));   // c u^H a
       const bool next = l == l0 && (own ? jown + G : jown) == i + 1;
       for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
-        const cplx v = cfma(x[k], f, c[k]);
-        c[k] = v;
+        const cplx v = cfma(x[k], f, cl[k]);
+        cl[k] = v;
         if (next && k > i) publish(pub + (size_t)m * (i + 1) + k, v);
       }
     }
@@ -418,25 +557,28 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
       cplx* x = xs + (size_t)(i & ring) * m;
       if (up_x != 1.0)
         for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) x[k] = cscale(x[k], up_x);
+      if (row_i) x[i] = z;   // u
       for (int l = ls; l < nl; l += 2) {
         cplx* c0 = col(l);
         cplx* c1 = l + 1 < nl ? col(l + 1) : nullptr;
-        cplx w0 = mk(0.0), w1 = mk(0.0);
-        for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) {
+        cplx w0 = mk(0.0), w1 = mk(0.0), f1 = mk(0.0);
+        for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
           const cplx v = cconj(x[k]);
           w0 = cfma(v, c0[k], w0);
           if (c1) w1 = cfma(v, c1[k], w1);
         }
-        const int h0 = half;
-        if (row_i) {
-          s_aj[h0][0] = c0[i];
-          if (c1) s_aj[h0][1] = c1[i];
+        cta_part2(w0.x, w0.y, red[half]);
+        if (c1) cta_part2(w1.x, w1.y, red[half] + 2);
+        __syncthreads();
+        cplx f0;
+        if (c1) {
+          const double f = cta_coef<2, false>(red[half], cc, 0.0, mk(0.0));
+          f0 = cta_value(f, 0);
+          f1 = cta_value(f, 1);
+        } else {
+          f0 = cta_value(cta_coef<1, false>(red[half], cc, 0.0, mk(0.0)), 0);
         }
-        cta_sum4(w0.x, w0.y, w1.x, w1.y, red, half);
-        const cplx q0 = s_aj[h0][0], q1 = c1 ? s_aj[h0][1] : mk(0.0);
-        const cplx f0 = cmul(cc, cfma(cconj(z), q0, w0));
-        const cplx f1 = cmul(cc, cfma(cconj(z), q1, w1));
-        if (row_i) x[i] = z;   // u
+        half ^= 1;
         for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
           c0[k] = cfma(x[k], f0, c0[k]);
           if (c1) c1[k] = cfma(x[k], f1, c1[k]);
@@ -449,8 +591,8 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
     if (i == jown) {   // H_i e_i
       cplx* c = col(li--);
       jown -= G;
-      const cplx t = cmul(cc, cconj(z)), g = cscale(t, up_x);
-      for (int k = tid; k < m; k += LT) c[k] = k > i ? cmul(g, c[k]) : k == i ? cfma(t, z, mk(1.0)) : mk(0.0);
+      const cplx t = cmul(cc, cconj(z));   // the column has its power of two already
+      for (int k = tid; k < m; k += LT) c[k] = k > i ? cmul(t, c[k]) : k == i ? cfma(t, z, mk(1.0)) : mk(0.0);
     }
   }
   if (in_smem)
