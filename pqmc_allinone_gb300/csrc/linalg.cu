@@ -6,6 +6,7 @@
 // GB300 runs FP64 at a small fraction of its FP32 rate, so every routine
 // spreads its work over all SMs: the factorisations are cooperative kernels
 // that pipeline over columns, the products are tiled GEMMs.
+#include <type_traits>
 #include "linalg.cuh"
 
 namespace pqmc {
@@ -328,6 +329,176 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
 }
 
 // ---------------------------------------------------------------------------
+// Columns j = b, b + G, ... of Q = H_0 ... H_(n-1), H_i = I + c_i u_i u_i^H, by
+// the triangular factor of their product: H_0 ... H_(n-1) = I + U T U^H with
+// T^-1 = diag(1/c_i) - (strictly upper part of U^H U) (T. Joffrain, T. M. Low,
+// E. S. Quintana-Orti, R. van de Geijn, F. G. Van Zee, Accumulating Householder
+// transformations, revisited, ACM TOMS 32, 2006).  So column j is
+// e_j + U y, T^-1 y = U^H e_j, in three steps: the products c_i u_i^H u_j,
+// published for the others; the triangular system, one unknown a step; and U y.
+//
+// Applying the reflectors to the column one after the other is the same number
+// of multiply-adds, but each waits for a sum over the CTA: 4.4k cycles a
+// reflector at 288 rows.  Here only the triangular system is a chain, of 1.1k
+// cycles a step, and FP64 issue and the loops' own instructions bound the rest
+// (76k, 153k and 159k cycles for the products, the system and U y of the last
+// column at 288 x 144; the whole factorisation takes 617 us with this and 733
+// without, 1054 and 1158 at 392 x 196).  One or two columns per CTA.  `gs` (n x n, column k holds
+// the products of column k) starts out LA_EMPTY like `pub`.
+__device__ __forceinline__ void form_q_ut(int m, int n, int b, int G, int nl, cplx* cols, cplx* pub, cplx* xs,
+                                          const cplx* s_z, const cplx* s_c, const double* s_up, cplx* s_y, int* s_fail) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  cplx* gs = pub + (size_t)m * n;
+  auto one = [](double up) { return __double2hiint(up) == 0x3ff00000; };
+  for (int l = 0; l < nl; ++l)
+    if (const int j = b + l * G; tid == (j & (LT - 1))) cols[(size_t)l * m + j] = s_z[j];   // u_j
+  __syncthreads();
+  // c_i u_i^H u_j: a lane per i, a quarter of the rows per warp
+  for (int l = 0; l < nl; ++l) {
+    const int j = b + l * G, len = (m - j + 3) / 4, k0 = j + warp * len, k1 = min(m, k0 + len);
+    const cplx* u = cols + (size_t)l * m;
+    for (int i0 = 0; i0 < j; i0 += 32) {
+      const int i = i0 + lane;
+      const double2* p = reinterpret_cast<const double2*>(pub) + (size_t)m * min(i, j - 1);
+      constexpr int AHEAD = 8;
+      double2 v[AHEAD];
+#pragma unroll
+      for (int q = 0; q < AHEAD; ++q) v[q] = k0 + q < k1 ? p[k0 + q] : make_double2(0.0, 0.0);
+      cplx acc = mk(0.0);
+      for (int k = k0; k < k1; k += AHEAD)
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q)
+          if (k + q < k1) {
+            const cplx x = mk(v[q].x, -v[q].y);
+            v[q] = k + q + AHEAD < k1 ? p[k + q + AHEAD] : make_double2(0.0, 0.0);
+            acc = cfma(x, u[k + q], acc);
+          }
+      if (i < j) xs[(size_t)warp * n + i] = acc;
+    }
+    __syncthreads();
+    for (int i = tid; i < j; i += LT) {
+      cplx g = cadd(cadd(xs[i], xs[(size_t)n + i]), cadd(xs[2 * (size_t)n + i], xs[3 * (size_t)n + i]));
+      if (!one(s_up[i])) g = cscale(g, s_up[i]);
+      publish(gs + (size_t)n * j + i, cmul(cconj(s_c[i]), g));
+    }
+    __syncthreads();   // the shares are read
+  }
+  // c_i (U^H e_j)_i, then from the last unknown to the first
+  const int jlast = b + (nl - 1) * G;
+  for (int l = 0; l < nl; ++l) {
+    const int j = b + l * G;
+    for (int i = tid; i <= j; i += LT) {
+      cplx v = i < j ? pub[(size_t)m * i + j] : s_z[j];
+      if (i < j && !one(s_up[i])) v = cscale(v, s_up[i]);
+      s_y[(size_t)l * n + i] = cmul(cconj(s_c[i]), cconj(v));
+    }
+  }
+  auto fetch_g = [&](int k) {
+    if (k > 0)
+      for (int i = tid; i < k; i += LT)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(xs + (size_t)(k & 3) * m + i)),
+                     "l"(gs + (size_t)n * k + i)
+                     : "memory");
+    fetch_commit();
+  };
+  for (int q = 0; q < 4; ++q) fetch_g(jlast - q);
+  bool ok = true;
+  const long long t0 = clock64();
+  auto product = [&](int k, int i) {   // c_i u_i^H u_k
+    cplx v = xs[(size_t)(k & 3) * m + i];
+    while ((unsigned long long)__double_as_longlong(v.x) == LA_EMPTY || (unsigned long long)__double_as_longlong(v.y) == LA_EMPTY) {
+      if (!ok || clock64() - t0 > (4LL << 30)) {
+        ok = false;
+        break;
+      }
+      unsigned long long x, y;
+      asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(gs + (size_t)n * k + i) : "memory");
+      v = mk(__longlong_as_double((long long)x), __longlong_as_double((long long)y));
+    }
+    return v;
+  };
+  // Two unknowns a step, k and k - 1, every thread forming the second for
+  // itself; the thread that holds it stores it when nobody reads it any more.
+  // The number of columns is a constant of the loop bodies: a multiply-add
+  // that a predicate switches off takes its 64 cycles all the same.
+  cplx late_y[2];
+  int late_k = -1, late_l = 0;
+  auto store_late = [&]() {
+    if (late_k >= 0)
+      for (int l = late_l; l < nl; ++l) s_y[(size_t)l * n + late_k] = late_y[l - late_l];
+    late_k = -1;
+  };
+  auto step = [&](auto cols_on, int k, int la) {
+    constexpr int NL = decltype(cols_on)::value;
+    const cplx d = product(k, k - 1);
+    cplx* yb = s_y + (size_t)la * n;
+    cplx y0[NL], y1[NL];
+#pragma unroll
+    for (int q = 0; q < NL; ++q) {
+      y0[q] = b + (la + q) * G >= k ? yb[q * n + k] : mk(0.0);
+      y1[q] = cfma(d, y0[q], yb[q * n + k - 1]);
+    }
+    for (int i = tid; i < k - 1; i += LT) {
+      const cplx v0 = product(k, i), v1 = product(k - 1, i);
+#pragma unroll
+      for (int q = 0; q < NL; ++q) yb[q * n + i] = cfma(v1, y1[q], cfma(v0, y0[q], yb[q * n + i]));
+    }
+    if (tid == ((k - 1) & (LT - 1))) {
+      late_k = k - 1;
+      late_l = la;
+#pragma unroll
+      for (int q = 0; q < NL; ++q) late_y[q] = y1[q];
+    }
+  };
+  for (int k = jlast; k > 0; k -= 2) {
+    fetch_wait<2>();
+    __syncthreads();   // unknowns k and k - 1 but for the product of the two
+    store_late();
+    const int la = nl > 1 && b < k - 1 ? 1 : 0;   // columns that have unknown k - 1
+    if (nl - la == 2) step(std::integral_constant<int, 2>(), k, la);
+    else step(std::integral_constant<int, 1>(), k, la);
+    fetch_g(k - 4);
+    fetch_g(k - 5);
+  }
+  __syncthreads();
+  store_late();
+  fetch_wait<0>();
+  if (!ok) *s_fail = 1;
+  __syncthreads();
+  // e_j + U y, own rows
+  for (int l = 0; l < nl; ++l)
+    for (int k = tid; k < m; k += LT) cols[(size_t)l * m + k] = mk(k == b + l * G ? 1.0 : 0.0);
+  for (int q = 0; q < 3; ++q) {
+    if (q <= jlast) fetch_col(pub + (size_t)m * q, xs + (size_t)q * m, q, m);
+    fetch_commit();
+  }
+  for (int i = 0; i <= jlast; ++i) {
+    fetch_wait<2>();
+    cplx* x = xs + (size_t)(i & 3) * m;
+    const int k0 = i + ((tid - i) & (LT - 1));
+    if (!one(s_up[i]))
+      for (int k = k0; k < m; k += LT) x[k] = cscale(x[k], s_up[i]);
+    if (tid == (i & (LT - 1))) x[i] = s_z[i];
+    if (nl == 2 && i <= b) {
+      const cplx ya = s_y[i], yb = s_y[(size_t)n + i];
+      for (int k = k0; k < m; k += LT) {
+        const cplx v = x[k];
+        cols[k] = cfma(v, ya, cols[k]);
+        cols[(size_t)m + k] = cfma(v, yb, cols[(size_t)m + k]);
+      }
+    } else {
+      const cplx y = s_y[(size_t)(nl - 1) * n + i];
+      cplx* c = cols + (size_t)(nl - 1) * m;
+      for (int k = k0; k < m; k += LT) c[k] = cfma(x[k], y, c[k]);
+    }
+    if (i + 3 <= jlast) fetch_col(pub + (size_t)m * (i + 3), xs + (size_t)((i + 3) & 3) * m, i + 3, m);
+    fetch_commit();
+  }
+  fetch_wait<0>();
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
 // Householder QR in place with Q formed (zgeqr2 + zung2r).  A is m x n
 // (lda = m), m >= n; d receives diag(R) (real in the LAPACK convention).
 // Matches zqdr (src/mod_matrixlib.f90:323-334) with the unit-diagonal R
@@ -344,7 +515,7 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
 // overlapping halves of one column's passage.  The next column comes first
 // and is published row by row.  (Every CTA with the norm and reflector of its
 // own, 2 of 6 multiply-adds a row and 2.1k cycles of root and division in the
-// chain: 875 us at 288 x 144, 1.35 ms at 392 x 196; now 733 us and 1.16 ms.)  Q's columns need only reflectors
+// chain: 875 us at 288 x 144 and 1.35 ms at 392 x 196, 733 us and 1.16 ms so.)  Q's columns need only reflectors
 // that their CTA has already seen, so their formation starts without waiting
 // for the rest.  Bound by that chain (n steps) and, in a step, by the FP64
 // pipe.  A column whose entries pass 2^+-256 is held times a power of two
@@ -359,7 +530,7 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
 // (else they stay in A).
 constexpr int QR_COPIES = 4, QR_SELF = 2 * QR_COPIES;
 __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d, cplx* Rout, cplx* lndet, cplx* pub,
-                                                 int in_smem, int nst, int* err) {
+                                                 int in_smem, int nst, int ut, int* err) {
   extern __shared__ cplx qr_dyn[];
   __shared__ double red[2][4][4];
   __shared__ int redi[4];
@@ -372,7 +543,8 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
   cplx* s_c = s_z + n;
   double* s_up = reinterpret_cast<double*>(s_c + n);   // power of two on x (1 but for vanishing remainders)
   int* s_exp = reinterpret_cast<int*>(s_up + 2 * ((n + 1) / 2));
-  cplx* cols = s_c + n + (n + 1) / 2 + (nl + 3) / 4;
+  cplx* s_y = s_c + n + (n + 1) / 2 + (nl + 3) / 4;   // ut: [nl][n]
+  cplx* cols = s_y + (ut ? nl * n : 0);
   auto col = [&](int l) { return in_smem ? cols + (size_t)l * m : A + (size_t)m * (b + (size_t)l * G); };
   int half = 0;
   if (tid == 0) s_fail = 0;
@@ -536,6 +708,18 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
     cta_sum4(ph, z1, z2, z3, red, half);
     if (tid == 0) lndet[0] = mk(0.0, ph);
   }
+  if (ut) {
+    form_q_ut(m, n, b, G, nl, cols, pub, xs, s_z, s_c, s_up, s_y, &s_fail);
+    if (s_fail) {   // read after the barrier that ends form_q_ut
+      if (tid == 0) atomicExch(err, PQMC_ERR_TIMEOUT);
+      return;
+    }
+    for (int l = 0; l < nl; ++l) {
+      cplx* dst = A + (size_t)m * (b + (size_t)l * G);
+      for (int k = tid; k < m; k += LT) dst[k] = col(l)[k];
+    }
+    return;
+  }
   // zung2r: column j of Q = H_1 ... H_j e_j, the local columns together; the
   // published columns come back through the ring, nst - 1 steps ahead
   const int jlast = b + (nl - 1) * G, ring = nst - 1;   // nst is 2 or 4
@@ -558,31 +742,31 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
       if (up_x != 1.0)
         for (int k = i + 1 + ((tid - i - 1) & (LT - 1)); k < m; k += LT) x[k] = cscale(x[k], up_x);
       if (row_i) x[i] = z;   // u
-      for (int l = ls; l < nl; l += 2) {
+      auto apply = [&](auto cols_on, int l) {
+        constexpr bool two = decltype(cols_on)::value == 2;
         cplx* c0 = col(l);
-        cplx* c1 = l + 1 < nl ? col(l + 1) : nullptr;
-        cplx w0 = mk(0.0), w1 = mk(0.0), f1 = mk(0.0);
+        cplx* c1 = two ? col(l + 1) : c0;
+        cplx w0 = mk(0.0), w1 = mk(0.0), f0, f1 = mk(0.0);
         for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
           const cplx v = cconj(x[k]);
           w0 = cfma(v, c0[k], w0);
-          if (c1) w1 = cfma(v, c1[k], w1);
+          if (two) w1 = cfma(v, c1[k], w1);
         }
         cta_part2(w0.x, w0.y, red[half]);
-        if (c1) cta_part2(w1.x, w1.y, red[half] + 2);
+        if (two) cta_part2(w1.x, w1.y, red[half] + 2);
         __syncthreads();
-        cplx f0;
-        if (c1) {
-          const double f = cta_coef<2, false>(red[half], cc, 0.0, mk(0.0));
-          f0 = cta_value(f, 0);
-          f1 = cta_value(f, 1);
-        } else {
-          f0 = cta_value(cta_coef<1, false>(red[half], cc, 0.0, mk(0.0)), 0);
-        }
+        const double f = cta_coef<two ? 2 : 1, false>(red[half], cc, 0.0, mk(0.0));
+        f0 = cta_value(f, 0);
+        if (two) f1 = cta_value(f, 1);
         half ^= 1;
         for (int k = i + ((tid - i) & (LT - 1)); k < m; k += LT) {
           c0[k] = cfma(x[k], f0, c0[k]);
-          if (c1) c1[k] = cfma(x[k], f1, c1[k]);
+          if (two) c1[k] = cfma(x[k], f1, c1[k]);
         }
+      };
+      for (int l = ls; l < nl; l += 2) {
+        if (l + 1 < nl) apply(std::integral_constant<int, 2>(), l);
+        else apply(std::integral_constant<int, 1>(), l);
       }
       const int in = i - (nst - 1);
       if (in >= 0) fetch_col(pub + (size_t)m * in, xs + (size_t)(in & ring) * m, in, m);
@@ -840,9 +1024,14 @@ int house_qr(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* work, int* er
 
 int house_qr_r(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* R, cplx* lndet, cplx* work, int* err) {
   PipeShape q;
-  PQMC_TRY(pipe_shape((const void*)k_house_qr, n, m, [&](int nl, int) { return (size_t)2 * n + (n + 1) / 2 + (nl + 3) / 4; }, &q));
-  PQMC_CUDA(cudaMemsetAsync(work, 0xff, sizeof(cplx) * (size_t)m * n, s));
-  void* args[] = {&m, &n, &A, &d, &R, &lndet, &work, &q.in_smem, &q.nst, &err};
+  // Q by the triangular factor where the work matrix (m x m) has room for its
+  // products behind the published columns (a square A has none)
+  const bool room = (size_t)m * (m - n) >= (size_t)n * n;
+  PQMC_TRY(pipe_shape((const void*)k_house_qr, n, m,
+                      [&](int nl, int in) { return (size_t)2 * n + (n + 1) / 2 + (nl + 3) / 4 + (room && in ? (size_t)nl * n : 0); }, &q));
+  int ut = room && q.in_smem && q.nst == 4 && n <= 2 * q.grid;
+  PQMC_CUDA(cudaMemsetAsync(work, 0xff, sizeof(cplx) * ((size_t)m * n + (ut ? (size_t)n * n : 0)), s));
+  void* args[] = {&m, &n, &A, &d, &R, &lndet, &work, &q.in_smem, &q.nst, &ut, &err};
   PQMC_CUDA(cudaLaunchCooperativeKernel((const void*)k_house_qr, q.grid, LT, args, q.smem, s));
   PQMC_LAUNCHED();
   return PQMC_OK;
