@@ -3,7 +3,7 @@
 //
 // Draws:   every CTA walks the family's ran2 stream (each proposal consumes
 //          a fixed number of draws, :84 and :117) and keeps its own part.
-// Phase 1: every CTA prepares some plaquettes in parallel, two warps each:
+// Phase 1: every CTA prepares plaquettes blockIdx, blockIdx + CTAs, .., two warps each:
 //          the phonon action difference and threshold (:203-228) on one, the
 //          new propagators and Delta = expKV_inv(old) expKV(new) - I
 //          (:230-245) on the other.
@@ -24,7 +24,7 @@
 // from the twelve 2x2 minors of the row pairs, and no separate FP32 screen.
 // The other CTAs need Ns^2 dim complex multiply-adds per accepted move, 4.3 us
 // of the whole chip at Ns = 392 (8.6 us a move with the hand-over).  A family
-// step at 4x4 with Gaussian proposals takes 49 us (413 with one worker CTA
+// step at 4x4 with Gaussian proposals takes 43 us (413 with one worker CTA
 // and 16 complex lanes), at 14x14 0.53 ms (0.91).
 #include <cooperative_groups.h>
 #include "chain.cuh"
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
   extern __shared__ cplx upd_dyn[];   // G(:,S) of the move being applied
   const int ns = M.ns, dim = DIM ? DIM : M.pf_dim[pf], npla = M.pf_npla[pf], pd = M.pdim;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ppb = blockDim.x >> 6;   // plaquettes a CTA prepares at a time
+  const int ppb = blockDim.x >> 6;   // plaquettes a CTA prepares at a time, at most
   const unsigned seq0 = ld_acquire(&sync->seq), arr0 = ld_acquire(&sync->arrived), done0 = ld_acquire(&sync->done);
 
   // ---- the family's ran2 stream: every CTA draws all of it (a chain of
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
     rng.iran = sc->rng[0]; rng.jran = sc->rng[1]; rng.kran = sc->rng[2];
     rng.mran = sc->rng[3]; rng.nran = sc->rng[4];
     for (int p = 0; p < npla; ++p) {
-      const bool mine = (p / ppb) % gridDim.x == blockIdx.x;
+      const bool mine = p % gridDim.x == blockIdx.x;
       if (M.proposal_kind == PQMC_PROPOSAL_GAUSSIAN) {
         const float u1 = rng.next(), u2 = rng.next();
         if (mine) {
@@ -213,8 +213,11 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
   // ---- phase 1: proposals of all plaquettes in parallel -------------------
   {
     const bool closed = (M.expkv_kind != PQMC_EXPKV_GENERAL);
-    for (int p0 = blockIdx.x * ppb; p0 < npla; p0 += gridDim.x * ppb) {
-      const int p = p0 + (warp >> 1);
+    // one plaquette per CTA while they last: two warps on SM quarters of their
+    // own (four plaquettes in one CTA: 38.6k cycles of a family's 103k at 4x4;
+    // so 26.9k, nearly all of it the exponentials of one plaquette)
+    for (int p0 = blockIdx.x; p0 < npla; p0 += gridDim.x * ppb) {
+      const int p = p0 + (warp >> 1) * gridDim.x;
       const bool on = p < npla;
       double jump = 0.0, xnew = 0.0;
       int b = 0;
