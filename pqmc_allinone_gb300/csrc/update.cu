@@ -24,7 +24,7 @@
 // from the twelve 2x2 minors of the row pairs, and no separate FP32 screen.
 // The other CTAs need Ns^2 dim complex multiply-adds per accepted move, 4.3 us
 // of the whole chip at Ns = 392 (8.6 us a move with the hand-over).  A family
-// step at 4x4 with Gaussian proposals takes 43 us (413 with one worker CTA
+// step at 4x4 with Gaussian proposals takes 40 us (413 with one worker CTA
 // and 16 complex lanes), at 14x14 0.53 ms (0.91).
 #include <cooperative_groups.h>
 #include "chain.cuh"
@@ -64,6 +64,17 @@ __device__ __forceinline__ double ldg_part(const cplx* p, int c) { return __ldcg
 __device__ __forceinline__ void st_part(cplx* p, int c, double v) { reinterpret_cast<double*>(p)[c] = v; }
 // index of the column pair (a < b) among 01 02 03 12 13 23
 __device__ __forceinline__ int pair_index(int a, int b) { return a * (7 - a) / 2 + b - a - 1; }
+
+// closed_norm by a whole warp: the two moduli, each a hypot, side by side
+__device__ __forceinline__ double closed_norm_warp(const DevModel& M, int pf, double x, int lane) {
+  if (M.expkv_kind != PQMC_EXPKV_EPSOCZ_BLOCK) return closed_norm(M, pf, x);
+  const int pd = M.pdim, k = lane & 1;
+  const cplx vx = cscale(M.v_coe[pf], x);
+  const size_t at = (size_t)pd * pd * pf + k + pd * 2;
+  const double c = cabsd(cadd(cmul(M.k_coe[pf], M.kmat[at]), cmul(vx, M.vmat[at])));
+  const double a = __shfl_sync(0xffffffffu, c, 0), b = __shfl_sync(0xffffffffu, c, 1);
+  return M.delt * sqrt(a * a + b * b);
+}
 
 constexpr int UPD_SPEC = 3;   // proposals CTA 0 evaluates at a time (the fourth SM quarter does the bookkeeping)
 // 4x4 blocks of one proposal, entry (i, j) at i + 4 j
@@ -213,24 +224,30 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
   // ---- phase 1: proposals of all plaquettes in parallel -------------------
   {
     const bool closed = (M.expkv_kind != PQMC_EXPKV_GENERAL);
+    __shared__ double s_jump[8];
     // one plaquette per CTA while they last: two warps on SM quarters of their
-    // own (four plaquettes in one CTA: 38.6k cycles of a family's 103k at 4x4;
-    // so 26.9k, nearly all of it the exponentials of one plaquette)
+    // own (four plaquettes in one CTA: 38.6k cycles of a family's 103k at 4x4; one
+    // and with nothing formed twice 20.5k, the exponentials of one plaquette)
     for (int p0 = blockIdx.x; p0 < npla; p0 += gridDim.x * ppb) {
+      if (p0 != blockIdx.x) __syncthreads();   // s_jump is read
       const int p = p0 + (warp >> 1) * gridDim.x;
       const bool on = p < npla;
       double jump = 0.0, xnew = 0.0;
       int b = 0;
       if (on) {
         b = M.bf[p + M.max_pla * pf];
-        if (M.proposal_kind == PQMC_PROPOSAL_GAUSSIAN) {
-          jump = pqmc_bm_gauss_jump(M.jump, pre[p].xnew, pre[p].dE);   // bit-identical with the oracle
-        } else {
+        // pqmc_bm_gauss_jump's two factors, a warp each (bit-identical with the oracle)
+        if (M.proposal_kind == PQMC_PROPOSAL_GAUSSIAN)
+          s_jump[warp] = warp & 1 ? pqmc_bm_cos2pi(pre[p].dE) : PQMC_BM_SQRT(PQMC_BM_MUL(-2.0, pqmc_bm_log(pre[p].xnew)));
+        else
           jump = M.jump * pre[p].xnew;
-        }
-        xnew = field[b + (size_t)M.n_bf * t] + jump;                // :92
       }
       __syncthreads();   // both warps of a plaquette have read its draws
+      if (on) {
+        if (M.proposal_kind == PQMC_PROPOSAL_GAUSSIAN)
+          jump = PQMC_BM_MUL(M.jump, PQMC_BM_MUL(s_jump[warp & ~1], s_jump[warp | 1]));
+        xnew = field[b + (size_t)M.n_bf * t] + jump;                // :92
+      }
       if (on && (warp & 1)) {
         const double dE = -M.delt * energy_diff(M, field, b, t, jump);  // :87-88
         const double thr = accept_threshold(M, dE, pre[p].r);
@@ -242,7 +259,7 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
       } else if (on) {
         double norm = 0.0, ch = 0.0, sh = 0.0;
         if (closed) {
-          norm = closed_norm(M, pf, xnew);
+          norm = closed_norm_warp(M, pf, xnew, lane);
           ch = cosh(norm);
           sh = sinh(norm);
         } else {
@@ -256,7 +273,8 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
           if (closed) {
             en = closed_entry(M, pf, p, xnew, false, i, j, norm, ch, sh);
             pre[p].enew[lane] = en;
-            pre[p].einv[lane] = closed_entry(M, pf, p, xnew, true, i, j, norm, ch, sh);
+            // the inverse: the off-diagonal blocks with the other sign (entries outside them are 0)
+            pre[p].einv[lane] = i == j || (en.x == 0.0 && en.y == 0.0) ? en : cneg(en);
           } else {
             en = pre[p].enew[lane];
           }
