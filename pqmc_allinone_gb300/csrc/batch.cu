@@ -140,31 +140,42 @@ __global__ void __launch_bounds__(256) k_bprep(const BDesc* D, int pf_first, int
   PlaqPre* pre = d.pre + (size_t)pf * M.max_pla;
   const double* field = d.field;
   const bool closed = (M.expkv_kind != PQMC_EXPKV_GENERAL);
-  // ---- scalars: one plaquette per lane ------------------------------------
-  if (warp == 0 && lane < PREP_PLA && p0 + lane < npla) {
+  // ---- scalars: one plaquette per lane, three warps on SM quarters of their
+  // own: the threshold, the norm with its cosh, the norm with its sinh (one
+  // after the other in one warp 20 us a launch at 8 chains of 72 sites, so 14)
+  const bool on = warp < 3 && lane < PREP_PLA && p0 + lane < npla;
+  double jump = 0.0, xnew = 0.0;
+  int b = 0;
+  if (on) {
     const int p = p0 + lane;
-    const int b = M.bf[p + M.max_pla * pf];
-    double jump;
+    b = M.bf[p + M.max_pla * pf];
     if (M.proposal_kind == PQMC_PROPOSAL_GAUSSIAN) {
       double u1 = pre[p].xnew, u2 = pre[p].dE;
       jump = pqmc_bm_gauss_jump(M.jump, u1, u2);   // bit-identical with the oracle
     } else {
       jump = M.jump * pre[p].xnew;
     }
-    const double xnew = field[b + (size_t)M.n_bf * t] + jump;
-    const double dE = -M.delt * energy_diff(M, field, b, t, jump);
-    pre[p].dE = dE;
-    pre[p].thr = b_threshold(M, dE, pre[p].r);
-    pre[p].xnew = xnew;
-    s_x[lane] = xnew;
-    if (closed) {
-      const double norm = closed_norm(M, pf, xnew);
-      s_norm[lane] = norm;
-      s_ch[lane] = cosh(norm);
-      s_sh[lane] = sinh(norm);
+    xnew = field[b + (size_t)M.n_bf * t] + jump;
+  }
+  __syncthreads();   // the draws are read
+  if (on) {
+    const int p = p0 + lane;
+    if (warp == 0) {
+      const double dE = -M.delt * energy_diff(M, field, b, t, jump);
+      pre[p].dE = dE;
+      pre[p].thr = b_threshold(M, dE, pre[p].r);
+      pre[p].xnew = xnew;
+    } else if (!closed) {
+      dev_get_expkv(M, pf, p, xnew, warp == 2, warp == 2 ? pre[p].einv : pre[p].enew);
     } else {
-      dev_get_expkv(M, pf, p, xnew, false, pre[p].enew);
-      dev_get_expkv(M, pf, p, xnew, true, pre[p].einv);
+      const double norm = closed_norm(M, pf, xnew);
+      if (warp == 1) {
+        s_x[lane] = xnew;
+        s_norm[lane] = norm;
+        s_ch[lane] = cosh(norm);
+      } else {
+        s_sh[lane] = sinh(norm);
+      }
     }
   }
   __syncthreads();
@@ -176,10 +187,11 @@ __global__ void __launch_bounds__(256) k_bprep(const BDesc* D, int pf_first, int
   cplx en = mk(0.0);
   if (act) {
     if (closed) {
-      const double xnew = s_x[q], norm = s_norm[q], ch = s_ch[q], sh = s_sh[q];
-      en = closed_entry(M, pf, p, xnew, false, i, j, norm, ch, sh);
+      const double xq = s_x[q], norm = s_norm[q], ch = s_ch[q], sh = s_sh[q];
+      en = closed_entry(M, pf, p, xq, false, i, j, norm, ch, sh);
       pre[p].enew[sl] = en;
-      pre[p].einv[sl] = closed_entry(M, pf, p, xnew, true, i, j, norm, ch, sh);
+      // the inverse: the off-diagonal blocks with the other sign (entries outside them are 0)
+      pre[p].einv[sl] = i == j || (en.x == 0.0 && en.y == 0.0) ? en : cneg(en);
     } else {
       en = pre[p].enew[sl];
     }
