@@ -278,28 +278,6 @@ __device__ __forceinline__ int cta_max(int v, int* red) {
   return v;
 }
 
-// Square root and reciprocal of a normal positive double from the hardware's
-// 32-bit-wide first guess by one step of Householder's third-order iteration
-// (A. S. Householder, The Numerical Treatment of a Single Nonlinear Equation,
-// 1970: x' = x (1 + e/2 + 3 e^2/8) for 1/sqrt(a), e = 1 - a x^2, and x' = x (1
-// + e + e^2) for 1/a, e = 1 - a x), which leaves e^3 < 2^-56 of a guess good to
-// 2^-19, and a Newton correction of the root.  11 FP64 instructions for the two.
-__device__ __forceinline__ double root_pos(double a) {
-  double x;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
-  const double e = fma(-(a * x), x, 1.0);
-  x = fma(x * e, fma(0.375, e, 0.5), x);
-  const double r = a * x;
-  const double hx = __hiloint2double(__double2hiint(x) - (1 << 20), __double2loint(x));   // x / 2
-  return fma(fma(-r, r, a), hx, r);
-}
-__device__ __forceinline__ double recip_pos(double a) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
-  const double e = fma(-a, x, 1.0);
-  return fma(x, fma(e, e, e), x);
-}
-
 // zlarfg for the column [alpha; x], ss = sum |x|^2, kept as the vector
 // u = [z; x], z = alpha - beta, that is z times zlarfg's v: then
 // H^H = I + c u u^H with c = 1/(beta z), and tau = -z/beta.  One square root
@@ -313,11 +291,11 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
   Reflector h;
   // signs and zeros are looked at as bits: an FP64 comparison costs what a multiplication costs
   const int sign = ~__double2hiint(alpha.x) & (int)0x80000000;
-  const double root = root_pos(n2);   // |beta|
+  const double root = sqrt(n2);   // |beta|
   h.beta = __hiloint2double(__double2hiint(root) | sign, __double2loint(root));
   h.z = mk(alpha.x - h.beta, alpha.y);
   // 1 / (|beta| |z|^2); c = conj(z) / (beta |z|^2)
-  const double r = recip_pos(root * fma(h.z.x, h.z.x, h.z.y * h.z.y));
+  const double r = 1.0 / (root * fma(h.z.x, h.z.x, h.z.y * h.z.y));
   const bool im = threadIdx.x & 1;   // a component per lane
   const double q = flip_sign((im ? h.z.y : h.z.x) * r, im != (sign != 0));
   h.c = mk(__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1));
@@ -797,9 +775,8 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
 // Bound like k_house_qr by the chain of a step: poll, the pivot search (on
 // the bits, as integers), one reciprocal, the next column's update.
 // A step's multipliers -(c[p] / pivot) are formed for 16 columns at a time,
-// a real component per lane (two FP64 instructions instead of four a column),
-// and the pivot's reciprocal by recip_pos: 196 columns and 392 right-hand
-// sides take 820 us (905 with a division and the multipliers in every lane).
+// a real component per lane (two FP64 instructions instead of four a column):
+// 196 columns and 392 right-hand sides took 905 us with them in every lane.
 __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx* B, int ldb, cplx* diag, int* perm,
                                                  int* info, cplx* pub, int in_smem, int nst, int* err) {
   extern __shared__ cplx lu_dyn[];
@@ -877,7 +854,7 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
     if (((__double_as_longlong(piv.x) | __double_as_longlong(piv.y)) << 1) != 0) {
       const int e = min(max(top_exp(piv) - 1023, -1000), 1000);
       if (e > -400 && e < 400) {
-        const double r = recip_pos(fma(piv.x, piv.x, piv.y * piv.y));
+        const double r = 1.0 / fma(piv.x, piv.x, piv.y * piv.y);
         rec = mk(piv.x * r, -piv.y * r);
       } else {
         const double s = pow2i(-e);
