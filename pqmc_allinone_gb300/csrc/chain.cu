@@ -134,20 +134,26 @@ __global__ void __launch_bounds__(PROP_THREADS, 2) k_propagate(DevModel M, cplx*
   const bool minus = comp == (forward ? 0 : 1);   // of ey below
   auto family = [&](int f) { return forward ? f : M.n_pf - 1 - f; };
   auto slice = [&](int it) { return (forward ? t_from + it : t_from - it) - 1; };
+  auto filled = [&](int f) {   // the first family from f on that has plaquettes (n_pf: none)
+    while (f < M.n_pf && M.pf_npla[family(f)] == 0) ++f;
+    return f;
+  };
+  const int f0 = filled(0);
   PropItem cur;
-  if (nt > 0 && M.n_pf > 0) prop_load(M, expkv, tid, family(0), slice(0), forward, cur);
+  if (nt > 0 && f0 < M.n_pf) prop_load(M, expkv, tid, family(f0), slice(0), forward, cur);
   __syncthreads();
   for (int it = 0; it < nt; ++it)
-    for (int f = 0; f < M.n_pf; ++f) {
+    for (int f = f0, fn; f < M.n_pf; f = fn) {
       const int pf = family(f), dim = M.pf_dim[pf], ni = 8 * M.pf_npla[pf];
+      fn = filled(f + 1);
       for (int i0 = 0; i0 < ni; i0 += nth) {
         const int i = i0 + tid;
         const bool on = i < ni && a < dim;
         PropItem nxt;
-        // the lane's next item: of this family, else the first of the next one
+        // the lane's next item: of this family, else the first of the next one with plaquettes
         if (i0 + nth < ni) prop_load(M, expkv, i + nth, pf, slice(it), forward, nxt);
-        else if (f + 1 < M.n_pf) prop_load(M, expkv, tid, family(f + 1), slice(it), forward, nxt);
-        else if (it + 1 < nt) prop_load(M, expkv, tid, family(0), slice(it + 1), forward, nxt);
+        else if (fn < M.n_pf) prop_load(M, expkv, tid, family(fn), slice(it), forward, nxt);
+        else if (it + 1 < nt) prop_load(M, expkv, tid, family(f0), slice(it + 1), forward, nxt);
         if (i0 + (tid & ~31) < ni) {   // any item in the warp
           double s = 0.0;
           if (on)

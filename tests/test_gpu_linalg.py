@@ -7,10 +7,12 @@ errors are a small multiple of eps * n; 1e-11 leaves two orders of room at
 the largest size.
 """
 import ctypes
+from dataclasses import replace
 
 import numpy as np
 import pytest
 
+from pqmc_allinone_gb300 import model as M
 from tests.helpers import SEED_WORDS, epsocz_small, general_bond_model, rel_fro
 
 pytestmark = pytest.mark.gpu
@@ -127,6 +129,38 @@ def test_propagation_in_passes(build, L):
     for c in (o, g):
         c.init_expkv()
     for t in (1, 3):   # through every slice from the right, and from both sides
+        for c in (o, g):
+            c.init_g(t)
+        assert rel_fro(g.g(), o.g()) < 1e-11
+    g.close()
+
+
+def _families_cut(keep, L=(4, 6)):
+    """epsocz_small with family keep[i][0] cut to its first keep[i][1] plaquettes, in that order."""
+    m, f = epsocz_small(L=L, ntime=4, ngroup=2, lam=0.8)
+    pfs = [m.spec.pfs[k] for k, _ in keep]
+    m = M.build_model(replace(m.spec, pfs=pfs), twist_seed=7, twist=1e-3)
+    m.pf = [M.PfTables(t.dim, min(n, t.n_pla), t.site_list[:n], t.crossing[:n], t.bc_phases[:n], t.bf_list[:n])
+            for t, (_, n) in zip(m.pf, keep)]
+    return m, f
+
+
+@pytest.mark.parametrize("L,keep", [((4, 6), [(0, 0), (0, 99), (1, 99), (2, 99), (3, 99)]),      # the first family empty
+                                    ((4, 6), [(0, 99), (1, 99), (1, 0), (1, 0), (2, 99), (3, 99)]),   # two in the middle
+                                    ((4, 6), [(0, 99), (1, 99), (2, 99), (3, 99), (0, 0)]),      # the last
+                                    ((4, 6), [(0, 0), (1, 0)]),                                  # all
+                                    ((12, 12), [(0, 99), (1, 3), (1, 0), (2, 99), (3, 65), (0, 0)])])   # and uneven ones
+def test_families_without_plaquettes(L, keep):
+    """Families of no plaquettes, and of different numbers, through every slice
+    in both directions; their slices leave the factors as they are."""
+    from oracle.oracle import OracleChain
+    from pqmc_allinone_gb300.engine import PqmcChain
+    m, f = _families_cut(keep, L)
+    o = OracleChain(m, field=f, seed_words=SEED_WORDS, meas=False)
+    g = PqmcChain(m, field=f, rng_words=SEED_WORDS, meas=False)
+    for c in (o, g):
+        c.init_expkv()
+    for t in (1, 3):
         for c in (o, g):
             c.init_g(t)
         assert rel_fro(g.g(), o.g()) < 1e-11
