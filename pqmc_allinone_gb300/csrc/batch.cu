@@ -530,10 +530,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
 #pragma unroll
       for (int m = 0; m < DS; ++m) gm[k][m] = bl[k][m] = Pair{{0.f, 0.f}, {0.f, 0.f}};
     int slot = 0;
-    for (int q0 = 0; q0 == 0 || q0 < K; q0 += SCAN_GAT) {
-      // the accepted sites' entries of the next columns
+    int q0 = 0, qe;
+    do {
+      // the accepted sites' entries of the next columns, in whole batches of the ring
       if (q0 > 0) __syncthreads();
-      const int qe = min(K, q0 + SCAN_GAT);
+      qe = min(K, q0 + SCAN_GAT);
+      if (qe < K && qe > res) qe -= (qe - res) % (ring / 2);
       for (int e = tid; e < 8 * (qe - q0); e += SCAN_THREADS) {
         const int q = q0 + (e >> 3), m = e & 3;
         if (m < dim) {
@@ -634,7 +636,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_bscan(const BDesc* D, int pf, 
           else read_back(ring / 2);
         }
       }
-    }
+      q0 = qe;
+    } while (q0 < K);
     __syncthreads();   // s_T, G(:,S), G(S,:)
     // ---- the new block: a = Geff(:,S) T, b = (I - Geff)(S,:) ----------------
     if (row) {

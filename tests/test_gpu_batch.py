@@ -580,3 +580,40 @@ def test_phase_timers_and_flush_rounds():
     assert all(0 < r <= launched for r in rounds), (rounds, launched)
     assert b.flush_rounds() == [0, 0]          # set_timing clears the counts
     b.close()
+
+
+def _three_site_model(L=15, ntime=4, ngroup=2, seed=1, **_):
+    """Families of three-site chains along x on a square lattice of L x L sites, L a multiple of 3."""
+    spec = general_bond_model(L=4)[0].spec
+    chain = [0, 1, 0, 1, 0, 1, 0, 1, 0]
+    pfs = [replace(spec.pfs[0], dim=3, tsl=[3, 0, 0, 1], offset=[o, 0], int_subsites=[0, 0, 1, 1, 0, 1, 2, 0, 1],
+                   kmat=[complex(v) for v in chain], vmat=[complex(v) for v in chain], bf_index=1) for o in range(3)]
+    m = M.build_model(replace(spec, lat_size=[L, L], pfs=pfs, beta=0.1 * ntime, ngroup=ngroup), twist_seed=3, twist=1e-3)
+    return m, M.field_gaussian(m, seed)
+
+
+@pytest.mark.parametrize("make,L,depth", [(epsocz_small, 10, 96), (epsocz_small, 14, 160), (_three_site_model, 15, 128)])
+def test_scan_chunks_past_the_resident_columns(make, L, depth):
+    """Delays at which the scan reads panel columns back, past the 64 that it
+    gathers the sites' entries of at a time: bit-identical for every chunk (1
+    and 2: one column a batch), and the chain of a delay of 64, which has no
+    second gather, to FP32 accumulation rounding."""
+    from pqmc_allinone_gb300.engine import PqmcBatch
+    m, f = make(L=L, ntime=4, ngroup=4, seed=77)
+    runs = {}
+    for key in [(64, 2)] + [(depth, qc) for qc in range(1, 9)]:
+        b = PqmcBatch([m], [f], [seed_words(970)], precision=1)
+        b.set_flush(0)
+        b.set_delay(key[0])
+        b.set_scan_chunk(key[1])
+        b.init()
+        b.sweep_slices(1, 1, 1)
+        runs[key] = (b.chains[0].field(), b.chains[0].g(), b.chains[0].state())
+        b.close()
+    f0, g0, s0 = runs[(depth, 1)]
+    assert s0["positive_accept"] * m.pf[0].dim > 72 * len(m.pf)   # more than 64 columns in a family's round
+    for qc in range(2, 9):
+        f1, g1, s1 = runs[(depth, qc)]
+        assert np.array_equal(f0, f1) and np.array_equal(g0, g1) and s0["ln_cw"] == s1["ln_cw"], qc
+    f1, g1, s1 = runs[(64, 2)]
+    assert np.array_equal(f0, f1) and rel_fro(g1, g0) < 2e-6
