@@ -323,8 +323,10 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
 // column at 288 x 144; the whole factorisation takes 617 us with this and 733
 // without, 1054 and 1158 at 392 x 196).  One or two columns per CTA.  `gs` (n x n, column k holds
 // the products of column k) starts out LA_EMPTY like `pub`.
+constexpr int UT_SUM = 16;   // terms of U y in a sum of their own: one after another they gave 1.06 times the error
 __device__ __forceinline__ void form_q_ut(int m, int n, int b, int G, int nl, cplx* cols, cplx* pub, cplx* xs,
-                                          const cplx* s_z, const cplx* s_c, const double* s_up, cplx* s_y, int* s_fail) {
+                                          const cplx* s_z, const cplx* s_c, const double* s_up, cplx* s_y, bool apart,
+                                          int* s_fail) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   cplx* gs = pub + (size_t)m * n;
   auto one = [](double up) { return __double2hiint(up) == 0x3ff00000; };
@@ -443,9 +445,21 @@ __device__ __forceinline__ void form_q_ut(int m, int n, int b, int G, int nl, cp
   fetch_wait<0>();
   if (!ok) *s_fail = 1;
   __syncthreads();
-  // e_j + U y, own rows
+  // e_j + U y, own rows; the terms in sums of UT_SUM where there is room
+  cplx* sums = apart ? s_y + (size_t)nl * n : cols;
+  auto flush = [&]() {
+    for (int l = 0; l < nl; ++l)
+      for (int k = tid; k < m; k += LT) {
+        const size_t e = (size_t)l * m + k;
+        cols[e] = cadd(cols[e], sums[e]);
+        sums[e] = mk(0.0);
+      }
+  };
   for (int l = 0; l < nl; ++l)
-    for (int k = tid; k < m; k += LT) cols[(size_t)l * m + k] = mk(k == b + l * G ? 1.0 : 0.0);
+    for (int k = tid; k < m; k += LT) {
+      sums[(size_t)l * m + k] = mk(0.0);
+      cols[(size_t)l * m + k] = mk(k == b + l * G ? 1.0 : 0.0);
+    }
   for (int q = 0; q < 3; ++q) {
     if (q <= jlast) fetch_col(pub + (size_t)m * q, xs + (size_t)q * m, q, m);
     fetch_commit();
@@ -461,17 +475,19 @@ __device__ __forceinline__ void form_q_ut(int m, int n, int b, int G, int nl, cp
       const cplx ya = s_y[i], yb = s_y[(size_t)n + i];
       for (int k = k0; k < m; k += LT) {
         const cplx v = x[k];
-        cols[k] = cfma(v, ya, cols[k]);
-        cols[(size_t)m + k] = cfma(v, yb, cols[(size_t)m + k]);
+        sums[k] = cfma(v, ya, sums[k]);
+        sums[(size_t)m + k] = cfma(v, yb, sums[(size_t)m + k]);
       }
     } else {
       const cplx y = s_y[(size_t)(nl - 1) * n + i];
-      cplx* c = cols + (size_t)(nl - 1) * m;
+      cplx* c = sums + (size_t)(nl - 1) * m;
       for (int k = k0; k < m; k += LT) c[k] = cfma(x[k], y, c[k]);
     }
+    if (apart && i % UT_SUM == UT_SUM - 1) flush();
     if (i + 3 <= jlast) fetch_col(pub + (size_t)m * (i + 3), xs + (size_t)((i + 3) & 3) * m, i + 3, m);
     fetch_commit();
   }
+  if (apart) flush();
   fetch_wait<0>();
   __syncthreads();
 }
@@ -505,9 +521,10 @@ __device__ __forceinline__ void form_q_ut(int m, int n, int b, int G, int nl, cp
 // QR_COPIES copies of {c, (beta, up)}, so that not every CTA polls one sector.
 //
 // dynamic shared memory: nst columns of the ring, z and c of n reflectors, the local columns' exponents, the local columns if `in_smem`
-// (else they stay in A).
+// (else they stay in A).  Four CTAs an SM: the compiler takes 80 registers and
+// spills without the bound (12x12: 16.29 ms a start, 15.96 with it).
 constexpr int QR_COPIES = 4, QR_SELF = 2 * QR_COPIES;
-__global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d, cplx* Rout, cplx* lndet, cplx* pub,
+__global__ void __launch_bounds__(LT, 4) k_house_qr(int m, int n, cplx* A, cplx* d, cplx* Rout, cplx* lndet, cplx* pub,
                                                  int in_smem, int nst, int ut, int* err) {
   extern __shared__ cplx qr_dyn[];
   __shared__ double red[2][4][4];
@@ -521,8 +538,8 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
   cplx* s_c = s_z + n;
   double* s_up = reinterpret_cast<double*>(s_c + n);   // power of two on x (1 but for vanishing remainders)
   int* s_exp = reinterpret_cast<int*>(s_up + 2 * ((n + 1) / 2));
-  cplx* s_y = s_c + n + (n + 1) / 2 + (nl + 3) / 4;   // ut: [nl][n]
-  cplx* cols = s_y + (ut ? nl * n : 0);
+  cplx* s_y = s_c + n + (n + 1) / 2 + (nl + 3) / 4;   // ut: [nl][n], and with 2 the sums of U y, [nl][m]
+  cplx* cols = s_y + (ut ? (size_t)nl * n : 0) + (ut == 2 ? (size_t)nl * m : 0);
   auto col = [&](int l) { return in_smem ? cols + (size_t)l * m : A + (size_t)m * (b + (size_t)l * G); };
   int half = 0;
   if (tid == 0) s_fail = 0;
@@ -687,7 +704,7 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
     if (tid == 0) lndet[0] = mk(0.0, ph);
   }
   if (ut) {
-    form_q_ut(m, n, b, G, nl, cols, pub, xs, s_z, s_c, s_up, s_y, &s_fail);
+    form_q_ut(m, n, b, G, nl, cols, pub, xs, s_z, s_c, s_up, s_y, ut == 2, &s_fail);
     if (s_fail) {   // read after the barrier that ends form_q_ut
       if (tid == 0) atomicExch(err, PQMC_ERR_TIMEOUT);
       return;
@@ -777,6 +794,14 @@ __global__ void __launch_bounds__(LT) k_house_qr(int m, int n, cplx* A, cplx* d,
 // A step's multipliers -(c[p] / pivot) are formed for 16 columns at a time,
 // a real component per lane (two FP64 instructions instead of four a column):
 // 196 columns and 392 right-hand sides took 905 us with them in every lane.
+//
+// A right-hand side's terms are summed LU_SUM at a time apart from its
+// entries (`sums`) and added to them then, in both passes: one term after
+// another each rounds at the entry's size, and G came out with twice the error
+// of dot products over 32 lanes (1.2e-15 and 6.4e-16 at n = 100; 6.5e-16 so).
+// Columns of A keep the plain order, which the pivots and the chain depend on;
+// so do right-hand sides in global memory in the first pass (n past ~590).
+constexpr int LU_SUM = 16;
 __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx* B, int ldb, cplx* diag, int* perm,
                                                  int* info, cplx* pub, int in_smem, int nst, int* err) {
   extern __shared__ cplx lu_dyn[];
@@ -787,17 +812,30 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
   const int nl = (T - b + G - 1) / G;
   cplx* xs = lu_dyn;
   cplx* s_rec = xs + (size_t)nst * n;          // reciprocals of the pivots
-  cplx* s_sol = s_rec + n;                     // a solution in progress (!in_smem)
-  int* s_prow = reinterpret_cast<int*>(s_sol + (in_smem ? 0 : n));
+  int* s_prow = reinterpret_cast<int*>(s_rec + n);
   int* s_ord = s_prow + n;                     // step at which a row became the pivot row
-  cplx* cols = s_rec + n + (in_smem ? 0 : n) + (2 * n + 3) / 4;
+  cplx* sums = s_rec + n + (2 * n + 3) / 4;    // per local right-hand side (!in_smem: of the one in work)
+  const int lr = b >= n ? 0 : min(nl, (n - b + G - 1) / G);   // first local right-hand side
+  cplx* cols = sums + (in_smem ? (size_t)(nl - lr) * n : (size_t)n);
   auto gcol = [&](int l) {
     const size_t j = b + (size_t)l * G;
     return j < (size_t)n ? A + (size_t)n * j : B + (size_t)ldb * (j - n);
   };
   auto col = [&](int l) { return in_smem ? cols + (size_t)l * n : gcol(l); };
+  auto sum = [&](int l) { return in_smem ? sums + (size_t)(l - lr) * n : sums; };
+  // own rows' sums of right-hand side l into its entries, but row p, which others read
+  auto flush = [&](int l, int p) {
+    cplx *c = col(l), *a = sum(l);
+    for (int k = tid; k < n; k += LT)
+      if (k != p) {
+        c[k] = cadd(c[k], a[k]);
+        a[k] = mk(0.0);
+      }
+  };
   if (tid == 0) s_fail = 0;
   for (int k = tid; k < n; k += LT) s_ord[k] = n;
+  if (in_smem)
+    for (int k = tid; k < (nl - lr) * n; k += LT) sums[k] = mk(0.0);
   if (in_smem)
     for (int l = 0; l < nl; ++l)
       for (int k = tid; k < n; k += LT) col(l)[k] = gcol(l)[k];
@@ -805,6 +843,7 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
   if (b == 0)
     for (int k = tid; k < n; k += LT) publish(pub + k, col(0)[k]);
   const bool last_owner = (n - 1) % G == b;
+  const bool apart = in_smem && lr < nl;   // right-hand sides with their terms apart
   int first_zero = 0;
   int li = 0, jown = b;   // the next local column, local and global
   for (int j = 0; j < n; ++j) {
@@ -874,13 +913,17 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
         perm[j] = p;
       }
     }
+    if (apart && j && j % LU_SUM == 0)
+      for (int l = lr; l < nl; ++l) flush(l, p);
     double fl = 0.0;   // -(c[p] / piv) of 16 columns at a time, a real component per lane
     for (int l = l0; l < nl; ++l) {
-      cplx* c = col(l);
+      cplx* c = apart && l >= lr ? sum(l) : col(l);
       const int lq = (l - l0) & 15;
       if (lq == 0) {
         const bool im = lane & 1;
-        const cplx v = col(min(l + (lane >> 1), nl - 1))[p];
+        const int lv = min(l + (lane >> 1), nl - 1);
+        cplx v = col(lv)[p];
+        if (apart && lv >= lr) v = cadd(v, sum(lv)[p]);
         fl = fma(flip_sign(rec.y, im), im ? v.x : v.y, -(rec.x * (im ? v.y : v.x)));
       }
       const cplx f = mk(__shfl_sync(0xffffffffu, fl, 2 * lq), __shfl_sync(0xffffffffu, fl, 2 * lq + 1));
@@ -898,27 +941,41 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
   }
   if (last_owner && tid == 0) info[0] = first_zero;
   // ---- back substitution: x_j = y(p_j) / u_jj, y(p_k) -= U(p_k, j) x_j -----
-  const int lr = b >= n ? 0 : (n - b + G - 1) / G;   // first local right-hand side
   if (lr >= nl) return;
   __threadfence();
   __syncthreads();
   const int nb = in_smem ? nl - lr : 1;
   for (int r0 = lr; r0 < nl; r0 += nb) {
+    if (in_smem)
+      for (int l = lr; l < nl; ++l) flush(l, -1);
+    else
+      for (int k = tid; k < n; k += LT) sums[k] = mk(0.0);
     for (int u = 0; u < nst - 1; ++u) {
       const int j = n - 1 - u;
       if (j >= 0) fetch_col(pub + (size_t)n * j, xs + (size_t)(j & (nst - 1)) * n, 0, n);
       fetch_commit();
     }
+    cplx done = mk(0.0);   // !in_smem: the last unknown, kept in the place of its row's sum
     for (int j = n - 1; j >= 0; --j) {
       if (nst == 4) fetch_wait<2>();
       else fetch_wait<0>();
       const cplx* u = xs + (size_t)(j & (nst - 1)) * n;
-      const int p = s_prow[j];
+      const int p = s_prow[j], pn = j > 0 ? s_prow[j - 1] : -1;
       const cplx rec = s_rec[j];
       __syncthreads();   // the rows of step j + 1 are in
+      if (!in_smem && tid == 0 && j < n - 1) sums[s_prow[j + 1]] = done;
+      if (j % LU_SUM == LU_SUM - 1)
+        for (int l = r0; l < r0 + nb; ++l) {
+          cplx *y = col(l), *a = sum(l);
+          for (int k = tid; k < n; k += LT)
+            if (s_ord[k] < j) {
+              y[k] = cadd(y[k], a[k]);
+              a[k] = mk(0.0);
+            }
+        }
       double xl = 0.0;   // y[p] / u_jj of 16 columns at a time, a real component per lane
       for (int l = r0; l < r0 + nb; ++l) {
-        cplx* y = col(l);
+        cplx *y = col(l), *a = sum(l);
         const int lq = (l - r0) & 15;
         if (lq == 0) {
           const bool im = lane & 1;
@@ -928,11 +985,13 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
         const cplx xj = mk(__shfl_sync(0xffffffffu, xl, 2 * lq), __shfl_sync(0xffffffffu, xl, 2 * lq + 1));
         const cplx f = cneg(xj);
         for (int k = tid; k < n; k += LT)
-          if (s_ord[k] < j) y[k] = cfma(u[k], f, y[k]);
-        if (tid == 0) {
-          if (in_smem) B[j + (size_t)ldb * (b + (size_t)l * G - n)] = xj;
-          else s_sol[j] = xj;
-        }
+          if (s_ord[k] < j) {
+            cplx t = a[k];
+            if (k == pn) t = cadd(t, y[k]);   // the row that the next step reads, complete
+            *(k == pn ? y + k : a + k) = cfma(u[k], f, t);
+          }
+        if (in_smem && tid == 0) B[j + (size_t)ldb * (b + (size_t)l * G - n)] = xj;
+        done = xj;
       }
       const int jn = j - (nst - 1);
       if (jn >= 0) fetch_col(pub + (size_t)n * jn, xs + (size_t)(jn & (nst - 1)) * n, 0, n);
@@ -940,7 +999,9 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
     }
     if (!in_smem) {
       __syncthreads();
-      for (int k = tid; k < n; k += LT) gcol(r0)[k] = s_sol[k];
+      if (tid == 0) sums[s_prow[0]] = done;
+      __syncthreads();
+      for (int k = tid; k < n; k += LT) gcol(r0)[k] = sums[s_prow[k]];
       __syncthreads();
     }
   }
@@ -987,7 +1048,8 @@ int coop_grid(const void* fn, int threads, int want, size_t smem) {
 // rows.  Two CTAs per SM while their columns fit in half its shared memory
 // (at Ns = 392, nelec = 196 a CTA has one column of the QR), one while they
 // fit in all of it, and past that the columns stay in global memory.
-// `fixed`: complex entries besides the ring and the columns.
+// `fixed`(grid, columns per CTA, in shared memory): complex entries besides
+// the ring and the columns.
 struct PipeShape {
   int grid, in_smem, nst;
   size_t smem;
@@ -1005,7 +1067,7 @@ static int pipe_shape(const void* fn, int ncol, int len, FIXED fixed, PipeShape*
     q.in_smem = o.in;
     q.nst = o.nst;
     const int nl = (ncol + q.grid - 1) / q.grid;
-    q.smem = sizeof(cplx) * ((size_t)o.nst * len + fixed(nl, o.in) + (o.in ? (size_t)nl * len : 0));
+    q.smem = sizeof(cplx) * ((size_t)o.nst * len + fixed(q.grid, nl, o.in) + (o.in ? (size_t)nl * len : 0));
     if (q.smem > o.lim || (&o == opt && nl > 2)) continue;
     PQMC_CUDA(raise_dyn_smem((const char*)fn, (int)q.smem));
     int per = 0;
@@ -1025,11 +1087,16 @@ int house_qr(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* work, int* er
 int house_qr_r(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* R, cplx* lndet, cplx* work, int* err) {
   PipeShape q;
   // Q by the triangular factor where the work matrix (m x m) has room for its
-  // products behind the published columns (a square A has none)
-  const bool room = (size_t)m * (m - n) >= (size_t)n * n;
-  PQMC_TRY(pipe_shape((const void*)k_house_qr, n, m,
-                      [&](int nl, int in) { return (size_t)2 * n + (n + 1) / 2 + (nl + 3) / 4 + (room && in ? (size_t)nl * n : 0); }, &q));
-  int ut = room && q.in_smem && q.nst == 4 && n <= 2 * q.grid;
+  // products behind the published columns (a square A has none), with the
+  // terms of U y in sums (2) where shared memory has room for those too
+  int ut = (size_t)m * (m - n) >= (size_t)n * n ? 2 : 0;
+  for (;; --ut) {
+    PQMC_TRY(pipe_shape((const void*)k_house_qr, n, m,
+                        [&](int, int nl, int in) {
+                          return (size_t)2 * n + (n + 1) / 2 + (nl + 3) / 4 + (ut && in ? (size_t)nl * n : 0) + (ut == 2 && in ? (size_t)nl * m : 0);
+                        }, &q));
+    if (ut == 0 || (q.in_smem && q.nst == 4 && n <= 2 * q.grid)) break;
+  }
   PQMC_CUDA(cudaMemsetAsync(work, 0xff, sizeof(cplx) * ((size_t)m * n + (ut ? (size_t)n * n : 0)), s));
   void* args[] = {&m, &n, &A, &d, &R, &lndet, &work, &q.in_smem, &q.nst, &ut, &err};
   PQMC_CUDA(cudaLaunchCooperativeKernel((const void*)k_house_qr, q.grid, LT, args, q.smem, s));
@@ -1041,7 +1108,7 @@ int lu_solve(cudaStream_t s, int n, cplx* A, int nrhs, cplx* B, int ldb, cplx* d
              int* err) {
   PipeShape q;
   PQMC_TRY(pipe_shape((const void*)k_lu_solve, n + nrhs, n,
-                      [&](int, int in) { return (size_t)n + (in ? 0 : n) + (2 * n + 3) / 4; }, &q));
+                      [&](int grid, int, int in) { return (size_t)n + (2 * n + 3) / 4 + (in ? (size_t)((nrhs + grid - 1) / grid) * n : (size_t)n); }, &q));
   PQMC_CUDA(cudaMemsetAsync(work, 0xff, sizeof(cplx) * (size_t)n * n, s));
   void* args[] = {&n, &A, &nrhs, &B, &ldb, &diag, &perm, &info, &work, &q.in_smem, &q.nst, &err};
   PQMC_CUDA(cudaLaunchCooperativeKernel((const void*)k_lu_solve, q.grid, LT, args, q.smem, s));

@@ -165,3 +165,55 @@ def test_families_without_plaquettes(L, keep):
             c.init_g(t)
         assert rel_fro(g.g(), o.g()) < 1e-11
     g.close()
+
+
+def test_lu_solve_sums_terms_apart(ns=392, ne=196, tol=7.4e-15):
+    """The error of G's first columns against extended precision, for a dense
+    unitary X^H R.  The multiply-adds of the kernels in numpy, two roundings
+    per component, give 8.6e-15 with the terms of the triangular solves added
+    one after another and 6.4e-15 with sums of 16 terms; the bound is the
+    geometric mean."""
+    torch = pytest.importorskip("torch")
+    from pqmc_allinone_gb300.abi import load_library
+    rng = np.random.default_rng(ns + ne)
+
+    def normal(a, b):
+        return rng.normal(size=(a, b)) + 1j * rng.normal(size=(a, b))
+
+    x, u = np.linalg.qr(normal(ns, ne))[0], np.linalg.qr(normal(ne, ne))[0]
+    r = np.linalg.qr(x @ u + 0.3 * normal(ns, ne) / np.sqrt(2 * ns))[0]
+    lib = load_library()
+    fn = lib.pqmc_cal_g_and_det_noalloc
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 3
+    fn.restype = ctypes.c_int
+    dev = [torch.from_numpy(np.asfortranarray(a).ravel(order="F").view(np.float64).copy()).cuda() for a in (x, r)]
+    out = torch.zeros(2 * ns * ns + 2, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert fn(dev[0].data_ptr(), dev[1].data_ptr(), ns, ne, out.data_ptr(), out[2 * ns * ns:].data_ptr(), None) == 0
+    g = out[:2 * ns * ns].cpu().numpy().view(np.complex128).reshape((ns, ns), order="F")
+    # 16 columns of the answer: a 64-bit solve, refined with residuals in extended precision
+    a, b = x.conj().T.astype(np.clongdouble) @ r.astype(np.clongdouble), x[:16].conj().T.astype(np.clongdouble)
+    inv = np.linalg.inv(a.astype(np.complex128))
+    y = (inv @ b.astype(np.complex128)).astype(np.clongdouble)
+    for _ in range(3):
+        y = y + inv @ (b - a @ y).astype(np.complex128)
+    ref = r.astype(np.clongdouble) @ y
+    err = float(np.linalg.norm((g[:, :16] - ref).astype(np.complex128)) / np.linalg.norm(ref.astype(np.complex128)))
+    assert err < tol, err
+
+
+def test_lu_solve_with_columns_in_global_memory():
+    """Finite temperature at Ns = 800: columns and right-hand sides past what the CTAs' shared memory holds."""
+    from oracle.finite_t import dense_g_and_weight
+    from oracle.oracle import OracleChain
+    from pqmc_allinone_gb300.engine import PqmcChain
+    m, f = epsocz_small(L=(20, 20), ntime=4, ngroup=2, alpha=0.3)
+    o = OracleChain(m, field=f, seed_words=SEED_WORDS, meas=False)
+    o.init_expkv()
+    g = PqmcChain(m, field=f, rng_words=SEED_WORDS, meas=False)
+    g.set_temperature(False)
+    g.init_expkv()
+    g.init_g(1)
+    gd, ld = dense_g_and_weight(o)
+    assert rel_fro(g.g(), gd) < 1e-10
+    assert abs(g.state()["ln_cw"].real - ld.real) <= 1e-9 * abs(ld.real)
