@@ -587,6 +587,10 @@ int update_setup(pqmc_chain* c) {
     set_error("update kernel needs two co-resident blocks");
     return PQMC_ERR_CUDA;
   }
+  // no more CTAs than have entries (151 shares of Ns = 150 leave the last one
+  // empty): a share without entries would pass no barrier between two moves
+  const long chunk = (elems + c->upd_blocks - 2) / (c->upd_blocks - 1);
+  c->upd_blocks = 1 + (int)((elems + chunk - 1) / chunk);
   return PQMC_OK;
 }
 

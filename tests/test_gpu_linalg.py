@@ -217,3 +217,28 @@ def test_lu_solve_with_columns_in_global_memory():
     gd, ld = dense_g_and_weight(o)
     assert rel_fro(g.g(), gd) < 1e-10
     assert abs(g.state()["ln_cw"].real - ld.real) <= 1e-9 * abs(ld.real)
+
+
+def test_update_without_empty_shares():
+    """Ns = 150: 22500 entries in shares of 150 are one share fewer than 152 SMs have CTAs for."""
+    from oracle.oracle import OracleChain
+    from pqmc_allinone_gb300.engine import PqmcChain
+    spec = general_bond_model(L=4)[0].spec
+    pfs = [replace(spec.pfs[0], tsl=[2, 0, 0, 1], offset=[o, 0], bf_index=1) for o in (0, 1)]
+    m = M.build_model(replace(spec, lat_size=[10, 15], pfs=pfs, beta=0.4, ngroup=2), twist_seed=3, twist=1e-3)
+    assert m.ns == 150
+    f = M.field_gaussian(m, 5)
+    o = OracleChain(m, field=f, seed_words=SEED_WORDS, meas=False)
+    g = PqmcChain(m, field=f, rng_words=SEED_WORDS, meas=False)
+    for c in (o, g):
+        c.init_expkv()
+        c.init_g(1)
+    for pf in (2, 1):
+        for c in (o, g):
+            c.right_evolve_g(m.ntime, pf)
+            c.update_phonon_field(pf, m.ntime)
+        so, sg = o.state(), g.state()
+        assert sg["rng"] == so["rng"] and np.array_equal(g.field(), o.field())
+        assert sg["positive_accept"] == so["positive_accept"] > 0
+        assert rel_fro(g.g(), o.g()) < 1e-10
+    g.close()
