@@ -236,8 +236,5 @@ extern "C" int pqmc_logweight_grad(pqmc_chain* c, double* logw_out, double* grad
   PQMC_CUDA(cudaMemcpyAsync(c->g, gtmp, sizeof(cplx) * (size_t)ns * ns, cudaMemcpyDeviceToDevice, s));
   PQMC_CUDA(cudaFreeAsync(gtmp, s));
   PQMC_CUDA(cudaFreeAsync(ck, s));
-  int late = 0;
-  PQMC_CUDA(cudaMemcpyAsync(&late, &c->sc->lin_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  PQMC_CUDA(cudaStreamSynchronize(s));
-  return late ? check_factor(c, "logweight_grad") : PQMC_OK;
+  return check_waits(c, "logweight_grad");
 }

@@ -338,6 +338,14 @@ int check_factor(pqmc_chain* c, const char* what) {
   return PQMC_OK;
 }
 
+// waits for the stream and reports a wait that ran out inside a kernel
+int check_waits(pqmc_chain* c, const char* what) {
+  int late = 0;
+  PQMC_CUDA(cudaMemcpyAsync(&late, &c->sc->lin_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  PQMC_CUDA(cudaStreamSynchronize(c->stream));
+  return late ? check_factor(c, what) : PQMC_OK;
+}
+
 // cal_g_and_det_T0 with the left factor held as X = lmat^H (Ns x nelec)
 static int cal_g_and_det(pqmc_chain* c, const cplx* X, const cplx* R, bool compare) {
   const int ns = c->ns, ne = c->nelec;
@@ -901,10 +909,7 @@ int pqmc_update_phonon_field(pqmc_chain* c, int pf_id, int time) {
     return PQMC_ERR_ARG;
   }
   PQMC_TRY(launch_update(c, pf_id - 1, time));
-  int late = 0;
-  PQMC_CUDA(cudaMemcpyAsync(&late, &c->sc->lin_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  PQMC_CUDA(cudaStreamSynchronize(c->stream));
-  return late ? check_factor(c, "update_phonon_field") : PQMC_OK;
+  return check_waits(c, "update_phonon_field");
 }
 
 int pqmc_left_evolve_g(pqmc_chain* c, int time, int pf_id, int two_way) {

@@ -151,6 +151,7 @@ int launch_update(pqmc_chain* c, int pf, int time);
 int update_setup(pqmc_chain* c);
 int launch_wrap(pqmc_chain* c, int pf, int time, bool left);
 int check_factor(pqmc_chain* c, const char* what);
+int check_waits(pqmc_chain* c, const char* what);
 int launch_propagate(pqmc_chain* c, cplx* X, int n, int t_from, int t_to, bool forward);
 int do_init_g(pqmc_chain* c, int start_time);
 int do_g_scratch(pqmc_chain* c, int time, bool forward, int loop);

@@ -10,6 +10,12 @@
 
 typedef double2 cplx;
 
+// Limit of a wait inside a kernel in clock cycles, ~2 s.  A build may set a
+// shorter one to see waits run out.
+#ifndef PQMC_WAIT_CYCLES
+#define PQMC_WAIT_CYCLES (4LL << 30)
+#endif
+
 __host__ __device__ __forceinline__ cplx mk(double r, double i = 0.0) { return make_double2(r, i); }
 __host__ __device__ __forceinline__ cplx cadd(cplx a, cplx b) { return mk(a.x + b.x, a.y + b.y); }
 __host__ __device__ __forceinline__ cplx csub(cplx a, cplx b) { return mk(a.x - b.x, a.y - b.y); }

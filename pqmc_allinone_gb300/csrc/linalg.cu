@@ -145,7 +145,7 @@ __device__ __forceinline__ bool poll_col(const cplx* src, cplx* dst, int k0, int
           dst[k + e * LT] = mk(__longlong_as_double((long long)x[e]), __longlong_as_double((long long)y[e]));
           need &= ~(1u << e);
         }
-      if (need && clock64() - t0 > (4LL << 30)) return false;
+      if (need && clock64() - t0 > PQMC_WAIT_CYCLES) return false;
     }
   }
   return true;
@@ -162,7 +162,7 @@ __device__ __forceinline__ bool poll_pair(const cplx* src, cplx* dst) {
       if ((threadIdx.x & 31) < 2) dst[w] = mk(__longlong_as_double((long long)x), __longlong_as_double((long long)y));
       return true;
     }
-    if (__any_sync(0xffffffffu, clock64() - t0 > (4LL << 30))) return false;
+    if (__any_sync(0xffffffffu, clock64() - t0 > PQMC_WAIT_CYCLES)) return false;
   }
 }
 
@@ -387,7 +387,7 @@ __device__ __forceinline__ void form_q_ut(int m, int n, int b, int G, int nl, cp
   auto product = [&](int k, int i) {   // c_i u_i^H u_k
     cplx v = xs[(size_t)(k & 3) * m + i];
     while ((unsigned long long)__double_as_longlong(v.x) == LA_EMPTY || (unsigned long long)__double_as_longlong(v.y) == LA_EMPTY) {
-      if (!ok || clock64() - t0 > (4LL << 30)) {
+      if (!ok || clock64() - t0 > PQMC_WAIT_CYCLES) {
         ok = false;
         break;
       }

@@ -523,7 +523,7 @@ int pqmc_sweep(pqmc_chain* c, int first_loop, int n_sweeps, int warmup, int meas
     if (c->have_global) PQMC_TRY(pqmc_global_step(c, loop, nullptr));
     PQMC_TRY(sweep_one(c, loop, warmup, meas_interval, meas_number, records, n_records_cap, &nrec));
   }
-  PQMC_CUDA(cudaStreamSynchronize(c->stream));
+  PQMC_TRY(check_waits(c, "sweep"));
   if (n_records) *n_records = nrec;
   return PQMC_OK;
 }
@@ -538,8 +538,7 @@ int pqmc_sweep_slices(pqmc_chain* c, int loop, int first_tc, int n_slices) {
   if (n_slices == 0) return PQMC_OK;
   int nrec = 0;
   PQMC_TRY(sweep_one(c, loop, 1 << 30, 1, 0, nullptr, 0, &nrec, first_tc, first_tc + n_slices - 1));
-  PQMC_CUDA(cudaStreamSynchronize(c->stream));
-  return PQMC_OK;
+  return check_waits(c, "sweep_slices");
 }
 
 }  // extern "C"

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <utility>
+#include "common.cuh"
 
 namespace pqmc {
 
@@ -32,7 +33,7 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint64_t* b, uint32_t parity) 
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* b, uint32_t parity) {
   const long long t0 = clock64();
   while (!mbar_try_wait(b, parity))
-    if (clock64() - t0 > (4LL << 30)) return false;
+    if (clock64() - t0 > PQMC_WAIT_CYCLES) return false;
   return true;
 }
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* b) {

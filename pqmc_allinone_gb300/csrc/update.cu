@@ -99,7 +99,7 @@ __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" 
 __device__ __forceinline__ bool wait_count(const unsigned* p, unsigned base, unsigned want) {
   const long long t0 = clock64();
   while (ld_acquire(p) - base < want)
-    if (clock64() - t0 > (4LL << 30)) return false;
+    if (clock64() - t0 > PQMC_WAIT_CYCLES) return false;
   return true;
 }
 
@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
         if (moves > 1) {
           if (lane == 0) ok = wait_count(&sync->done, done0, (unsigned)(moves - 1));
           ok = __shfl_sync(0xffffffffu, ok, 0);
+          if (!ok && lane == 0) atomicExch(&sc->lin_err, PQMC_ERR_TIMEOUT);   // whichever warp publishes
         }
         int found = -1, win = 0;
         for (int p0 = next; p0 < npla && found < 0; p0 += UPD_SPEC) {
