@@ -898,8 +898,8 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
       } else {
         const double s = pow2i(-e);
         const cplx q = cscale(piv, s);
-        const double r = s / fma(q.x, q.x, q.y * q.y);
-        rec = mk(q.x * r, -q.y * r);
+        const double r = 1.0 / fma(q.x, q.x, q.y * q.y);
+        rec = mk(q.x * r * s, -q.y * r * s);   // s last: s r can leave the range where the product does not
       }
     } else if (!first_zero) {
       first_zero = j + 1;

@@ -242,3 +242,27 @@ def test_update_without_empty_shares():
         assert sg["positive_accept"] == so["positive_accept"] > 0
         assert rel_fro(g.g(), o.g()) < 1e-10
     g.close()
+
+
+@pytest.mark.parametrize("exponent", [-1016, -500, 500, 1016])
+def test_lu_solve_at_the_ends_of_the_range(exponent):
+    """Pivots near 2^-1016 .. 2^1016: G = R (X^H R)^-1 X^H does not depend on
+    R's scale.  Backward-stable for a unitary X^H R of order 8: a few eps n,
+    below 1e-14; a reciprocal with bits lost below 2^-1022 gives 1e-13."""
+    torch = pytest.importorskip("torch")
+    from pqmc_allinone_gb300.abi import load_library
+    n = 8
+    rng = np.random.default_rng(5)
+    r = np.ldexp(1.0, exponent) * np.linalg.qr(rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n)))[0]
+    lib = load_library()
+    fn = lib.pqmc_cal_g_and_det_noalloc
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 3
+    fn.restype = ctypes.c_int
+    dev = [torch.from_numpy(np.asfortranarray(a).ravel(order="F").view(np.float64).copy()).cuda()
+           for a in (np.eye(n, dtype=np.complex128), r)]
+    out = torch.zeros(2 * n * n + 2, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert fn(dev[0].data_ptr(), dev[1].data_ptr(), n, n, out.data_ptr(), out[2 * n * n:].data_ptr(), None) == 0
+    o = out.cpu().numpy()
+    assert rel_fro(o[:2 * n * n].view(np.complex128).reshape((n, n), order="F"), np.eye(n)) < 1e-14
+    assert abs(o[-2] - n * exponent * np.log(2.0)) < 1e-11
