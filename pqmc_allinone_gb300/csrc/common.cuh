@@ -26,6 +26,12 @@ __host__ __device__ __forceinline__ cplx csub(cplx a, cplx b) { return mk(a.x - 
 __device__ __forceinline__ double flip_sign(double v, bool neg) {
   return __hiloint2double(__double2hiint(v) ^ (neg ? (int)0x80000000 : 0), __double2loint(v));
 }
+// power of two as a double, |e| <= 1022
+__device__ __forceinline__ double pow2i(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
+// biased exponent of the larger component
+__device__ __forceinline__ int top_exp(double2 v) {
+  return max((__double2hiint(v.x) & 0x7fffffff) >> 20, (__double2hiint(v.y) & 0x7fffffff) >> 20);
+}
 #endif
 __host__ __device__ __forceinline__ cplx cneg(cplx a) {
 #ifdef __CUDA_ARCH__

@@ -262,12 +262,6 @@ __device__ __forceinline__ double cta_sum1(double a, double (*red)[4]) {
   return cta_total(red[0]);
 }
 
-// power of two as a double, |e| <= 1022
-__device__ __forceinline__ double pow2i(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
-// biased exponent of the larger component
-__device__ __forceinline__ int top_exp(cplx v) {
-  return max((__double2hiint(v.x) & 0x7fffffff) >> 20, (__double2hiint(v.y) & 0x7fffffff) >> 20);
-}
 // the CTA's largest v >= 0 to every thread (two barriers)
 __device__ __forceinline__ int cta_max(int v, int* red) {
   v = __reduce_max_sync(0xffffffffu, v);

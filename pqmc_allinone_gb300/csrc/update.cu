@@ -473,7 +473,16 @@ __global__ void __launch_bounds__(256) k_update(DevModel M, DevScalars* sc, UpdC
               cof = cfma_part(B.r[io + 4 * c2], B.min[mo + pair_index(c0, c1)], cof, part);
               cof = flip_sign(cof, (i4 + j4) & 1);
               st_part(&B.g1[at], part, cof);
-              const double rd = flip_sign(part ? det.y : det.x, part) / (det.x * det.x + det.y * det.y);
+              // 1 / det = conj(det) / |det|^2, scaled by a power of two where the square could leave the range
+              const int de = top_exp(det) - 1023;
+              double rd;
+              if (de > -400 && de < 400) {
+                rd = flip_sign(part ? det.y : det.x, part) / (det.x * det.x + det.y * det.y);
+              } else {
+                const double sc = pow2i(-min(max(de, -1000), 1000));
+                const cplx ds = cscale(det, sc);
+                rd = flip_sign(part ? ds.y : ds.x, part) / (ds.x * ds.x + ds.y * ds.y) * sc;
+              }
               const cplx rdet = mk(__shfl_sync(0xffffffffu, rd, 0), __shfl_sync(0xffffffffu, rd, 16));
               __syncwarp();
               st_part(&B.w[j4 + 4 * i4], part, cfma_part(B.g1[at], rdet, 0.0, part));

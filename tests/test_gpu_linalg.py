@@ -266,3 +266,29 @@ def test_lu_solve_at_the_ends_of_the_range(exponent):
     o = out.cpu().numpy()
     assert rel_fro(o[:2 * n * n].view(np.complex128).reshape((n, n), order="F"), np.eye(n)) < 1e-14
     assert abs(o[-2] - n * exponent * np.log(2.0)) < 1e-11
+
+
+def test_update_with_a_determinant_past_the_square_root_of_the_range():
+    """A move whose |det R| is about 1e184: its square is infinite, 1 / det and the new G are not."""
+    from oracle.oracle import OracleChain
+    from pqmc_allinone_gb300.engine import PqmcChain
+    from pqmc_allinone_gb300.rng import seed_words
+    spec = general_bond_model(L=4)[0].spec
+    hop = np.diag([1, 1, 1], 1) + np.diag([1, 1, 1], -1)
+    pf = replace(spec.pfs[0], dim=4, tsl=[4, 0, 0, 1], offset=[0, 0], int_subsites=[0, 0, 1, 1, 0, 1, 2, 0, 1, 3, 0, 1],
+                 kmat=[complex(v) for v in hop.ravel()], vmat=[complex(v) for v in np.eye(4).ravel()], bf_index=1)
+    m = M.build_model(replace(spec, pfs=[pf], beta=0.4, ngroup=2), twist_seed=3, twist=1e-3)
+    m.D, m.M, m.jump_distance = 1e-9, 0.0, 5700.0   # a spring so soft that such a jump is accepted
+    f = np.zeros((m.n_bf, m.ntime), order="F")
+    o = OracleChain(m, field=f, seed_words=seed_words(4), meas=False)
+    g = PqmcChain(m, field=f, rng_words=seed_words(4), meas=False)
+    for c in (o, g):
+        c.init_expkv()
+        c.init_g(1)
+    before = g.g()
+    for c in (o, g):
+        c.update_phonon_field(1, 1)
+    assert o.state()["positive_accept"] == g.state()["positive_accept"] == 1 and o.state()["ln_cw"].real > 400
+    assert np.array_equal(g.field(), o.field())
+    assert rel_fro(o.g(), before) > 0.1 and rel_fro(g.g(), o.g()) < 1e-10
+    g.close()
