@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <atomic>
+#include <mutex>
 #include "../../include/pqmc_gb300.h"
 #include "../../include/pqmc_boxmuller.h"
 
@@ -100,9 +101,15 @@ inline void count_launch(int n = 1) { g_launches.fetch_add(n, std::memory_order_
   } while (0)
 
 // raise a kernel's dynamic shared-memory limit to at least `bytes`, never
-// lower it: batches of different sizes live side by side in one context
+// lower it: batches of different sizes live side by side in one context, and
+// chains of different sizes on threads of their own (the look and the set
+// under one lock, or the smaller request could be the last to be set)
+namespace pqmc {
+inline std::mutex g_smem_lock;
+}
 template <typename F>
 inline cudaError_t raise_dyn_smem(F* fn, int bytes) {
+  const std::lock_guard<std::mutex> lock(pqmc::g_smem_lock);
   cudaFuncAttributes a;
   cudaError_t e = cudaFuncGetAttributes(&a, (const void*)fn);
   if (e != cudaSuccess) return e;
