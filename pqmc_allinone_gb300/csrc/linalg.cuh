@@ -6,8 +6,9 @@ namespace pqmc {
 // C = alpha*op(A)*op(B) + beta*C, ta/tb in {'N','C'}
 int zgemm(cudaStream_t s, char ta, char tb, int m, int n, int k, cplx alpha, const cplx* A, int lda,
           const cplx* B, int ldb, cplx beta, cplx* C, int ldc);
-// Householder QR, Q overwrites A (m x n), d = diag(R); work: m x n scratch,
-// err: device word that takes PQMC_ERR_TIMEOUT if a wait inside ran out
+// Householder QR, Q overwrites A (m x n), d = diag(R); work: m x m scratch (m
+// n words are used, and n n more where m m has room for them); err: device
+// word that takes PQMC_ERR_TIMEOUT if a wait inside ran out
 int house_qr(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* work, int* err);
 // the same, also returning R (n x n upper triangle, column-major) and
 // ln det Q (a phase) when R / lndet are not null
