@@ -292,3 +292,31 @@ def test_update_with_a_determinant_past_the_square_root_of_the_range():
     assert np.array_equal(g.field(), o.field())
     assert rel_fro(o.g(), before) > 0.1 and rel_fro(g.g(), o.g()) < 1e-10
     g.close()
+
+
+def test_a_family_without_plaquettes_changes_nothing():
+    """Sweep, weight and gradient, and a mixed-precision batch, with and without it: the same bits."""
+    torch = pytest.importorskip("torch")
+    from pqmc_allinone_gb300.autograd import log_weight
+    from pqmc_allinone_gb300.engine import PqmcBatch, PqmcChain
+    out = []
+    for keep in ([(0, 99), (1, 99), (2, 99), (3, 99)], [(2, 0), (0, 99), (1, 99), (3, 0), (2, 99), (3, 99), (1, 0)]):
+        m, f = _families_cut(keep)
+        c = PqmcChain(m, field=f, rng_words=SEED_WORDS, meas=False)
+        x = torch.from_numpy(np.ascontiguousarray(f)[None].copy()).cuda().requires_grad_(True)
+        w = log_weight(x, [c])
+        (grad,) = torch.autograd.grad(w.sum(), x)
+        c.set_field(f)
+        c.init_expkv()
+        c.init_g(1)
+        c.sweep_slices(1, 1, m.ntime)
+        c.sweep_slices(2, 1, m.ntime)
+        b = PqmcBatch([m], [f], [SEED_WORDS], precision=1)
+        b.init()
+        b.sweep(1)
+        b.sweep(2)
+        out.append((w.detach().cpu().numpy(), grad.cpu().numpy(), c.field(), c.g(), b.chains[0].field(), b.chains[0].g()))
+        b.close()
+        c.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
