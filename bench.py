@@ -556,17 +556,17 @@ def run_mixed(args, world, rank, local):
                            "rounds included)",
             "flush_rounds_group0": rounds_g0,
             "peak_source": f"{pk['source']} HBM copy bandwidth; bf16 sustained for the tensor figure",
-            "scan": {"kernel": "k_bscan (sequential ratio scan, one CTA per chain)",
+            "scan": {"kernel": "k_bscan (sequential ratio scan, a CTA or a cluster of CTAs per chain)",
                      "sm_cycles_per_accepted_move": sc_cyc / max(1, sc_acc),
                      "sm_cycles_per_proposal": sc_cyc / max(1, sc_acc + sc_rej),
                      "accepted": sc_acc, "rejected": sc_rej,
                      "definition": "device clock64 of every scan CTA from its start to its last bookkeeping, "
                                    "summed over the two phase-timed blocks of all chains, over the moves it "
-                                   "accepted (the scan's cost model: ~17k cycles per accepted move, 11k of them the "
-                                   "panel stream)"},
-            "dominant_by_time": "k_bscan: the sequential ratio scan, one CTA per chain, latency-bound by the "
-                                "Markov order, neither an HBM nor a tensor-pipe kernel (its cycles per accepted "
-                                "move are under scan)"}
+                                   "accepted (most of a move is the pass over the panel columns: the round's first "
+                                   "ones from shared memory, the later ones read back from L2)"},
+            "dominant_by_time": "k_bscan: the sequential ratio scan, a CTA or a cluster of CTAs per chain, "
+                                "latency-bound by the Markov order, neither an HBM nor a tensor-pipe kernel (its "
+                                "cycles per accepted move are under scan)"}
     total_ms = sum(v[0] for v in phases.values())
     phase_out = {k: {"ms_per_step": v[0] / 2, "share": v[0] / total_ms if total_ms else None,
                      "launch_groups": v[1]} for k, v in phases.items()}

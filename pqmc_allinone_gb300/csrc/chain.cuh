@@ -55,7 +55,7 @@ struct PlaqPre {
   cplx delta[16];   // Delta = expKV_inv(old) expKV(new) - I
   cplx enew[16];    // expKV(new)
   cplx einv[16];    // expKV_inv(new)
-  float2 deltaf[16];// Delta rounded to FP32 for the fast test
+  float2 deltaf[16];// Delta rounded to FP32 for the mixed batch's scan
   float4 deltad[16];// Delta in double-float {re_hi, im_hi, re_lo, im_lo} (mixed batch)
   double dE;        // -dtau * (E_new - E_old)
   double xnew;

@@ -5,7 +5,8 @@
 //
 // GB300 runs FP64 at a small fraction of its FP32 rate, so every routine
 // spreads its work over all SMs: the factorisations are cooperative kernels
-// that pipeline over columns, the products are tiled GEMMs.
+// that pipeline over columns, the products give every warp its share of the
+// outputs and of the sums.
 #include <type_traits>
 #include "linalg.cuh"
 #include "warp_sum.cuh"
@@ -291,8 +292,9 @@ __device__ __forceinline__ Reflector reflector(cplx alpha, double ss, double n2)
 // reflector at 288 rows.  Here only the triangular system is a chain, of 1.1k
 // cycles a step, and FP64 issue and the loops' own instructions bound the rest
 // (76k, 153k and 159k cycles for the products, the system and U y of the last
-// column at 288 x 144; the whole factorisation takes 617 us with this and 733
-// without, 1054 and 1158 at 392 x 196).  One or two columns per CTA.  `gs` (n x n, column k holds
+// column at 288 x 144; the whole factorisation took 617 us with this and 733
+// without, 1054 and 1158 at 392 x 196; 628 and 1072 with sqrt(), a division and
+// the sums of UT_SUM).  One or two columns per CTA.  `gs` (n x n, column k holds
 // the products of column k) starts out LA_EMPTY like `pub`.
 constexpr int UT_SUM = 16;   // terms of U y in a sum of their own: one after another they gave 1.06 times the error
 __device__ __forceinline__ void form_q_ut(int m, int n, int b, int G, int nl, cplx* cols, cplx* pub, cplx* xs,
@@ -480,7 +482,8 @@ __device__ __forceinline__ void form_q_ut(int m, int n, int b, int G, int nl, cp
 // overlapping halves of one column's passage.  The next column comes first
 // and is published row by row.  (Every CTA with the norm and reflector of its
 // own, 2 of 6 multiply-adds a row and 2.1k cycles of root and division in the
-// chain: 875 us at 288 x 144 and 1.35 ms at 392 x 196, 733 us and 1.16 ms so.)  Q's columns need only reflectors
+// chain: 875 us at 288 x 144 and 1.35 ms at 392 x 196; 733 us and 1.16 ms so,
+// with Q by reflectors.)  Q's columns need only reflectors
 // that their CTA has already seen, so their formation starts without waiting
 // for the rest.  Bound by that chain (n steps) and, in a step, by the FP64
 // pipe.  A column whose entries pass 2^+-256 is held times a power of two
@@ -764,7 +767,8 @@ __global__ void __launch_bounds__(LT, 4) k_house_qr(int m, int n, cplx* A, cplx*
 // the bits, as integers), one reciprocal, the next column's update.
 // A step's multipliers -(c[p] / pivot) are formed for 16 columns at a time,
 // a real component per lane (two FP64 instructions instead of four a column):
-// 196 columns and 392 right-hand sides took 905 us with them in every lane.
+// 196 columns and 392 right-hand sides took 905 us with them in every lane,
+// 820 so, and 880 to 950 with a division for the reciprocal and the sums below.
 //
 // A right-hand side's terms are summed LU_SUM at a time apart from its
 // entries (`sums`) and added to them then, in both passes: one term after

@@ -24,8 +24,8 @@
 // from the twelve 2x2 minors of the row pairs, and no separate FP32 screen.
 // The other CTAs need Ns^2 dim complex multiply-adds per accepted move, 4.3 us
 // of the whole chip at Ns = 392 (8.6 us a move with the hand-over).  A family
-// step at 4x4 with Gaussian proposals takes 40 us (413 with one worker CTA
-// and 16 complex lanes), at 14x14 0.53 ms (0.91).
+// step at 4x4 with Gaussian proposals takes 41 us (413 with one worker CTA
+// and 16 complex lanes), at 14x14 0.48 ms (0.91).
 #include <cooperative_groups.h>
 #include "chain.cuh"
 #include "linalg.cuh"
