@@ -7,6 +7,7 @@
 // spreads its work over all SMs: the factorisations are cooperative kernels
 // that pipeline over columns, the products give every warp its share of the
 // outputs and of the sums.
+#include <algorithm>
 #include <type_traits>
 #include "linalg.cuh"
 #include "warp_sum.cuh"
@@ -774,11 +775,14 @@ __global__ void __launch_bounds__(LT, 4) k_house_qr(int m, int n, cplx* A, cplx*
 // entries (`sums`) and added to them then, in both passes: one term after
 // another each rounds at the entry's size, and G came out with twice the error
 // of dot products over 32 lanes (1.2e-15 and 6.4e-16 at n = 100; 6.5e-16 so).
-// Columns of A keep the plain order, which the pivots and the chain depend on;
-// so do right-hand sides in global memory in the first pass (n past ~590).
+// Columns of A keep the plain order, which the pivots and the chain depend on.
+// `nsum` columns of sums: where they are one for each of a CTA's right-hand
+// sides (`apart`) both passes use them; where shared memory has room for fewer
+// the elimination keeps the plain order and the substitution takes nsum
+// right-hand sides at a time (at n = 100: 7.4e-16).
 constexpr int LU_SUM = 16;
 __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx* B, int ldb, cplx* diag, int* perm,
-                                                 int* info, cplx* pub, int in_smem, int nst, int* err) {
+                                                 int* info, cplx* pub, int in_smem, int nst, int nsum, int apart, int* err) {
   extern __shared__ cplx lu_dyn[];
   __shared__ unsigned long long s_key[2][4];
   __shared__ int s_row[2][4];
@@ -789,15 +793,15 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
   cplx* s_rec = xs + (size_t)nst * n;          // reciprocals of the pivots
   int* s_prow = reinterpret_cast<int*>(s_rec + n);
   int* s_ord = s_prow + n;                     // step at which a row became the pivot row
-  cplx* sums = s_rec + n + (2 * n + 3) / 4;    // per local right-hand side (!in_smem: of the one in work)
+  cplx* sums = s_rec + n + (2 * n + 3) / 4;    // [nsum][n]
   const int lr = b >= n ? 0 : min(nl, (n - b + G - 1) / G);   // first local right-hand side
-  cplx* cols = sums + (in_smem ? (size_t)(nl - lr) * n : (size_t)n);
+  cplx* cols = sums + (size_t)nsum * n;
   auto gcol = [&](int l) {
     const size_t j = b + (size_t)l * G;
     return j < (size_t)n ? A + (size_t)n * j : B + (size_t)ldb * (j - n);
   };
   auto col = [&](int l) { return in_smem ? cols + (size_t)l * n : gcol(l); };
-  auto sum = [&](int l) { return in_smem ? sums + (size_t)(l - lr) * n : sums; };
+  auto sum = [&](int l) { return sums + (size_t)(l - lr) * n; };   // apart
   // own rows' sums of right-hand side l into its entries, but row p, which others read
   auto flush = [&](int l, int p) {
     cplx *c = col(l), *a = sum(l);
@@ -809,7 +813,7 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
   };
   if (tid == 0) s_fail = 0;
   for (int k = tid; k < n; k += LT) s_ord[k] = n;
-  if (in_smem)
+  if (apart)
     for (int k = tid; k < (nl - lr) * n; k += LT) sums[k] = mk(0.0);
   if (in_smem)
     for (int l = 0; l < nl; ++l)
@@ -818,7 +822,6 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
   if (b == 0)
     for (int k = tid; k < n; k += LT) publish(pub + k, col(0)[k]);
   const bool last_owner = (n - 1) % G == b;
-  const bool apart = in_smem && lr < nl;   // right-hand sides with their terms apart
   int first_zero = 0;
   int li = 0, jown = b;   // the next local column, local and global
   for (int j = 0; j < n; ++j) {
@@ -919,12 +922,13 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
   if (lr >= nl) return;
   __threadfence();
   __syncthreads();
-  const int nb = in_smem ? nl - lr : 1;
-  for (int r0 = lr; r0 < nl; r0 += nb) {
-    if (in_smem)
-      for (int l = lr; l < nl; ++l) flush(l, -1);
-    else
-      for (int k = tid; k < n; k += LT) sums[k] = mk(0.0);
+  if (apart)
+    for (int l = lr; l < nl; ++l) flush(l, -1);
+  for (int r0 = lr; r0 < nl; r0 += nsum) {
+    const int nb = min(nsum, nl - r0);
+    if (!apart)
+      for (int l = 0; l < nb; ++l)
+        for (int k = tid; k < n; k += LT) sums[(size_t)l * n + k] = mk(0.0);
     for (int u = 0; u < nst - 1; ++u) {
       const int j = n - 1 - u;
       if (j >= 0) fetch_col(pub + (size_t)n * j, xs + (size_t)(j & (nst - 1)) * n, 0, n);
@@ -941,7 +945,7 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
       if (!in_smem && tid == 0 && j < n - 1) sums[s_prow[j + 1]] = done;
       if (j % LU_SUM == LU_SUM - 1)
         for (int l = r0; l < r0 + nb; ++l) {
-          cplx *y = col(l), *a = sum(l);
+          cplx *y = col(l), *a = sums + (size_t)(l - r0) * n;
           for (int k = tid; k < n; k += LT)
             if (s_ord[k] < j) {
               y[k] = cadd(y[k], a[k]);
@@ -950,7 +954,7 @@ __global__ void __launch_bounds__(LT) k_lu_solve(int n, cplx* A, int nrhs, cplx*
         }
       double xl = 0.0;   // y[p] / u_jj of 16 columns at a time, a real component per lane
       for (int l = r0; l < r0 + nb; ++l) {
-        cplx *y = col(l), *a = sum(l);
+        cplx *y = col(l), *a = sums + (size_t)(l - r0) * n;
         const int lq = (l - r0) & 15;
         if (lq == 0) {
           const bool im = lane & 1;
@@ -1022,28 +1026,35 @@ int coop_grid(const void* fn, int threads, int want, size_t smem) {
 // Grid and shared memory of a column pipeline over `ncol` columns of `len`
 // rows.  Two CTAs per SM while their columns fit in half its shared memory
 // (at Ns = 392, nelec = 196 a CTA has one column of the QR), one while they
-// fit in all of it, and past that the columns stay in global memory.
-// `fixed`(grid, columns per CTA, in shared memory): complex entries besides
-// the ring and the columns.
+// fit in all of it, and past that the columns stay in global memory: the
+// first of the shapes `from` .. `to` - 1 that fits (grid 0: none).
+// `fixed`(grid, columns per CTA, in shared memory, room): complex entries
+// besides the ring and the columns, of `room` that are left.
 struct PipeShape {
   int grid, in_smem, nst;
   size_t smem;
 };
+enum { PIPE_ONE, PIPE_TWO, PIPE_TWO_SHORT, PIPE_ALL, PIPE_ALL_SHORT, PIPE_GLOBAL, PIPE_GLOBAL_SHORT, PIPE_END };
 template <typename FIXED>
-static int pipe_shape(const void* fn, int ncol, int len, FIXED fixed, PipeShape* out) {
+static int pipe_shape(const void* fn, int ncol, int len, int from, int to, FIXED fixed, PipeShape* out) {
   int dev = 0, nsm = 0;
   PQMC_CUDA(cudaGetDevice(&dev));
   PQMC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const struct { int per, nst, in; size_t lim; } opt[] = {
-      {1, 4, 1, 110 * 1024}, {2, 4, 1, 110 * 1024}, {1, 4, 1, 220 * 1024}, {1, 2, 1, 220 * 1024}, {1, 4, 0, 220 * 1024}, {1, 2, 0, 220 * 1024}};
-  for (const auto& o : opt) {
+  const struct { int per, nst, in; size_t lim; } opt[PIPE_END] = {
+      {1, 4, 1, 110 * 1024}, {2, 4, 1, 110 * 1024}, {2, 2, 1, 110 * 1024}, {1, 4, 1, 220 * 1024},
+      {1, 2, 1, 220 * 1024}, {1, 4, 0, 220 * 1024}, {1, 2, 0, 220 * 1024}};
+  out->grid = 0;
+  for (int k = from; k < to; ++k) {
+    const auto& o = opt[k];
     PipeShape q;
     q.grid = ncol < o.per * nsm ? ncol : o.per * nsm;
     q.in_smem = o.in;
     q.nst = o.nst;
     const int nl = (ncol + q.grid - 1) / q.grid;
-    q.smem = sizeof(cplx) * ((size_t)o.nst * len + fixed(q.grid, nl, o.in) + (o.in ? (size_t)nl * len : 0));
-    if (q.smem > o.lim || (&o == opt && nl > 2)) continue;
+    const size_t used = (size_t)o.nst * len + (o.in ? (size_t)nl * len : 0), most = o.lim / sizeof(cplx);
+    if (used > most || (k == PIPE_ONE && nl > 2)) continue;
+    q.smem = sizeof(cplx) * (used + fixed(q.grid, nl, o.in, most - used));
+    if (q.smem > o.lim) continue;
     PQMC_CUDA(raise_dyn_smem((const char*)fn, (int)q.smem));
     int per = 0;
     PQMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, LT, q.smem));
@@ -1051,6 +1062,9 @@ static int pipe_shape(const void* fn, int ncol, int len, FIXED fixed, PipeShape*
     *out = q;
     return PQMC_OK;
   }
+  return PQMC_OK;
+}
+static int pipe_none(int len) {
   set_error("dense factorisation: columns of %d entries do not fit in shared memory", len);
   return PQMC_ERR_ARG;
 }
@@ -1065,11 +1079,13 @@ int house_qr_r(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* R, cplx* ln
   // products behind the published columns (a square A has none), with the
   // terms of U y in sums (2) where shared memory has room for those too
   int ut = (size_t)m * (m - n) >= (size_t)n * n ? 2 : 0;
+  const auto fixed = [&](int, int nl, int in, size_t) {
+    return (size_t)2 * n + (n + 1) / 2 + (nl + 3) / 4 + (ut && in ? (size_t)nl * n : 0) + (ut == 2 && in ? (size_t)nl * m : 0);
+  };
   for (;; --ut) {
-    PQMC_TRY(pipe_shape((const void*)k_house_qr, n, m,
-                        [&](int, int nl, int in) {
-                          return (size_t)2 * n + (n + 1) / 2 + (nl + 3) / 4 + (ut && in ? (size_t)nl * n : 0) + (ut == 2 && in ? (size_t)nl * m : 0);
-                        }, &q));
+    PQMC_TRY(pipe_shape((const void*)k_house_qr, n, m, PIPE_ONE, PIPE_TWO_SHORT, fixed, &q));
+    if (!q.grid) PQMC_TRY(pipe_shape((const void*)k_house_qr, n, m, PIPE_ALL, PIPE_END, fixed, &q));
+    if (!q.grid) return pipe_none(m);
     if (ut == 0 || (q.in_smem && q.nst == 4 && n <= 2 * q.grid)) break;
   }
   PQMC_CUDA(cudaMemsetAsync(work, 0xff, sizeof(cplx) * ((size_t)m * n + (ut ? (size_t)n * n : 0)), s));
@@ -1082,10 +1098,24 @@ int house_qr_r(cudaStream_t s, int m, int n, cplx* A, cplx* d, cplx* R, cplx* ln
 int lu_solve(cudaStream_t s, int n, cplx* A, int nrhs, cplx* B, int ldb, cplx* diag, int* perm, int* info, cplx* work,
              int* err) {
   PipeShape q;
-  PQMC_TRY(pipe_shape((const void*)k_lu_solve, n + nrhs, n,
-                      [&](int grid, int, int in) { return (size_t)n + (2 * n + 3) / 4 + (in ? (size_t)((nrhs + grid - 1) / grid) * n : (size_t)n); }, &q));
+  // sums for every right-hand side of a CTA while that leaves two CTAs an SM,
+  // past that for as many as fit
+  int nsum = 0, apart = 1;
+  const auto fixed = [&](int grid, int, int in, size_t room) {
+    const size_t base = (size_t)n + (2 * n + 3) / 4;
+    const int rhs = (nrhs + grid - 1) / grid;
+    nsum = rhs;
+    if (!apart) nsum = std::min(rhs, in && room > base ? std::max(1, (int)((room - base) / n)) : 1);
+    return base + (size_t)nsum * n;
+  };
+  PQMC_TRY(pipe_shape((const void*)k_lu_solve, n + nrhs, n, PIPE_ONE, PIPE_ALL, fixed, &q));
+  if (!q.grid) {
+    apart = 0;
+    PQMC_TRY(pipe_shape((const void*)k_lu_solve, n + nrhs, n, PIPE_TWO, PIPE_END, fixed, &q));
+    if (!q.grid) return pipe_none(n);
+  }
   PQMC_CUDA(cudaMemsetAsync(work, 0xff, sizeof(cplx) * (size_t)n * n, s));
-  void* args[] = {&n, &A, &nrhs, &B, &ldb, &diag, &perm, &info, &work, &q.in_smem, &q.nst, &err};
+  void* args[] = {&n, &A, &nrhs, &B, &ldb, &diag, &perm, &info, &work, &q.in_smem, &q.nst, &nsum, &apart, &err};
   PQMC_CUDA(cudaLaunchCooperativeKernel((const void*)k_lu_solve, q.grid, LT, args, q.smem, s));
   PQMC_LAUNCHED();
   return PQMC_OK;

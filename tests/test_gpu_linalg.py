@@ -202,12 +202,15 @@ def test_lu_solve_sums_terms_apart(ns=392, ne=196, tol=7.4e-15):
     assert err < tol, err
 
 
-def test_lu_solve_with_columns_in_global_memory():
-    """Finite temperature at Ns = 800: columns and right-hand sides past what the CTAs' shared memory holds."""
+@pytest.mark.parametrize("L", [(16, 22), (20, 22)])
+def test_lu_solve_past_the_shared_memory(L):
+    """Finite temperature at Ns = 704, where the substitution takes one of a
+    CTA's right-hand sides at a time, and 880, where the columns stay in
+    global memory."""
     from oracle.finite_t import dense_g_and_weight
     from oracle.oracle import OracleChain
     from pqmc_allinone_gb300.engine import PqmcChain
-    m, f = epsocz_small(L=(20, 20), ntime=4, ngroup=2, alpha=0.3)
+    m, f = epsocz_small(L=L, ntime=4, ngroup=2, alpha=0.3)
     o = OracleChain(m, field=f, seed_words=SEED_WORDS, meas=False)
     o.init_expkv()
     g = PqmcChain(m, field=f, rng_words=SEED_WORDS, meas=False)
